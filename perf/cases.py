@@ -47,7 +47,7 @@ KB = 0.0019872041  # kcal/mol/K
 def listed():
     return [
         # the smallest: a peptide-sized molecule in vacuum, where launches and latency count
-        dict(name="chain_200_steps", kind="steps", system="chain", n=200, fp64=False, constrained=False, steps=50),
+        dict(name="chain_224_steps", kind="steps", system="chain", n=224, fp64=False, constrained=False, steps=50),
         # a small periodic box with constrained O-H bonds, a short run
         dict(name="water_1536_constrained", kind="steps", system="water", n=1536, fp64=False, constrained=True, steps=20),
         # the reference-precision run of 5,000 atoms
@@ -88,6 +88,8 @@ def draw(rng):
     n = int(math.exp(rng.uniform(math.log(150), math.log(hi))))
     if system == "water":
         n = max(n // 3 * 3, 192)
+    elif n < 1500:
+        n = max(n // 32 * 32, 160)
     most = 50 if n < 10000 else 20 if n < 60000 else 5
     if kind in ("forces", "build", "trait"):
         steps = 1
@@ -220,9 +222,9 @@ def _dt(case):
 
 
 def _batch_sizes(case):
-    """Uneven systems around the mean size."""
+    """Uneven systems, the largest 16 times the smallest, the largest first."""
     k = case["systems"]
-    return [max(60, int(case["n"] * 4.0 ** (2.0 * i / max(k - 1, 1) - 1.0))) for i in range(k)]
+    return [max(60, int(case["n"] * 4.0 ** (1.0 - 2.0 * i / max(k - 1, 1)))) for i in range(k)]
 
 
 def _moved(pos, seed):
