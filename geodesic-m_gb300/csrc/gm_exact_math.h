@@ -12,6 +12,16 @@
  *            FMA, and RN(q + r y) is the correctly rounded quotient when y is
  *            the correctly rounded reciprocal (away from overflow and
  *            underflow).  Three FP64 operations instead of a division.
+ * gm_min_image: d - L round(d / L), round half away from zero, each operation
+ *            rounded on its own: the reference's min_image
+ *            (neighbor.rs:74-76).  Away from |d| = L/2 the rounded quotient
+ *            is known without the division: 0 below it, +-1 between L/2 and
+ *            1.4 L, so the value is d, or d -+ L rounded once; both tests
+ *            are integer comparisons of the high words, 0.4 % clear of L/2.
+ *            An FP64 division and round are ~20 operations of a pipe with
+ *            1/64 of the FP32 rate (the divisions were a third of the FP64
+ *            pair kernel in a periodic box).  The value is the general
+ *            expression's for every d (a zero may differ in its sign).
  */
 #ifndef GM_EXACT_MATH_H
 #define GM_EXACT_MATH_H
@@ -46,6 +56,28 @@ GM_HD long long gm_f2fix(float v) {
         r = q + ((rem > half || (rem == half && (q & 1))) ? 1 : 0);
     }
     return (b >> 31) ? -r : r;
+}
+
+GM_HD int gm_hi_word(double v) {
+#ifdef __CUDA_ARCH__
+    return __double2hiint(v);
+#else
+    unsigned long long b;
+    memcpy(&b, &v, sizeof b);
+    return (int)(unsigned)(b >> 32);
+#endif
+}
+
+GM_HD double gm_min_image(double d, double L) {
+    const int hd = gm_hi_word(d) & 0x7fffffff, hl = gm_hi_word(L);
+    if (hd < hl - 0x101000) return d; /* |d| < L/2 (1 - 2^-8) */
+#ifdef __CUDA_ARCH__
+    if (hd > hl - 0xff000 && hd < hl + 0x70000) return __dsub_rn(d, copysign(L, d));
+    return __dsub_rn(d, __dmul_rn(L, round(__ddiv_rn(d, L))));
+#else
+    if (hd > hl - 0xff000 && hd < hl + 0x70000) return d - copysign(L, d);
+    return d - L * round(d / L);
+#endif
 }
 
 GM_HD double gm_div_by_dt(double num, double dt, double y) {

@@ -248,9 +248,10 @@ struct ForceArgs {
     const int *list, *count, *gmax;
     int ntypes;
     const float4 *tab32;     // (sigma_ij^2, 24 epsilon_ij) per type pair, each a double-float (hi, lo)
-    const double2 *tab64;    // (sigma_ij, epsilon_ij)
+    const double2 *tab64;    // (sigma_ij^2, 24 epsilon_ij)
     PairConst pc;            // the mixed pair kernel's constants
     double rc2_64, rsw_64, rc_64, inv_wsw_64;
+    float rc2_pre;           // FP64 kernel's FP32 pre-test: beyond it a pair is outside the cutoff for certain
     int coulomb;
     float box[3], inv_box[3];
     double box64[3];
@@ -311,14 +312,6 @@ struct ClusterArgs {
     int mi;                               // constraint differences at the nearest image of box64
     double box64[3];
 };
-
-// d taken to the nearest periodic image of a box of length L: the reference's
-// min_image, d - L * round(d / L) with round half away from zero; each
-// operation rounded on its own (never contracted into an FMA, whatever the
-// translation unit's -fmad setting), so the bits are the reference's
-__device__ __forceinline__ double gm_min_image(double d, double L) {
-    return __dsub_rn(d, __dmul_rn(L, round(__ddiv_rn(d, L))));
-}
 
 void gm_launch_half_kick(int n, double *vel, const long long *force, const double *inv_mass, double dt_half,
                          const DevStatus *st, cudaStream_t s);

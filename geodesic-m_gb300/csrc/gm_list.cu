@@ -28,11 +28,6 @@
 namespace {
 
 
-__device__ __forceinline__ double exact_min_image(double d, double L) {
-    // neighbor.rs:74-76: d - L * round(d / L), no contraction
-    return __dsub_rn(d, __dmul_rn(L, round(__ddiv_rn(d, L))));
-}
-
 __device__ __forceinline__ double exact_wrap(double x, double L) {
     // neighbor.rs:86-88: x - L * floor(x / L)
     return __dsub_rn(x, __dmul_rn(L, floor(__ddiv_rn(x, L))));
@@ -535,9 +530,9 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
                         bool in = (sure >> k) & 1u;
                         if (!in) {
                             // the reference's own FP64 decision
-                            double ex_ = exact_min_image(__dsub_rn(a.pos[jo], a.pos[my_orig]), bx[0]);
-                            double ey_ = exact_min_image(__dsub_rn(a.pos[n + jo], a.pos[n + my_orig]), bx[1]);
-                            double ez_ = exact_min_image(__dsub_rn(a.pos[2 * n + jo], a.pos[2 * n + my_orig]), bx[2]);
+                            double ex_ = gm_min_image(__dsub_rn(a.pos[jo], a.pos[my_orig]), bx[0]);
+                            double ey_ = gm_min_image(__dsub_rn(a.pos[n + jo], a.pos[n + my_orig]), bx[1]);
+                            double ez_ = gm_min_image(__dsub_rn(a.pos[2 * n + jo], a.pos[2 * n + my_orig]), bx[2]);
                             double rr = __dadd_rn(__dadd_rn(__dmul_rn(ex_, ex_), __dmul_rn(ey_, ey_)), __dmul_rn(ez_, ez_));
                             in = rr <= rl2_64;
                         }

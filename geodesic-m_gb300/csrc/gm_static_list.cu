@@ -70,11 +70,6 @@ int scratch_for(int device, Scratch **out) {
     return GM_OK;
 }
 
-__device__ __forceinline__ double min_image(double d, double L) {
-    // neighbor.rs:74-76: d - L * round(d / L), no contraction
-    return __dsub_rn(d, __dmul_rn(L, round(__ddiv_rn(d, L))));
-}
-
 // Cells searched along one axis around cell c: two on each side (cells are
 // at least half the list radius wide), the whole axis when that would meet
 // itself around a periodic box.
@@ -135,9 +130,9 @@ __device__ void for_each_partner(const PairTest &t, int i, F &&f) {
                 for (int k = t.S->cell_start[cell]; k < a1; k++) {
                     const int j = t.S->perm[k];
                     if (j <= i) continue;
-                    const double dx = min_image(__dsub_rn(t.pos[j], xi), t.box[0]);
-                    const double dy = min_image(__dsub_rn(t.pos[n + j], yi), t.box[1]);
-                    const double dz = min_image(__dsub_rn(t.pos[2 * n + j], zi), t.box[2]);
+                    const double dx = gm_min_image(__dsub_rn(t.pos[j], xi), t.box[0]);
+                    const double dy = gm_min_image(__dsub_rn(t.pos[n + j], yi), t.box[1]);
+                    const double dz = gm_min_image(__dsub_rn(t.pos[2 * n + j], zi), t.box[2]);
                     const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
                     if (!(r2 <= t.rl2)) continue;
                     if (e1 > e0 && in_row(t.excl, e0, e1, j)) continue;
