@@ -292,6 +292,13 @@ ForceArgs force_args(gm_ctx *c) {
     a.rc_64 = rc;
     a.inv_wsw_64 = 1.0 / (rc - rsw);
     {
+        // the FP32 distance carries the box's FP32 rounding for image pairs
+        double L = 0.0;
+        for (int d = 0; d < 3 && c->p.periodic; d++) L = std::max(L, c->p.box[d]);
+        const double r = rc + 1e-3 + 1e-6 * (L + rc);
+        a.rc2_pre = (float)(r * r * (1.0 + 1e-5));
+    }
+    {
         // double-float constants of the mixed pair kernel
         auto split = [](double x, float &h, float &l) { h = (float)x; l = (float)(x - (double)h); };
         PairConst &k = a.pc;
@@ -1321,7 +1328,7 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
                 // nonbonded.rs:46-47 Lorentz-Berthelot, evaluated as the reference does
                 const double sg = 0.5 * (sg_[a] + sg_[b]);
                 const double ep = std::sqrt(ep_[a] * ep_[b]);
-                tab64[T2 * (size_t)sy + a * (size_t)c->ntypes + b] = make_double2(sg, ep);
+                tab64[T2 * (size_t)sy + a * (size_t)c->ntypes + b] = make_double2(sg * sg, 24.0 * ep);
                 // the mixed pair kernel's double-float (sigma^2, 24 epsilon)
                 const double s2 = sg * sg, e24 = 24.0 * ep;
                 const float s2h = (float)s2, e24h = (float)e24;

@@ -42,18 +42,46 @@ pair_kernel_mixed(int n, int n_slots, int cap, int split, const float4 *__restri
                                                   tab, s_tab, k, force, epart, st, group_sys, e_sys);
 }
 
-// FP64 nonbonded kernel (the FP64 path): the reference's arithmetic
-// (force/nonbonded.rs:20-82) in FP64 on the sorted FP64 copies.  The same
-// work split as the mixed kernel (a 32-atom group's columns over `split`
-// warps, 2/4/8 warps per block, optional persistent grid), and the same
-// summation: FP64 sums over chunks of 32 entries folded into int64, so every
-// launch shape gives the same bits.
+// 1/sqrt(x) in FP64 from the MUFU seed: the seed's argument is x truncated to
+// FP32 and the seed is widened again by moving bits (no conversion
+// instruction: those run on the FP64 pipe), then one cubically convergent step,
+// y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 (|e| < 2^-20, so the error of the
+// step is below 2^-60): five FP64 operations, within 2 ulp.  x is a squared
+// distance, far inside FP32's normal range for every pair inside a cutoff
+// and away from contact; outside it (x < 2^-100 or beyond 2^100) the library's
+// square root and a division are used.
+__device__ __forceinline__ double rsqrt64(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    if ((unsigned)(hi - ((1023 - 100) << 20)) >= (unsigned)(200 << 20)) return 1.0 / sqrt(x);
+    const unsigned f = __funnelshift_l((unsigned)lo, (unsigned)hi, 3) + 0x40000000u;
+    const unsigned g = __float_as_uint(rsqrt_approx(__uint_as_float(f)));
+    const double y = __hiloint2double((int)((g >> 3) + (896u << 20)), (int)(g << 29));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// FP64 nonbonded kernel (the FP64 path): force/nonbonded.rs:20-82 in FP64 on
+// the sorted FP64 copies.  The same work split as the mixed kernel (a 32-atom
+// group's columns over `split` warps, 2/4/8 warps per block, optional
+// persistent grid), and the same summation: FP64 sums over chunks of 32
+// entries folded into int64, so every launch shape gives the same bits.
+// Bound: the FP64 pipe (one warp instruction per 16 cycles and SM), so the
+// work is moved off it where that costs no bit of precision:
+//   * an entry beyond the cutoff (42 % of a column) is dropped by an FP32
+//     distance from the slot records with a margin (rc2_pre) that covers its
+//     rounding, and the FP64 cutoff test is an integer comparison;
+//   * the nearest image is taken without a division (gm_min_image);
+//   * one reciprocal square root (rsqrt64) replaces a square root and a
+//     division, and the switch multiplies by 1 / (cutoff - switch radius).
+// An in-cutoff pair takes 28 (inside the switch radius) to 44 FP64 operations;
+// it took ~55 to ~85, and three more divisions in a periodic box.
 template <bool PERIODIC, bool COULOMB, bool BATCH, int W>
 __global__ void __launch_bounds__(W * 32)
 pair_kernel_f64(int n, int n_slots, int cap, int split, const double4 *__restrict__ p64,
                 const int *__restrict__ type_s, const int *__restrict__ perm, const int *__restrict__ list,
                 const int *__restrict__ count, const int *__restrict__ gmax, int ntypes,
-                const double2 *__restrict__ tab, double rc2, double rsw, double rc, double bx, double by, double bz,
+                const double2 *__restrict__ tab, const float4 *__restrict__ coord, float rc2_pre, double rc2,
+                double rsw, double inv_w, double bx, double by, double bz, float3 ibox,
                 long long *__restrict__ force, double *__restrict__ epart, DevStatus *st,
                 const int *__restrict__ group_sys, long long *e_sys) {
     extern __shared__ double2 s_tab64[];
@@ -62,7 +90,8 @@ pair_kernel_f64(int n, int n_slots, int cap, int split, const double4 *__restric
         __syncthreads();
     }
     const int lane = threadIdx.x & 31;
-    const double wsw = rc - rsw;
+    const double dsw0 = -30.0 * inv_w;  // dS/dr = -30 u^2 (1 - u)^2 / (cutoff - switch radius)
+    const unsigned long long rc2_bits = (unsigned long long)__double_as_longlong(rc2);
     const int n_work = (n_slots / 32) * split;
     for (int wid = blockIdx.x * W + (threadIdx.x >> 5); wid < n_work; wid += gridDim.x * W) {
     const int group = wid / split, part = wid - group * split;
@@ -70,8 +99,9 @@ pair_kernel_f64(int n, int n_slots, int cap, int split, const double4 *__restric
     const int atom = perm[s];  // -1 on a padding slot
     const bool valid = atom >= 0;
     double4 mi = make_double4(0, 0, 0, 0);
+    float4 mh = make_float4(0.f, 0.f, 0.f, 0.f), ml = mh;
     int cnt = 0, ti = 0;
-    if (valid) { mi = p64[s]; cnt = count[s]; ti = type_s[s]; }
+    if (valid) { mi = p64[s]; gm_ld_coord(coord + 2 * s, mh, ml); cnt = count[s]; ti = type_s[s]; }
     const double2 *trow = (BATCH ? tab + (size_t)group_sys[group] * ntypes * ntypes : s_tab64) + ti * ntypes;
     const double qi = mi.w * kCoulomb64;
     const int gm = gmax[group];
@@ -86,6 +116,18 @@ pair_kernel_f64(int n, int n_slots, int cap, int split, const double4 *__restric
         const int e1 = min(e0 + kChunk, min(e_end, cnt));
         for (int e = e0; e < e1; e++) {
             const int j = __ldg(L + (size_t)e * 32);
+            {
+                float4 jh, jl;
+                gm_ld_coord(coord + 2 * j, jh, jl);
+                float x = (jh.x - mh.x) + (jl.x - ml.x), y = (jh.y - mh.y) + (jl.y - ml.y),
+                      z = (jh.z - mh.z) + (jl.z - ml.z);
+                if (PERIODIC) {
+                    x = fmaf(-(float)bx, rintf(x * ibox.x), x);
+                    y = fmaf(-(float)by, rintf(y * ibox.y), y);
+                    z = fmaf(-(float)bz, rintf(z * ibox.z), z);
+                }
+                if (fmaf(z, z, fmaf(y, y, x * x)) > rc2_pre) continue;
+            }
             const double4 pj = p64[j];
             double dx = pj.x - mi.x, dy = pj.y - mi.y, dz = pj.z - mi.z;
             if (PERIODIC) {
@@ -93,35 +135,35 @@ pair_kernel_f64(int n, int n_slots, int cap, int split, const double4 *__restric
                 dy = gm_min_image(dy, by);
                 dz = gm_min_image(dz, bz);
             }
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 > rc2 || r2 == 0.0) continue;
-            const double r = sqrt(r2);
-            const double rinv = 1.0 / r;
-            const double2 p = trow[type_s[j]];
-            double v = 0.0, fr = 0.0;  // fr = F_r (radial magnitude)
-            if (p.y != 0.0) {
-                const double sr = p.x * rinv;
-                const double s2 = sr * sr, s4 = s2 * s2, s6 = s2 * s4, s12 = s6 * s6;
-                v = 4.0 * p.y * (s12 - s6);
-                fr = 24.0 * p.y * rinv * (2.0 * s12 - s6);
-            }
+            const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+            // r2 > rc2 or r2 == 0 on the bits (r2 >= 0); a NaN goes on and is flagged
+            const unsigned long long rb = (unsigned long long)__double_as_longlong(r2);
+            if (rb - 1 >= rc2_bits && rb <= 0x7ff0000000000000ull) continue;
+            const double rinv = rsqrt64(r2), rinv2 = rinv * rinv;
+            const double2 p = trow[type_s[j]];  // (sigma^2, 24 epsilon)
+            const double x = p.x * rinv2, x3 = x * x * x, ex3 = p.y * x3;
+            // F_r r and V
+            double fr = ex3 * fma(2.0, x3, -1.0);
+            double v = ex3 * (1.0 / 6.0) * (x3 - 1.0);
             if (COULOMB) {
                 const double vc = qi * pj.w * rinv;
                 v += vc;
-                fr += vc * rinv;
+                fr += vc;
             }
+            const double r = r2 * rinv;
             if (r > rsw) {
-                const double u = (r - rsw) / wsw;
+                const double u = (r - rsw) * inv_w;
                 const double u2 = u * u;
-                const double sw = 1.0 - 10.0 * u2 * u + 15.0 * u2 * u2 - 6.0 * u2 * u2 * u;
-                const double dsw = -30.0 * u2 * (1.0 - u) * (1.0 - u) / wsw;
-                fr = fr * sw - v * dsw;
+                const double sw = fma(u2 * u, fma(u, fma(-6.0, u, 15.0), -10.0), 1.0);
+                const double om = 1.0 - u;
+                const double dsw = dsw0 * (u2 * (om * om));
+                fr = fma(fr, sw, -(v * dsw * r));
                 v *= sw;
             }
-            const double g = fr * rinv;
-            fx -= g * dx;
-            fy -= g * dy;
-            fz -= g * dz;
+            const double g = fr * rinv2;
+            fx = fma(-g, dx, fx);
+            fy = fma(-g, dy, fy);
+            fz = fma(-g, dz, fz);
             eacc += v;
         }
         ax += gm_to_fix_checked(fx, bad);
@@ -232,7 +274,8 @@ void gm_launch_pair(const ForceArgs &a, bool fp64, cudaStream_t s) {
 #define GM_PAIR64W(P, Q, B, WW)                                                                                   \
     pair_kernel_f64<P, Q, B, WW><<<blocks64, WW * 32, smem, s>>>(                                                  \
         a.n, a.n_slots, a.cap, a.split, a.pos64s, a.type_sorted, a.perm, a.list, a.count, a.gmax, a.ntypes, a.tab64, \
-        a.rc2_64, a.rsw_64, a.rc_64, a.box64[0], a.box64[1], a.box64[2], a.force, a.epart, a.status, a.group_sys, \
+        a.coord, a.rc2_pre, a.rc2_64, a.rsw_64, a.inv_wsw_64, a.box64[0], a.box64[1], a.box64[2],                   \
+        make_float3(a.inv_box[0], a.inv_box[1], a.inv_box[2]), a.force, a.epart, a.status, a.group_sys, \
         a.e_sys)
 #define GM_PAIR64(P, Q, B) { if (W == 2) GM_PAIR64W(P, Q, B, 2); else if (W == 8) GM_PAIR64W(P, Q, B, 8); \
                              else GM_PAIR64W(P, Q, B, 4); }
