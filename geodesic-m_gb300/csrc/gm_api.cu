@@ -80,6 +80,7 @@ struct gm_ctx {
     // list
     int cap = 0, cap_seg = 0, n_groups = 0;  // list entries per atom; staging entries per atom and z layer
     int split = 1;                   // warps per group in the pair kernel
+    int term_chunk = 128;            // bonded terms per work item of the persistent kernel
     int pair_warps = 4, pair_grid = 0;  // FP32 pair kernel block size and grid (0: one item per warp)
     int *d_list = nullptr, *d_count = nullptr, *d_gmax = nullptr, *d_stage = nullptr;
     bool built = false;
@@ -274,6 +275,7 @@ ForceArgs force_args(gm_ctx *c) {
     a.e_sys = c->n_sys > 1 ? c->d_e_sys : nullptr;
     a.cap = c->cap;
     a.split = c->split;
+    a.term_chunk = c->term_chunk;
     a.pair_warps = c->pair_warps;
     a.pair_grid = c->pair_grid;
     a.coord = c->d_coord;
@@ -307,10 +309,13 @@ ForceArgs force_args(gm_ctx *c) {
         split(rsw, k.rsw, k.rsw_lo);
         split(1.0 / (rc - rsw), k.inv_w, k.inv_w_lo);
         split(-30.0 / (rc - rsw), k.mds, k.mds_lo);
+        double lmin = c->p.box[0];
         for (int d = 0; d < 3; d++) {
             split(c->p.box[d], k.box[d], k.box_lo[d]);
             k.inv_box[d] = (float)(1.0 / c->p.box[d]);
+            lmin = std::min(lmin, c->p.box[d]);
         }
+        k.img2 = (float)(0.49 * lmin * 0.49 * lmin);
     }
     a.coulomb = c->p.coulomb;
     for (int d = 0; d < 3; d++) {
@@ -1595,11 +1600,18 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
     cudaMemset(c->d_gmax, 0, sizeof(int) * (size_t)c->n_groups);
     c->n_epart = c->n_groups * GM_MAX_SPLIT + c->bonded_blocks + c->blocks14;
     {
-        // enough warps in flight to hide the gather latency: about 48 per SM
+        // about eight work items per resident warp (24 per SM), so that the
+        // last wave of the queue is short: with two or three (48 warps' worth
+        // of items) a fifth of the persistent kernel's warp time was the wait
+        // at its barrier.  A small system's items shrink to one chunk of
+        // columns and 32 bonded terms: its step is the longest item's latency
+        // (224 atoms: 61 us with 64 columns and 128 terms an item).
         int dev_sms = 0;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device);
-        const int want = 48 * std::max(dev_sms, 1);
-        c->split = std::max(1, std::min(GM_MAX_SPLIT, (want + c->n_groups - 1) / std::max(c->n_groups, 1)));
+        const int warps = 24 * std::max(dev_sms, 1);
+        c->split = std::max(1, std::min(GM_MAX_SPLIT, (8 * warps + c->n_groups - 1) / std::max(c->n_groups, 1)));
+        const long long terms = (long long)c->n_bonds + c->n_angles + c->n_diheds + c->n14;
+        c->term_chunk = terms > 32ll * warps ? 128 : 32;
     }
     TRY(dalloc(c, &c->d_epart, (size_t)c->n_epart));
     TRY(dalloc(c, &c->d_energy, 1));
@@ -2392,12 +2404,13 @@ int32_t gm_ensemble_energies(gm_ctx *c, double *e_pot, double *e_kin) {
 /* ---- autotuner ---------------------------------------------------------- */
 
 int32_t gm_pair_shape(gm_ctx *c, int32_t split, int32_t warps_per_block, int32_t grid) {
-    if (!c || split < 1 || split > GM_MAX_SPLIT || grid < 0 ||
+    if (!c || split < 1 || split > GM_SET_SPLIT || grid < 0 ||
         (warps_per_block != 2 && warps_per_block != 4 && warps_per_block != 8))
         return GM_ERR_INVALID_ARGUMENT;
     c->split = split;
     c->pair_warps = warps_per_block;
     c->pair_grid = grid;
+    c->persist_blocks = 0;
     drop_graph(c);  // the captured step holds the old launch shape
     return GM_OK;
 }
@@ -2462,6 +2475,8 @@ int32_t gm_autotune(gm_ctx *c, int32_t reps, int64_t *choice) {
         GM_CUDA(c, cudaMemsetAsync(c->d_sync, 0, sizeof(StepSync), c->stream));
         for (int sp : splits) {
             c->split = sp;
+            c->persist_blocks = 0;
+            if (persistent_grid(c) != GM_OK) continue;
             ForceArgs fa = force_args(c);
             gm_launch_forces_persistent(fa, c->d_sync, c->persist_blocks, c->stream);  // warm-up
             cudaEventRecord(e0, c->stream);
@@ -2477,6 +2492,7 @@ int32_t gm_autotune(gm_ctx *c, int32_t reps, int64_t *choice) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     c->split = bs;
+    c->persist_blocks = 0;
     GM_CUDA(c, cudaGetLastError());
     // the timing runs added forces many times over: evaluate them once more
     c->launches += seq_forces(c, c->stream);

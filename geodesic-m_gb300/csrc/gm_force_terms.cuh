@@ -29,7 +29,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // Minimum image of a pair difference held as dh (a multiple of 2^-8) plus
 // dl: the image shift n L is taken with L as a double-float, dh - n L_hi is
 // exact (Sterbenz), and the result is put back on the 2^-8 grid so that its
-// square stays exact.
+// square stays exact.  n = 0 leaves both unchanged.
 __device__ __forceinline__ void image_df(float &dh, float &dl, float L, float Llo, float iL) {
     const float k = rintf(dh * iL);
     dh = fmaf(-k, L, dh);
@@ -47,13 +47,26 @@ __device__ __forceinline__ void image_df(float &dh, float &dl, float L, float Ll
 //     2^-8 A and lo = the FP32 remainder.  dh = hj - hi is exact, each dh^2
 //     is exact (|dh| < 16 A) and so is their sum S; r^2 = S + c with
 //     c = dl (2 dh + dl), renormalised to (Rh, Rl).
+//   * Image (periodic): a raw S up to (0.49 box)^2 proves that no component
+//     needs one, so a row of 32 pairs pays one comparison and a vote, and the
+//     image (24 operations) only where a lane may cross a face.
 //   * 1/r^2 and 1/r: MUFU approximations corrected by one residual each.
 //   * LJ below the switch radius and the Coulomb term in double-float; the
 //     switch polynomial S(u) and dS/du in double-float; LJ inside the switch
-//     band (under 1e-2 kcal/mol/A there) in plain FP32.
+//     band (under 1e-2 kcal/mol/A there) in plain FP32.  Sums whose larger
+//     term is known take a Fast2Sum (the same two words as the TwoSum, three
+//     operations fewer).
 //   * F_i -= G d accumulated per lane with TwoSum over chunks of 32 entries;
 //     each chunk's (hi, lo) sum is folded into int64 fixed point, so the
-//     result is independent of how the columns are split over warps.
+//     result is independent of how the columns are split over warps.  (Biased
+//     accumulators that take half the operations, and a reassociated switch
+//     band, were tried: as exact against FP64, but not the same bits, and a
+//     trajectory of rigid-bond water doubles a 1e-10 difference every five
+//     steps.)
+// Bound: FP32 issue, then the L1 gathers (one wavefront per lane and entry).
+// A row of a column takes about 130 instructions inside the switch radius and
+// 210 in the band (137 and 231 before, and 24 more of each in a periodic box):
+// a step of 98,304 atoms of water executes 397 M warp instructions (479 M).
 // The list columns are ordered by build distance (inside the switch radius,
 // the switch band, then the shell beyond the cutoff), so a warp's 32 lanes
 // usually take the same branch and skip whole regions together.
@@ -74,20 +87,25 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
                 const int *__restrict__ group_sys, long long *e_sys) {
     const unsigned full = 0xffffffffu;
     const int group = wid / split, part = wid - group * split;
-    const int s = group * 32 + lane;
-    const int atom = perm[s];  // -1 on a padding slot
-    const bool valid = atom >= 0;
-    float4 mh = make_float4(0.f, 0.f, 0.f, 0.f), ml = mh;
-    int cnt = 0;
-    if (valid) { gm_ld_coord(coord + 2 * s, mh, ml); cnt = count[s]; }
-    const float4 *trow = (BATCH ? tab + (size_t)group_sys[group] * ntypes * ntypes : s_tab) +
-                         (valid ? gm_slot_type(ml.w) : 0) * ntypes;
-    const gm_df qi = gm_df_make(mh.w, ml.w);
     const int gm = gmax[group];
     const int per = ((gm + split - 1) / split + kChunk - 1) / kChunk * kChunk;
     const int e_begin = part * per, e_end = min(gm, e_begin + per);
-    const int *L = list + (size_t)group * 32 * cap + lane;
+    if (e_begin >= e_end) {  // no columns left for this part
+        if (ENERGY && lane == 0) epart[wid] = 0.0;
+        return;
+    }
+    const int s = group * 32 + lane;
+    const int atom = perm[s];  // -1 on a padding slot
+    const bool valid = atom >= 0;
+    // a padding lane stands on slot 0 and gathers slot 0: r2 == 0 drops it
     const int self = valid ? s : 0;
+    float4 mh, ml;
+    gm_ld_coord(coord + 2 * self, mh, ml);
+    const int cnt = valid ? count[s] : 0;
+    const float4 *trow = (BATCH ? tab + (size_t)group_sys[group] * ntypes * ntypes : s_tab) +
+                         (valid ? gm_slot_type(ml.w) : 0) * ntypes;
+    const gm_df qi = gm_df_make(mh.w, ml.w);
+    const int *L = list + (size_t)group * 32 * cap + lane;
     long long ax = 0, ay = 0, az = 0;
     double eacc = 0.0;
     unsigned int bad = 0;
@@ -107,91 +125,88 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
             for (int u = 0; u < kBatch; u++) gm_ld_coord(coord + 2 * jj[u], jhv[u], jlv[u]);
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {
-            const float4 jh = jhv[u], jl = jlv[u];
-            float d_h[3] = {jh.x - mh.x, jh.y - mh.y, jh.z - mh.z};
-            float d_l[3] = {jl.x - ml.x, jl.y - ml.y, jl.z - ml.z};
-            if (PERIODIC) {
+                const float4 jh = jhv[u], jl = jlv[u];
+                float d_h[3] = {jh.x - mh.x, jh.y - mh.y, jh.z - mh.z};
+                float d_l[3] = {jl.x - ml.x, jl.y - ml.y, jl.z - ml.z};
+                float S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));  // exact
+                if (PERIODIC) {
+                    if (__any_sync(full, S > k.img2)) {
 #pragma unroll
-                for (int d = 0; d < 3; d++) image_df(d_h[d], d_l[d], k.box[d], k.box_lo[d], k.inv_box[d]);
-            }
-            const float S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));  // exact
-            const float c = fmaf(d_l[2], fmaf(2.f, d_h[2], d_l[2]),
-                                 fmaf(d_l[1], fmaf(2.f, d_h[1], d_l[1]), d_l[0] * fmaf(2.f, d_h[0], d_l[0])));
-            const gm_df R = gm_fast_sum(S, c);  // r^2
-            const bool in = R.h <= k.rc2 && R.h > 0.f;
-            if (!__any_sync(full, in)) continue;  // warp-uniform: the shell beyond the cutoff
-            const float Rh = in ? R.h : 1.f, Rl = in ? R.l : 0.f;
-            // 1/r^2 = y (1 + rho - Rl y), rho = 1 - Rh y
-            const float y = rcp_approx(Rh);
-            const float rho = fmaf(-Rh, y, 1.f);
-            const gm_df inv = gm_df_make(y, y * fmaf(-Rl, y, rho));
-            // 1/r = z (1 - tau / 2), tau = (Rh + Rl) z^2 - 1 from exact products
-            const float z = rsqrt_approx(Rh);
-            const float a = __fmul_rn(Rh, z), ea = fmaf(Rh, z, -a);
-            const float tau = fmaf(Rl, y, fmaf(ea, z, fmaf(a, z, -1.f)));
-            const gm_df rinv = gm_df_make(z, -0.5f * z * tau);
-            const float4 p = BATCH ? __ldg(trow + gm_slot_type(jl.w)) : trow[gm_slot_type(jl.w)];
-            gm_df Vc = gm_df_make(0.f, 0.f), Gc = Vc;
-            if (COULOMB) {
-                Vc = gm_dmul(gm_dmul(qi, gm_df_make(jh.w, jl.w)), rinv);  // k q_i q_j / r
-                Gc = gm_dmul(Vc, inv);                                     // (k q_i q_j / r^2) / r
-            }
-            gm_df G = Gc;  // F_r / r
-            float v = 0.f;
-            const bool near = in && R.h <= k.rsw2;
-            const bool band = in && !near;
-            if (__any_sync(full, near) && near) {
-                const gm_df x = gm_dmul(gm_df_make(p.x, p.y), inv);  // (sigma / r)^2
-                const gm_df x3 = gm_dmul(gm_dsqr(x), x);
-                gm_df w2 = gm_two_sum(x3.h + x3.h, -1.f);  // 2 x3 - 1
-                w2.l += x3.l + x3.l;
-                const gm_df g = gm_dmul(gm_dmul(gm_dmul(gm_df_make(p.z, p.w), x3), w2), inv);
-                G = gm_dadd(g, Gc);
-                v = p.z * (1.f / 6.f) * x3.h * (x3.h - 1.f) + (Vc.h + Vc.l);
-            }
-            if (__any_sync(full, band) && band) {
-                // LJ in FP32 (tiny here), then V S and F_r S - V dS/dr
-                // (products rounded where the compiler could otherwise fuse them
-                // into the sums that follow)
-                const float xs = p.x * y, x3 = __fmul_rn(__fmul_rn(xs, xs), xs);
-                const float vlj = p.z * (1.f / 6.f) * x3 * (x3 - 1.f);
-                const float glj = p.z * x3 * fmaf(2.f, x3, -1.f) * y;
-                const gm_df V = gm_dadd(Vc, gm_df_make(vlj, 0.f));
-                const gm_df G0 = gm_dadd(Gc, gm_df_make(glj, 0.f));
-                const gm_df r = gm_dmul(gm_df_make(Rh, Rl), rinv);
-                gm_df u0 = gm_two_sum(r.h, -k.rsw);
-                u0.l += r.l - k.rsw_lo;
-                const gm_df uu = gm_dmul(u0, gm_df_make(k.inv_w, k.inv_w_lo));
-                const gm_df u2 = gm_dsqr(uu), u3 = gm_dmul(u2, uu);
-                // S = 1 + u^3 (-10 + u (15 - 6 u))
-                const float p6 = __fmul_rn(6.f, uu.h), e6 = fmaf(6.f, uu.h, -p6);
-                gm_df t = gm_two_sum(15.f, -p6);
-                t.l -= fmaf(6.f, uu.l, e6);
-                t = gm_dmul(uu, t);
-                gm_df t3 = gm_two_sum(-10.f, t.h);
-                t3.l += t.l;
-                t = gm_dmul(u3, t3);
-                gm_df sw = gm_two_sum(1.f, t.h);
-                sw.l += t.l;
-                // dS/dr = -30 u^2 (1 - u)^2 / w
-                gm_df om = gm_two_sum(1.f, -uu.h);
-                om.l -= uu.l;
-                const gm_df ds = gm_dmul(gm_dmul(u2, gm_dsqr(om)), gm_df_make(k.mds, k.mds_lo));
-                G = gm_dadd(gm_dmul(G0, sw), gm_dneg(gm_dmul(gm_dmul(V, ds), rinv)));
-                v = (V.h + V.l) * (sw.h + sw.l);
-            }
-            if (in) {
-                // F_i -= G d, each product with its exact error
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const float pr = __fmul_rn(G.h, d_h[d]);
-                    const float er = fmaf(G.h, d_l[d], fmaf(G.l, d_h[d], fmaf(G.h, d_h[d], -pr)));
-                    gm_df sum = gm_two_sum(acc[d].h, -pr);
-                    sum.l += acc[d].l - er;
-                    acc[d] = sum;
+                        for (int d = 0; d < 3; d++) image_df(d_h[d], d_l[d], k.box[d], k.box_lo[d], k.inv_box[d]);
+                        S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));
+                    }
                 }
-                if (ENERGY) ev += v;
-            }
+                const float c = fmaf(d_l[2], fmaf(2.f, d_h[2], d_l[2]),
+                                     fmaf(d_l[1], fmaf(2.f, d_h[1], d_l[1]), d_l[0] * fmaf(2.f, d_h[0], d_l[0])));
+                const gm_df R = gm_fast_sum(S, c);  // r^2
+                const bool in = R.h <= k.rc2 && R.h > 0.f;
+                if (!__any_sync(full, in)) continue;  // warp-uniform: the shell beyond the cutoff
+                if (in) {
+                    // 1/r^2 = y (1 + rho - Rl y), rho = 1 - Rh y
+                    const float y = rcp_approx(R.h);
+                    const float rho = fmaf(-R.h, y, 1.f);
+                    const gm_df inv = gm_df_make(y, y * fmaf(-R.l, y, rho));
+                    // 1/r = z (1 - tau / 2), tau = (Rh + Rl) z^2 - 1 from exact products
+                    const float z = rsqrt_approx(R.h);
+                    const float rz = __fmul_rn(R.h, z), ez = fmaf(R.h, z, -rz);
+                    const float tau = fmaf(R.l, y, fmaf(ez, z, fmaf(rz, z, -1.f)));
+                    const gm_df rinv = gm_df_make(z, -0.5f * z * tau);
+                    const float4 p = BATCH ? __ldg(trow + gm_slot_type(jl.w)) : trow[gm_slot_type(jl.w)];
+                    gm_df Vc = gm_df_make(0.f, 0.f), Gc = Vc;
+                    if (COULOMB) {
+                        Vc = gm_dmul(gm_dmul(qi, gm_df_make(jh.w, jl.w)), rinv);  // k q_i q_j / r
+                        Gc = gm_dmul(Vc, inv);                                     // (k q_i q_j / r^2) / r
+                    }
+                    gm_df G;  // F_r / r
+                    if (R.h <= k.rsw2) {
+                        const gm_df x = gm_dmul(gm_df_make(p.x, p.y), inv);  // (sigma / r)^2
+                        const gm_df x3 = gm_dmul(gm_dsqr(x), x);
+                        gm_df w2 = gm_two_sum(x3.h + x3.h, -1.f);  // 2 x3 - 1
+                        w2.l = fmaf(2.f, x3.l, w2.l);
+                        const gm_df g = gm_dmul(gm_dmul(gm_dmul(gm_df_make(p.z, p.w), x3), w2), inv);
+                        G = gm_dadd(g, Gc);
+                        if (ENERGY) ev += p.z * (1.f / 6.f) * x3.h * (x3.h - 1.f) + (Vc.h + Vc.l);
+                    } else {
+                        // LJ in FP32 (tiny here), then V S and F_r S - V dS/dr
+                        // (products rounded where the compiler could otherwise fuse them
+                        // into the sums that follow)
+                        const float xs = p.x * y, x3 = __fmul_rn(__fmul_rn(xs, xs), xs);
+                        const float vlj = p.z * (1.f / 6.f) * x3 * (x3 - 1.f);
+                        const float glj = p.z * x3 * fmaf(2.f, x3, -1.f) * y;
+                        const gm_df V = gm_dadd(Vc, gm_df_make(vlj, 0.f));
+                        const gm_df G0 = gm_dadd(Gc, gm_df_make(glj, 0.f));
+                        // r = r^2 / r, whose head and its error are rz and ez
+                        gm_df u0 = gm_fast_sum(rz, -k.rsw);
+                        u0.l += fmaf(R.l, z, fmaf(R.h, rinv.l, ez)) - k.rsw_lo;
+                        const gm_df uu = gm_dmul(u0, gm_df_make(k.inv_w, k.inv_w_lo));
+                        const gm_df u2 = gm_dsqr(uu), u3 = gm_dmul(u2, uu);
+                        // S = 1 + u^3 (-10 + u (15 - 6 u))
+                        const float p6 = __fmul_rn(6.f, uu.h), e6 = fmaf(6.f, uu.h, -p6);
+                        gm_df t = gm_fast_sum(15.f, -p6);
+                        t.l -= fmaf(6.f, uu.l, e6);
+                        t = gm_dmul(uu, t);
+                        gm_df t3 = gm_fast_sum(-10.f, t.h);
+                        t3.l += t.l;
+                        t = gm_dmul(u3, t3);
+                        gm_df sw = gm_fast_sum(1.f, t.h);
+                        sw.l += t.l;
+                        // dS/dr = -30 u^2 (1 - u)^2 / w
+                        gm_df om = gm_fast_sum(1.f, -uu.h);
+                        om.l -= uu.l;
+                        const gm_df ds = gm_dmul(gm_dmul(u2, gm_dsqr(om)), gm_df_make(k.mds, k.mds_lo));
+                        G = gm_dadd(gm_dmul(G0, sw), gm_dneg(gm_dmul(gm_dmul(V, ds), rinv)));
+                        if (ENERGY) ev += __fmul_rn(V.h + V.l, sw.h + sw.l);
+                    }
+                    // F_i -= G d, each product with its exact error
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        const float pr = __fmul_rn(G.h, d_h[d]);
+                        const float er = fmaf(G.h, d_l[d], fmaf(G.l, d_h[d], fmaf(G.h, d_h[d], -pr)));
+                        gm_df sum = gm_two_sum(acc[d].h, -pr);
+                        sum.l += acc[d].l - er;
+                        acc[d] = sum;
+                    }
+                }
             }
         }
         ax += gm_to_fix_checked(acc[0].h, bad) + gm_f2fix(acc[0].l);
@@ -199,7 +214,7 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
         az += gm_to_fix_checked(acc[2].h, bad) + gm_f2fix(acc[2].l);
         if (ENERGY) eacc += (double)ev;
     }
-    if (valid && e_begin < e_end) {
+    if (valid) {
         gm_atomic_fix_add(force + atom, ax);
         gm_atomic_fix_add(force + n + atom, ay);
         gm_atomic_fix_add(force + 2 * n + atom, az);

@@ -34,7 +34,8 @@ constexpr double GM_FORCE_TO_ACCEL = 20.455 * 20.455;  // kcal/mol/A/amu -> A/ps
 // in shared memory while it fits in 48 KB, in L1 otherwise).
 #define GM_MAX_TYPES 64
 #define GM_WARP 32
-#define GM_MAX_SPLIT 16      // largest number of warps per 32-atom group
+#define GM_MAX_SPLIT 32      // largest number of work items per 32-atom group in the pair kernels
+#define GM_SET_SPLIT 16      // largest one gm_pair_shape accepts and gm_autotune tries
 // The list build runs GM_NSEG warps per 32-atom group, one per z layer of the
 // 5 x 5 x (span + 4) cell box the group's candidates come from (cells are at
 // least half the list radius wide).  Each warp fills its own staging segment;
@@ -141,7 +142,15 @@ __device__ __forceinline__ void gm_add_sys_energy(long long *e_sys, int sy, doub
 // then a tree over the block (fixed order; every caller gets the same bits).
 __device__ __forceinline__ double gm_block_sum256(const double *x, int n, double *s) {
     double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += 256) acc += x[i];
+    int i = threadIdx.x;
+    for (; i + 15 * 256 < n; i += 16 * 256) {  // 16 loads in flight, added in order
+        double v[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) v[k] = x[i + 256 * k];
+#pragma unroll
+        for (int k = 0; k < 16; k++) acc += v[k];
+    }
+    for (; i < n; i += 256) acc += x[i];
     s[threadIdx.x] = acc;
     __syncthreads();
     for (int k = 128; k > 0; k >>= 1) {
@@ -231,6 +240,7 @@ struct PairConst {
     float inv_w, inv_w_lo;    // 1 / (cutoff - switch radius)
     float mds, mds_lo;        // -30 / (cutoff - switch radius): dS/dr = mds u^2 (1 - u)^2
     float box[3], box_lo[3], inv_box[3];
+    float img2;               // raw squared distances up to it need no image: (0.49 box)^2
 };
 
 struct ForceArgs {
@@ -239,6 +249,7 @@ struct ForceArgs {
     const int *group_sys, *atom_sys;
     long long *e_sys;        // per-system potential energy, fixed point 2^-32 kcal/mol (batches), or nullptr
     int split;               // warps per 32-atom group in the FP32 pair kernel
+    int term_chunk;          // bonded terms (or 1-4 pairs) per work item of the persistent kernel
     int pair_warps;          // warps per block of the FP32 pair kernel (2, 4, 8)
     int pair_grid;           // blocks of the FP32 pair kernel (0: one work item per warp; fewer: persistent)
     const float4 *coord;     // per slot (hi, lo) pairs: one 32-byte sector per gathered atom
@@ -370,7 +381,8 @@ struct StepArgs {
     unsigned int *sys_flag;
     StepSync *sync;
 };
-// Blocks of the cooperative grid (all co-resident); 0 when the form does not apply.
+// Blocks of the cooperative grid (all co-resident, no more than the work
+// items and atoms fill); 0 when the form does not apply.
 int gm_step_persistent_blocks(const ForceArgs &fa);
 void gm_launch_step_persistent(const ForceArgs &fa, const StepArgs &sa, const PackArgs &pk, int blocks,
                                cudaStream_t s);

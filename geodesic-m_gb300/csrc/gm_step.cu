@@ -5,7 +5,8 @@
 // the list that the graph's conditional rebuild left after it):
 //   1. forces F(x_k): every warp takes work items from one queue: the pair
 //      items of the mixed kernel (pair_item_mixed, a 32-atom group's share of
-//      list columns) and 128-term chunks of the bonded terms and 1-4 pairs,
+//      list columns) and chunks of the bonded terms and 1-4 pairs (128 terms,
+//      32 in a small system),
 //      spread evenly through the queue so that each SM mixes FP32 pair work
 //      with FP64 bonded work.  Skipped when the forces at x_k are summed
 //      already (the first launch of a call: the call starts with current
@@ -36,7 +37,6 @@ namespace {
 
 constexpr int kStepThreads = 128;
 constexpr int kStepMinBlocks = 6;  // 24 warps per SM: at most 80 registers a thread
-constexpr int kTermsPerTicket = 128;  // bonded terms (or 1-4 pairs) per work item, 32 per lane pass
 // ~64 ns per poll: about a quarter of a second before a block gives up
 constexpr unsigned kBarrierPolls = 1u << 22;
 
@@ -98,6 +98,19 @@ __device__ __forceinline__ void term_block_warp(const ForceArgs &fa, int blk, in
     if (lane == 0 && blk < (P14 ? fa.blocks14 : fa.bonded_blocks)) (P14 ? fa.epart14 : fa.epart_bonded)[blk] = v;
 }
 
+// Terms of a bonded ticket: the force phase alone keeps whole 64-term blocks
+// (their energy partials).
+template <bool STEP>
+__host__ __device__ __forceinline__ int ticket_terms(const ForceArgs &fa) {
+    return !STEP && fa.term_chunk < GM_BONDED_THREADS ? GM_BONDED_THREADS : fa.term_chunk;
+}
+__host__ __device__ __forceinline__ int bonded_tickets(const ForceArgs &fa, int chunk) {
+    return (fa.n_bonds + fa.n_angles + fa.n_diheds + chunk - 1) / chunk;
+}
+__host__ __device__ __forceinline__ int pair14_tickets(const ForceArgs &fa, int chunk) {
+    return (fa.n14 + chunk - 1) / chunk;
+}
+
 // STEP: one BAB step (phases 1-3 above, a cooperative launch).  !STEP: phase
 // 1 alone with energies (the pair items' partials, the 64-term blocks'
 // partials and the per-system energies of the force kernels, the same bits),
@@ -118,12 +131,11 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
             for (int t = threadIdx.x; t < fa.ntypes * fa.ntypes; t += blockDim.x) s_tab[t] = fa.tab32[t];
             __syncthreads();
         }
-        // tickets: n_pair pair items and nbw bonded tickets (kTermsPerTicket
-        // bonded terms or 1-4 pairs each), the bonded ones at t = k * stride
+        // tickets: n_pair pair items and nbw bonded tickets (chunk bonded
+        // terms or 1-4 pairs each), the bonded ones at t = k * stride
         const int n_pair = fa.n_groups * fa.split;
-        const int cb = (fa.n_bonds + fa.n_angles + fa.n_diheds + kTermsPerTicket - 1) / kTermsPerTicket;
-        const int c14 = (fa.n14 + kTermsPerTicket - 1) / kTermsPerTicket;
-        const int nbw = cb + c14, total = n_pair + nbw;
+        const int chunk = ticket_terms<STEP>(fa), cb = bonded_tickets(fa, chunk);
+        const int nbw = cb + pair14_tickets(fa, chunk), total = n_pair + nbw;
         const int stride = nbw > 0 ? total / nbw : 1;
         for (;;) {
             int t = 0;
@@ -136,14 +148,14 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
                 const bool b14 = q >= cb;
                 if (STEP) {
                     int first = -1;
-                    const int base = (b14 ? q - cb : q) * kTermsPerTicket + lane;
-                    for (int u = 0; u < kTermsPerTicket; u += 32) {
+                    const int base = (b14 ? q - cb : q) * chunk + lane;
+                    for (int u = 0; u < chunk; u += 32) {
                         if (b14) pair14_term<MI>(fa, base + u, bad, first);
                         else bonded_term<MI>(fa, base + u, bad, first);
                     }
                 } else {
-                    const int blk0 = (b14 ? q - cb : q) * (kTermsPerTicket / GM_BONDED_THREADS);
-                    for (int h = 0; h < kTermsPerTicket / GM_BONDED_THREADS; h++) {
+                    const int blk0 = (b14 ? q - cb : q) * (chunk / GM_BONDED_THREADS);
+                    for (int h = 0; h < chunk / GM_BONDED_THREADS; h++) {
                         if (b14) term_block_warp<MI, true>(fa, blk0 + h, lane, bad);
                         else term_block_warp<MI, false>(fa, blk0 + h, lane, bad);
                     }
@@ -268,7 +280,13 @@ int gm_step_persistent_blocks(const ForceArgs &fa) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick<true>(fa, gtab), kStepThreads, smem) != cudaSuccess)
         return 0;
-    return per_sm * sms;
+    // no more blocks than the tickets (a warp each) or the atoms fill: a
+    // small system's barrier waits for fewer arrivals
+    const int chunk = ticket_terms<true>(fa), warps = kStepThreads / 32;
+    const long long tickets = (long long)fa.n_groups * fa.split + bonded_tickets(fa, chunk) + pair14_tickets(fa, chunk);
+    const long long fill = (tickets + warps - 1) / warps, atoms = ((long long)fa.n + kStepThreads - 1) / kStepThreads;
+    const long long want = fill > atoms ? fill : atoms;
+    return (int)(want < (long long)per_sm * sms ? (want > 0 ? want : 1) : (long long)per_sm * sms);
 }
 
 void gm_launch_step_persistent(const ForceArgs &fa, const StepArgs &sa, const PackArgs &pk, int blocks,
