@@ -395,33 +395,83 @@ __device__ __forceinline__ float rel_r2(float4 c, float mx, float my, float mz, 
     return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 
+// A float as an integer of the same order, for the warp's integer min / max
+// reductions (and back: the map is its own inverse).
+__device__ __forceinline__ int ordered_int(float v) {
+    const int b = __float_as_int(v);
+    return b >= 0 ? b : b ^ 0x7fffffff;
+}
+__device__ __forceinline__ float warp_min(float v) {
+    const int r = __reduce_min_sync(0xffffffffu, ordered_int(v));
+    return __int_as_float(r >= 0 ? r : r ^ 0x7fffffff);
+}
+__device__ __forceinline__ float warp_max(float v) {
+    const int r = __reduce_max_sync(0xffffffffu, ordered_int(v));
+    return __int_as_float(r >= 0 ? r : r ^ 0x7fffffff);
+}
+
+// Distance of |d| beyond a half extent h, squared.
+__device__ __forceinline__ float beyond2(float d, float h) {
+    const float e = fmaxf(fabsf(d) - h, 0.f);
+    return e * e;
+}
+
+// Candidates a warp holds in shared memory between two rounds of tests (as
+// many bytes as a quarter as many staged words).
+constexpr int kRound = 256, kRoundY = 64;
+// Rows of 32 ints that 32 candidates (a word) take in the staging buffer: their
+// slots, then each lane's accept mask and the two bits of its bucket masks.
+constexpr int kWordRows = 4;
+// Groups (per system) up to which the build splits a layer's y rows over
+// warps: 162 groups 125 us against 191, 48 groups 66 against 144; 750 groups
+// 291 against 259, 3,072 groups 921 against 793 (partly filled words).
+constexpr int kYSplitGroups = 300;
+
 // One block per group, one warp per z layer: warp `seg` tests the candidates
-// of z layer `seg` of each row box its lanes need and stages them; the block
-// then concatenates the layers into each lane's list column.
+// of z layer `seg` of each row box its lanes need and stages what each lane
+// accepts; the block then writes the layers, one after the other, into each
+// lane's list column.
+//   * The candidates of the row box (5 x 5 x (span + 4) cells) pass 32 at a
+//     time, one a lane, and only those within the list radius of the lanes'
+//     bounding box are kept, in order, up to 256 in shared memory: 40 % of a
+//     row box is out of every lane's reach, and each candidate kept out saves
+//     32 distance tests.
+//   * Every lane tests the round's candidates, 32 a word, without a branch:
+//     an accept bit and the two bits of the distance bucket.  Bits near the
+//     list radius (decided in FP64) and pairs as close as the lane's farthest
+//     exclusion are looked at one by one; there are few.  A round with no
+//     candidate across a face takes no periodic image.
+//   * A system of few groups splits each layer into its five y rows as well
+//     (YS = 5: 25 warps per group, in the same order): its build is the time
+//     of one warp.
+//   * The words (not the entries) are staged, coalesced, and their bits counted
+//     per bucket; when every layer's counts are known each lane walks its own
+//     bits, eight words at a time, and stores each entry once, in its place.
+// Bound: issue.  98,304 atoms of water: 800 us; 1,800 us with a test of every
+// candidate of the row boxes, a walk per 32 candidates and every entry staged
+// (1.5 GB of DRAM traffic).
 // Each lane's column is written in distance-bucket order (GM_NBUCKET buckets
 // of the build-time distance, bounds in bucket_r2): inside the switch radius,
 // the switch band, the shell beyond the cutoff.  Within a bucket the entries
 // keep the single-warp sweep order.  The pair kernel's lanes then meet the
 // same kind of pair at the same entry and branch together.
-template <bool PERIODIC>
-__global__ void __launch_bounds__(GM_NSEG * 32)
+template <bool PERIODIC, int YS>
+__global__ void __launch_bounds__(GM_NSEG * YS * 32, YS == 1 ? 5 : 1)
 build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucket_r2) {
-    // candidates of the current batch: coordinates relative to the group's
-    // first atom (FP32; the rounding, under 1e-5 A for candidates within a
-    // few list radii, stays far inside the FP64 re-decision margin) and
-    // caller indices
-    __shared__ float4 s_rel[GM_NSEG][32];
-    __shared__ int s_orig[GM_NSEG][32];
-    __shared__ int s_cnt[GM_NSEG][GM_NBUCKET][32];
+    // the round's candidates: coordinates relative to the group's first atom
+    // (FP32; the rounding, under 1e-5 A for candidates within a few list
+    // radii, stays far inside the FP64 re-decision margin) and slot; the
+    // words being written out in the second part
+    constexpr int NSEG = GM_NSEG * YS, ROUND = YS == 1 ? kRound : kRoundY;
+    __shared__ float4 s_rel[NSEG][ROUND];
+    __shared__ int s_cnt[NSEG][GM_NBUCKET][32];
+    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int group = blockIdx.x, seg = wib;
-    const int gseg = group * GM_NSEG + seg;
+    const int gseg = group * NSEG + seg;
     if (group * 32 >= a.n_slots) return;
     const int sys = a.group_sys[group];
     if (!a.sys_flag[sys]) return;  // block-uniform: the system keeps its list
-    // the unrolled candidate loop below reads all 32 staging entries
-    s_rel[wib][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-    s_orig[wib][lane] = 0;
     const int soff = a.sys_slot_off[sys], coff = a.sys_cell_off[sys];
     const int ns = a.sys_atom_off[sys + 1] - a.sys_atom_off[sys];
     const int s = group * 32 + lane;
@@ -445,126 +495,205 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
         my_orig = a.perm[s];
         my_cell = a.cell_sorted[s];
     }
-    // own exclusions (caller indices, ascending); up to 8 kept in registers
+    // own exclusions as slots, up to 8 kept in registers, and the largest
+    // squared distance among them: pairs beyond it skip the scan.  The atom
+    // itself (distance 0) is no candidate either.
     int e0 = 0, e1 = 0;
     int ex[8];
     if (valid) { e0 = a.excl_start[my_orig]; e1 = a.excl_start[my_orig + 1]; }
     const int ne = e1 - e0;
+    float ex_r2 = 0.f;
+    for (int k = 0; k < ne; k++) {
+        float4 ch, cl;
+        gm_ld_coord(a.coord + 2 * a.slot_of[a.excl[e0 + k]], ch, cl);
+        const float4 c = make_float4((ch.x - rh.x) + (cl.x - rl.x), (ch.y - rh.y) + (cl.y - rl.y),
+                                     (ch.z - rh.z) + (cl.z - rl.z), 0.f);
+        ex_r2 = fmaxf(ex_r2, rel_r2<PERIODIC>(c, mx, my, mz, g));
+    }
 #pragma unroll
-    for (int k = 0; k < 8; k++) ex[k] = (k < ne) ? a.excl[e0 + k] : -1;
-    // the exclusions span [ex_lo, ex_hi] in caller index: candidates outside
-    // skip the scan
-    const int ex_lo = ne > 0 ? ex[0] : INT_MAX, ex_hi = ne > 0 ? a.excl[e1 - 1] : INT_MIN;
+    for (int k = 0; k < 8; k++) ex[k] = k < ne ? a.slot_of[a.excl[e0 + k]] : s;
     // Candidate regions, one per distinct cell row (cy, cz) among the lanes:
     // a group of 32 sorted atoms usually lies in one row of cells, sometimes
     // straddles the end of a row.  Sweeping each row's own 5 x 5 x (span + 4)
     // box keeps the regions tight (one box over both rows would cover the
-    // whole row); a lane tests only the candidates of its own row's box, so
-    // it never meets a candidate twice.  This warp takes z layer `seg` of
-    // each box.
+    // whole row); a lane tests only the candidates of one box, so it never
+    // meets a candidate twice.  This warp takes z layer `seg` (and with YS a
+    // share of its y rows) of each box.
     const int cx = my_cell % g.nc[0], cy = (my_cell / g.nc[0]) % g.nc[1], cz = my_cell / (g.nc[0] * g.nc[1]);
     const int row_id = valid ? cz * g.nc[1] + cy : -1;
-    const int cap_seg = a.cap_seg;
-    int *my_stage = a.stage + (size_t)gseg * 32 * cap_seg + lane;
-    int cnt = 0;
-    int nb[GM_NBUCKET] = {0, 0, 0, 0};  // staged entries per bucket
+    const int cap_words = a.cap_seg / (YS * kWordRows);
+    int *stage = a.stage + (size_t)gseg * cap_words * (kWordRows * 32) + lane;
+    int n_words = 0;                    // words met (staged while they fit)
+    int nb[GM_NBUCKET] = {0, 0, 0, 0};  // accepted entries per bucket
     const double bx[3] = {a.box[0], a.box[1], a.box[2]};
-    unsigned remaining = __ballot_sync(0xffffffffu, valid);
+    const float slack = 1e-3f + (PERIODIC ? 2e-7f * fmaxf(g.box[0], fmaxf(g.box[1], g.box[2])) : 0.f);
+    unsigned remaining = __ballot_sync(full, valid);
     while (remaining) {
         const int leader = __ffs(remaining) - 1;
-        const int R = __shfl_sync(0xffffffffu, row_id, leader);
-        const bool mine = valid && row_id == R;
-        remaining &= ~__ballot_sync(0xffffffffu, mine);
-        const int xmin = __reduce_min_sync(0xffffffffu, mine ? cx : INT_MAX);
-        const int xmax = __reduce_max_sync(0xffffffffu, mine ? cx : INT_MIN);
-        const int yR = R % g.nc[1], zR = R / g.nc[1];
+        const int R = __shfl_sync(full, row_id, leader);
+        bool mine = valid && row_id == R;
+        int ymin = R % g.nc[1], ymax = ymin;
+        const int zR = R / g.nc[1];
+        int xmin, xmax;
+        if (!PERIODIC) {
+            // Near a droplet's surface 32 atoms may lie in many short rows of
+            // one layer: one sweep over all of them when it visits fewer cells
+            // (a row's own box is about 5 x 6 cells).  Candidates keep their
+            // order; the extra ones are out of reach of the lanes they are
+            // new to.
+            const bool layer = valid && cz == zR && ((remaining >> lane) & 1u);
+            const unsigned peers = __match_any_sync(full, layer ? row_id : -1 - lane);
+            const int rows = __popc(__ballot_sync(full, layer && (peers & ((1u << lane) - 1u)) == 0));
+            ymin = __reduce_min_sync(full, layer ? cy : INT_MAX);
+            ymax = __reduce_max_sync(full, layer ? cy : INT_MIN);
+            xmin = __reduce_min_sync(full, layer ? cx : INT_MAX);
+            xmax = __reduce_max_sync(full, layer ? cx : INT_MIN);
+            if (rows > 1 && ymax - ymin < 28 && (xmax - xmin + 5) * (ymax - ymin + 5) <= 30 * rows) mine = layer;
+            else ymin = ymax = R % g.nc[1];
+        }
+        remaining &= ~__ballot_sync(full, mine);
+        xmin = __reduce_min_sync(full, mine ? cx : INT_MAX);
+        xmax = __reduce_max_sync(full, mine ? cx : INT_MIN);
         Range rx = dim_range(xmin, xmax, g.nc[0], g.periodic, g.full[0]);
-        Range ry = dim_range(yR, yR, g.nc[1], g.periodic, g.full[1]);
+        Range ry = dim_range(ymin, ymax, g.nc[1], g.periodic, g.full[1]);
         Range rz = dim_range(zR, zR, g.nc[2], g.periodic, g.full[2]);
-        const int zz = rz.lo + seg;
-        if (zz > rz.hi) continue;  // warp-uniform
+        if (YS > 1) {
+            const int per = (ry.hi - ry.lo + YS) / YS;
+            ry.lo += seg % YS * per;
+            ry.hi = min(ry.hi, ry.lo + per - 1);
+        }
+        const int zz = rz.lo + seg / YS;
+        if (zz > rz.hi || ry.lo > ry.hi) continue;  // warp-uniform
         const int z = rz.wrap ? wrapi(zz, g.nc[2]) : zz;
-        for (int yy = ry.lo; yy <= ry.hi; yy++) {
-            const int y = ry.wrap ? wrapi(yy, g.nc[1]) : yy;
-            // the x extent as one or two runs of consecutive cells
-            int seg_lo[2], seg_hi[2], nrun;
-            if (!rx.wrap) { seg_lo[0] = rx.lo; seg_hi[0] = rx.hi; nrun = 1; }
-            else if (rx.lo < 0) { seg_lo[0] = rx.lo + g.nc[0]; seg_hi[0] = g.nc[0] - 1; seg_lo[1] = 0; seg_hi[1] = rx.hi; nrun = 2; }
-            else if (rx.hi >= g.nc[0]) { seg_lo[0] = rx.lo; seg_hi[0] = g.nc[0] - 1; seg_lo[1] = 0; seg_hi[1] = rx.hi - g.nc[0]; nrun = 2; }
-            else { seg_lo[0] = rx.lo; seg_hi[0] = rx.hi; nrun = 1; }
-            for (int sg = 0; sg < nrun; sg++) {
-                const int row = (z * g.nc[1] + y) * g.nc[0];
-                // the system's slots, made global
-                const int b0 = soff + cell_start[row + seg_lo[sg]], b1 = soff + cell_start[row + seg_hi[sg] + 1];
-                for (int base = b0; base < b1; base += 32) {
-                    const int t = base + lane;
-                    __syncwarp();
-                    if (t < b1) {
-                        float4 ch, cl;
-                        gm_ld_coord(a.coord + 2 * t, ch, cl);
-                        s_rel[wib][lane] = make_float4((ch.x - rh.x) + (cl.x - rl.x), (ch.y - rh.y) + (cl.y - rl.y),
-                                                       (ch.z - rh.z) + (cl.z - rl.z), 0.f);
-                        s_orig[wib][lane] = a.perm[t];
-                    }
-                    __syncwarp();
-                    if (!mine) continue;
-                    const int m = min(32, b1 - base);
-                    // distance tests of all 32 staged candidates: bit k of
-                    // `near` within the list radius plus the margin, of `sure`
-                    // within it minus the margin
-                    unsigned near = 0, sure = 0;
-#pragma unroll
-                    for (int k = 0; k < 32; k++) {
-                        const float r2 = rel_r2<PERIODIC>(s_rel[wib][k], mx, my, mz, g);
-                        near |= (r2 <= rl2_hi ? 1u : 0u) << k;
-                        sure |= (r2 <= rl2_lo ? 1u : 0u) << k;
-                    }
-                    near &= m < 32 ? (1u << m) - 1u : 0xffffffffu;
-                    const int self = s - base;
-                    if (self >= 0 && self < 32) near &= ~(1u << self);
-                    // the accepted candidates, in order
-                    while (near) {
-                        const int k = __ffs(near) - 1;
-                        near &= near - 1;
-                        const int jo = s_orig[wib][k];
-                        bool in = (sure >> k) & 1u;
-                        if (!in) {
-                            // the reference's own FP64 decision
-                            double ex_ = gm_min_image(__dsub_rn(a.pos[jo], a.pos[my_orig]), bx[0]);
-                            double ey_ = gm_min_image(__dsub_rn(a.pos[n + jo], a.pos[n + my_orig]), bx[1]);
-                            double ez_ = gm_min_image(__dsub_rn(a.pos[2 * n + jo], a.pos[2 * n + my_orig]), bx[2]);
-                            double rr = __dadd_rn(__dadd_rn(__dmul_rn(ex_, ex_), __dmul_rn(ey_, ey_)), __dmul_rn(ez_, ez_));
-                            in = rr <= rl2_64;
-                        }
-                        if (!in) continue;
-                        if (jo >= ex_lo && jo <= ex_hi) {
-                            bool excluded = false;
-#pragma unroll
-                            for (int q = 0; q < 8; q++) excluded |= (ex[q] == jo);
-                            if (ne > 8)
-                                for (int q = e0 + 8; q < e1; q++) excluded |= (a.excl[q] == jo);
-                            if (excluded) continue;
-                        }
-                        // the distance bucket, for accepted candidates only
-                        // (the same r2 as the test above)
-                        const float r2 = rel_r2<PERIODIC>(s_rel[wib][k], mx, my, mz, g);
-                        const int bk = (r2 > bucket_r2.x ? 1 : 0) + (r2 > bucket_r2.y ? 1 : 0) + (r2 > bucket_r2.z ? 1 : 0);
-                        if (cnt < cap_seg) {
-                            my_stage[(size_t)cnt * 32] = (base + k) | (bk << GM_BUCKET_SHIFT);
-#pragma unroll
-                            for (int q = 0; q < GM_NBUCKET; q++) nb[q] += bk == q;
-                        }
-                        cnt++;
-                    }
-                }
+        // the lanes' bounding box
+        const float lox = warp_min(mine ? mx : FLT_MAX), hix = warp_max(mine ? mx : -FLT_MAX);
+        const float loy = warp_min(mine ? my : FLT_MAX), hiy = warp_max(mine ? my : -FLT_MAX);
+        const float loz = warp_min(mine ? mz : FLT_MAX), hiz = warp_max(mine ? mz : -FLT_MAX);
+        const float bcx = 0.5f * (lox + hix), bcy = 0.5f * (loy + hiy), bcz = 0.5f * (loz + hiz);
+        // half extents, wider by the FP32 roundings of the tests below
+        const float bhx = 0.5f * (hix - lox) + slack, bhy = 0.5f * (hiy - loy) + slack, bhz = 0.5f * (hiz - loz) + slack;
+        // The x extent of each y row as one or two runs of consecutive cells
+        // (at most 32): lane r holds the slots [run_b, run_e) of run r.
+        int x0[2], x1[2], nrun = 1;
+        x0[0] = rx.lo; x1[0] = rx.hi; x0[1] = 0; x1[1] = -1;
+        if (rx.wrap && rx.lo < 0) { x0[0] = rx.lo + g.nc[0]; x1[0] = g.nc[0] - 1; x0[1] = 0; x1[1] = rx.hi; nrun = 2; }
+        else if (rx.wrap && rx.hi >= g.nc[0]) { x1[0] = g.nc[0] - 1; x0[1] = 0; x1[1] = rx.hi - g.nc[0]; nrun = 2; }
+        const int runs = (ry.hi - ry.lo + 1) * nrun;
+        int run_b = 0, run_e = 0;
+        if (lane < runs) {
+            const int yy = ry.lo + lane / nrun, sg = lane - lane / nrun * nrun;
+            const int row = (z * g.nc[1] + (ry.wrap ? wrapi(yy, g.nc[1]) : yy)) * g.nc[0];
+            run_b = soff + cell_start[row + x0[sg]];
+            run_e = soff + cell_start[row + x1[sg] + 1];
+        }
+        int run = 0, base = __shfl_sync(full, run_b, 0), end = __shfl_sync(full, run_e, 0);
+        int held = 0;               // candidates of the round
+        bool image = false;         // periodic: one of them may need the image
+        for (;;) {
+            while (base >= end && ++run < runs) {
+                base = __shfl_sync(full, run_b, run);
+                end = __shfl_sync(full, run_e, run);
             }
+            const bool more = run < runs;
+            if (more) {
+                const int t = base + lane;
+                base += 32;
+                float4 c = make_float4(0.f, 0.f, 0.f, __int_as_float(t));
+                bool keep = false, far = false;
+                if (t < end) {
+                    float4 ch, cl;
+                    gm_ld_coord(a.coord + 2 * t, ch, cl);
+                    c.x = (ch.x - rh.x) + (cl.x - rl.x);
+                    c.y = (ch.y - rh.y) + (cl.y - rl.y);
+                    c.z = (ch.z - rh.z) + (cl.z - rl.z);
+                    float dx = c.x - bcx, dy = c.y - bcy, dz = c.z - bcz;
+                    if (PERIODIC) {
+                        // a raw difference below half the box from every lane
+                        // of the bounding box needs no image
+                        far = fabsf(dx) + bhx >= 0.49f * g.box[0] || fabsf(dy) + bhy >= 0.49f * g.box[1] ||
+                              fabsf(dz) + bhz >= 0.49f * g.box[2];
+                        dx = fmaf(-g.box[0], rintf(dx * g.inv_box[0]), dx);
+                        dy = fmaf(-g.box[1], rintf(dy * g.inv_box[1]), dy);
+                        dz = fmaf(-g.box[2], rintf(dz * g.inv_box[2]), dz);
+                    }
+                    keep = beyond2(dx, bhx) + beyond2(dy, bhy) + beyond2(dz, bhz) <= rl2_hi;
+                }
+                const unsigned kept = __ballot_sync(full, keep);
+                if (keep) s_rel[wib][held + __popc(kept & ((1u << lane) - 1u))] = c;
+                held += __popc(kept);
+                if (PERIODIC) image |= __any_sync(full, keep && far);
+            }
+            if (more && held <= ROUND - 32) continue;
+            if (held == 0) break;
+            // ---- a round: all lanes test, 32 candidates a word
+            __syncwarp();
+            for (int w0 = 0; w0 < held; w0 += 32) {
+                unsigned acc = 0, blo = 0, bhi = 0, look = 0;
+                auto test = [&](float r2, int k) {
+                    const bool in = r2 <= rl2_hi, far1 = r2 > bucket_r2.y;
+                    acc |= (in ? 1u : 0u) << k;
+                    bhi |= (far1 ? 1u : 0u) << k;
+                    blo |= (r2 > (far1 ? bucket_r2.z : bucket_r2.x) ? 1u : 0u) << k;
+                    look |= (in && (r2 > rl2_lo || r2 <= ex_r2) ? 1u : 0u) << k;
+                };
+                if (PERIODIC && image) {
+#pragma unroll
+                    for (int k = 0; k < 32; k++) test(rel_r2<true>(s_rel[wib][w0 + k], mx, my, mz, g), k);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 32; k++) test(rel_r2<false>(s_rel[wib][w0 + k], mx, my, mz, g), k);
+                }
+                const int m = held - w0;
+                const unsigned live = !mine ? 0u : m < 32 ? (1u << m) - 1u : full;
+                acc &= live;
+                look &= live;
+                while (look) {
+                    const int k = __ffs(look) - 1;
+                    look &= look - 1;
+                    const float4 c = s_rel[wib][w0 + k];
+                    const int slot = __float_as_int(c.w);
+                    const float r2 = rel_r2<PERIODIC>(c, mx, my, mz, g);
+                    bool drop = false;
+                    if (r2 > rl2_lo) {
+                        // the reference's own FP64 decision
+                        const int jo = a.perm[slot];
+                        double ex_ = gm_min_image(__dsub_rn(a.pos[jo], a.pos[my_orig]), bx[0]);
+                        double ey_ = gm_min_image(__dsub_rn(a.pos[n + jo], a.pos[n + my_orig]), bx[1]);
+                        double ez_ = gm_min_image(__dsub_rn(a.pos[2 * n + jo], a.pos[2 * n + my_orig]), bx[2]);
+                        double rr = __dadd_rn(__dadd_rn(__dmul_rn(ex_, ex_), __dmul_rn(ey_, ey_)), __dmul_rn(ez_, ez_));
+                        drop = !(rr <= rl2_64);
+                    }
+                    if (r2 <= ex_r2) {
+                        drop |= slot == s;
+#pragma unroll
+                        for (int q = 0; q < 8; q++) drop |= ex[q] == slot;
+                        for (int q = e0 + 8; q < e1; q++) drop |= a.slot_of[a.excl[q]] == slot;
+                    }
+                    if (drop) acc &= ~(1u << k);
+                }
+                if (n_words < cap_words) {  // (else flagged below, and not counted either)
+                    nb[0] += __popc(acc & ~(blo | bhi));
+                    nb[1] += __popc(acc & blo & ~bhi);
+                    nb[2] += __popc(acc & bhi & ~blo);
+                    nb[3] += __popc(acc & blo & bhi);
+                    int *row = stage + (size_t)n_words * (kWordRows * 32);
+                    row[0] = __float_as_int(s_rel[wib][w0 + lane].w);
+                    row[32] = (int)acc;
+                    row[64] = (int)blo;
+                    row[96] = (int)bhi;
+                }
+                n_words++;
+            }
+            __syncwarp();
+            held = 0;
+            image = false;
+            if (!more) break;
         }
     }
-    // concatenate the layers: lane l's layer k goes after its layers < k
-    int lmax = cnt;
-    for (int o = 16; o > 0; o >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
-    if (lane == 0) atomicMax(&a.status->max_layer, (unsigned)lmax);
-    const int staged = cnt < cap_seg ? cnt : cap_seg;
+    // the layers' entries go into the column one layer after the other
+    if (lane == 0) atomicMax(&a.status->max_layer, (unsigned)(n_words * kWordRows * YS));
+    const bool over = n_words > cap_words;
+    n_words = min(n_words, cap_words);
 #pragma unroll
     for (int q = 0; q < GM_NBUCKET; q++) s_cnt[seg][q][lane] = nb[q];
     __syncthreads();
@@ -576,7 +705,7 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
     for (int q = 0; q < GM_NBUCKET; q++) {
         int before = 0, all = 0;
 #pragma unroll
-        for (int k = 0; k < GM_NSEG; k++) {
+        for (int k = 0; k < NSEG; k++) {
             const int ck = s_cnt[k][q][lane];
             before += k < seg ? ck : 0;
             all += ck;
@@ -584,24 +713,44 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
         off[q] = total + before;
         total += all;
     }
-    int smax = staged;
-    for (int o = 16; o > 0; o >>= 1) smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, o));
     int *my_list = a.list + (size_t)group * 32 * cap + lane;
-    for (int e = 0; e < smax; e++) {
-        if (e < staged) {
-            const int v = my_stage[(size_t)e * 32];
-            const int bk = v >> GM_BUCKET_SHIFT;
+    constexpr int WB = ROUND / 32;  // words at a time: [row][word][lane]
+    int *buf = reinterpret_cast<int *>(s_rel[wib]);
+    for (int w0 = 0; w0 < n_words; w0 += WB) {
+        const int words = min(WB, n_words - w0);
+        __syncwarp();
+        const int *row = stage + (size_t)w0 * (kWordRows * 32);
+        int v[WB * kWordRows];
+#pragma unroll
+        for (int k = 0; k < WB * kWordRows; k++) v[k] = k < words * kWordRows ? row[k * 32] : 0;
+#pragma unroll
+        for (int k = 0; k < WB * kWordRows; k++) buf[((k % kWordRows) * WB + k / kWordRows) * 32 + lane] = v[k];
+        __syncwarp();
+        int w = 0;
+        unsigned acc = (unsigned)buf[WB * 32 + lane], blo = (unsigned)buf[2 * WB * 32 + lane],
+                 bhi = (unsigned)buf[3 * WB * 32 + lane];
+        for (;;) {
+            while (acc == 0 && ++w < words) {
+                acc = (unsigned)buf[(WB + w) * 32 + lane];
+                blo = (unsigned)buf[(2 * WB + w) * 32 + lane];
+                bhi = (unsigned)buf[(3 * WB + w) * 32 + lane];
+            }
+            if (acc == 0) break;
+            const int k = __ffs(acc) - 1;
+            acc &= acc - 1;
+            const int bk = ((blo >> k) & 1u) + 2 * ((bhi >> k) & 1u);
             int pos = 0;
 #pragma unroll
             for (int q = 0; q < GM_NBUCKET; q++) {
                 if (bk == q) { pos = off[q]; off[q]++; }
             }
-            if (pos < cap) my_list[(size_t)pos * 32] = v & GM_SLOT_MASK;
+            if (pos < cap) my_list[(size_t)pos * 32] = buf[w * 32 + k];
         }
     }
+    if (over && lane == 0) atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
     if (seg == 0) {
         if (valid) a.count[s] = total < cap ? total : cap;
-        if (valid && (cnt > cap_seg || total > cap)) atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
+        if (valid && total > cap) atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
         int c = valid ? (total < cap ? total : cap) : 0;
         int tm = valid ? total : 0;
         for (int o = 16; o > 0; o >>= 1) {
@@ -612,8 +761,6 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
             a.gmax[group] = c;
             atomicMax(&a.status->max_count, (unsigned)tm);
         }
-    } else if (valid && cnt > cap_seg) {
-        atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
     }
 }
 
@@ -664,8 +811,11 @@ void gm_launch_build(const ListArgs &a, cudaStream_t s) {
     // bucket bounds: the switch radius, the cutoff, halfway to the list radius
     const double rsh = 0.5 * (a.r_cut + a.r_list);
     const float3 bk = make_float3((float)(a.r_switch * a.r_switch), (float)(a.r_cut * a.r_cut), (float)(rsh * rsh));
-    if (a.periodic)
-        build_kernel<true><<<groups, GM_NSEG * 32, 0, s>>>(a, (float)(rl2 - margin), (float)(rl2 + margin), rl2, bk);
-    else
-        build_kernel<false><<<groups, GM_NSEG * 32, 0, s>>>(a, (float)(rl2 - margin), (float)(rl2 + margin), rl2, bk);
+    const float lo = (float)(rl2 - margin), hi = (float)(rl2 + margin);
+    // a system's rebuild covers groups / n_sys groups on average
+    const bool ysplit = groups / a.n_sys <= kYSplitGroups;
+#define GM_BUILD(P, Y) build_kernel<P, Y><<<groups, GM_NSEG * Y * 32, 0, s>>>(a, lo, hi, rl2, bk)
+    if (a.periodic) { if (ysplit) GM_BUILD(true, 5); else GM_BUILD(true, 1); }
+    else { if (ysplit) GM_BUILD(false, 5); else GM_BUILD(false, 1); }
+#undef GM_BUILD
 }
