@@ -98,7 +98,9 @@ struct gm_ctx {
     int n14 = 0, blocks14 = 0;
     int *d_p14i = nullptr, *d_p14j = nullptr;
     // constraints
-    int n_constr = 0, n_clusters = 0, n_single = 0, n_star_end = 0, n_warp_end = 0;
+    int n_constr = 0, n_clusters = 0, n_star_end = 0, n_warp_end = 0, n_lane_warps = 0;
+    int4 *d_lanes = nullptr;
+    int *d_lane_width = nullptr;
     int *d_ci = nullptr, *d_cj = nullptr, *d_cl_cstart = nullptr, *d_cl_cons = nullptr, *d_cl_astart = nullptr,
         *d_cl_atoms = nullptr, *d_cl_acstart = nullptr, *d_cl_acons = nullptr, *d_cl_iters = nullptr,
         *d_cl_worst_idx = nullptr;
@@ -353,8 +355,10 @@ ForceArgs force_args(gm_ctx *c) {
 ClusterArgs cluster_args(gm_ctx *c) {
     ClusterArgs a{};
     a.n_clusters = c->n_clusters;
-    a.n_single = c->n_single;
     a.n_star_end = c->n_star_end;
+    a.n_lane_warps = c->n_lane_warps;
+    a.lanes = c->d_lanes;
+    a.lane_width = c->d_lane_width;
     a.n_warp_end = c->n_warp_end;
     a.cl_cstart = c->d_cl_cstart; a.cl_cons = c->d_cl_cons;
     a.cl_astart = c->d_cl_astart; a.cl_atoms = c->d_cl_atoms;
@@ -1024,12 +1028,12 @@ void build_clusters(gm_ctx *c, const std::vector<int> &ci, const std::vector<int
         if (it == root_id.end()) { it = root_id.emplace(r, (int)ccons.size()).first; ccons.emplace_back(); catoms.emplace_back(); }
         ccons[(size_t)it->second].push_back(k);  // ascending k
     }
-    // clusters in four classes, in this order: one constraint on two atoms
-    // (one per thread), stars of 2-8 constraints on one centre atom (one per
-    // thread), other clusters of 2-32 constraints on at most 32 atoms with at
-    // most 8 constraints per atom (one per warp), the rest; within a class by
-    // size (stable), so a warp's threads run loops of the same lengths.  The
-    // solution does not depend on the cluster order.
+    // clusters in classes, in this order: one constraint on two atoms, stars
+    // of 2-8 constraints on one centre atom (both one constraint per lane),
+    // other clusters of 2-32 constraints on at most 32 atoms with at most 8
+    // constraints per atom (one per warp), the rest; within a class by size
+    // (stable), so a warp's lanes run loops of the same lengths.  The solution
+    // does not depend on the cluster order.
     const size_t ncl = ccons.size();
     std::vector<int> cls(ncl);
     for (size_t q = 0; q < ncl; q++) {
@@ -1059,8 +1063,7 @@ void build_clusters(gm_ctx *c, const std::vector<int> &ci, const std::vector<int
         if (cls[x] != cls[y]) return cls[x] < cls[y];
         return ccons[x].size() < ccons[y].size();
     });
-    c->n_single = (int)std::count(cls.begin(), cls.end(), 0);
-    c->n_star_end = c->n_single + (int)std::count(cls.begin(), cls.end(), 1);
+    c->n_star_end = (int)(std::count(cls.begin(), cls.end(), 0) + std::count(cls.begin(), cls.end(), 1));
     c->n_warp_end = c->n_star_end + (int)std::count(cls.begin(), cls.end(), 2);
     cstart.assign(1, 0);
     astart.assign(1, 0);
@@ -1084,6 +1087,33 @@ void build_clusters(gm_ctx *c, const std::vector<int> &ci, const std::vector<int
         }
         astart.push_back((int)atoms.size());
     }
+}
+
+// The stars' lanes: clusters [0, n_star_end), ordered by size, each on an
+// aligned group of 1, 2, 4 or 8 lanes; a warp holds groups of one width.
+void build_lanes(const gm_ctx *c, const std::vector<int> &cstart, const std::vector<int> &cons, std::vector<int4> &lanes,
+                 std::vector<int> &width) {
+    for (int cl = 0; cl < c->n_star_end; cl++) {
+        const int c0 = cstart[(size_t)cl], nc = cstart[(size_t)cl + 1] - c0;
+        const int w = nc == 1 ? 1 : nc == 2 ? 2 : nc <= 4 ? 4 : 8;
+        const bool full = lanes.size() == 32 * width.size();
+        if (full || width.back() != w) {
+            while (lanes.size() < 32 * width.size()) lanes.push_back(make_int4(0, 0, -1, -1));
+            width.push_back(w);
+        }
+        const int k0 = cons[(size_t)c0], i0 = c->h_ci[(size_t)k0], j0 = c->h_cj[(size_t)k0];
+        int cen = i0;
+        if (nc > 1) {
+            const int k1 = cons[(size_t)c0 + 1];
+            cen = (i0 == c->h_ci[(size_t)k1] || i0 == c->h_cj[(size_t)k1]) ? i0 : j0;
+        }
+        for (int q = 0; q < w; q++) {
+            if (q >= nc) { lanes.push_back(make_int4(cen, cen, -1, cl)); continue; }
+            const int k = cons[(size_t)(c0 + q)], i = c->h_ci[(size_t)k];
+            lanes.push_back(make_int4(cen, i == cen ? c->h_cj[(size_t)k] : i, k, cl));
+        }
+    }
+    while (lanes.size() < 32 * width.size()) lanes.push_back(make_int4(0, 0, -1, -1));
 }
 
 }  // namespace
@@ -1472,14 +1502,21 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         // the kernels index these prefix tables without bounds checks
         if (cstart.empty() || cstart.front() != 0 || cstart.back() != c->n_constr || astart.size() != cstart.size() ||
             astart.front() != 0 || astart.back() != (int)cat.size() || acstart.size() != cat.size() + 1 ||
-            acstart.front() != 0 || acstart.back() != (int)acons.size() || c->n_single > c->n_star_end ||
-            c->n_star_end > c->n_warp_end || c->n_warp_end > c->n_clusters) {
+            acstart.front() != 0 || acstart.back() != (int)acons.size() || c->n_star_end > c->n_warp_end || c->n_warp_end > c->n_clusters) {
             fail(c, GM_ERR_DEVICE, "inconsistent constraint cluster tables");
             return bail(GM_ERR_DEVICE);
         }
         TRY(dupload(c, &c->d_ci, c->h_ci.data(), c->h_ci.size()));
         TRY(dupload(c, &c->d_cj, c->h_cj.data(), c->h_cj.size()));
         TRY(dupload(c, &c->d_cdsq, t->constr_dsq, (size_t)c->n_constr));
+        {
+            std::vector<int4> lanes;
+            std::vector<int> width;
+            build_lanes(c, cstart, cons, lanes, width);
+            c->n_lane_warps = (int)width.size();
+            TRY(dupload(c, &c->d_lanes, lanes.data(), lanes.size()));
+            TRY(dupload(c, &c->d_lane_width, width.data(), width.size()));
+        }
         TRY(dupload(c, &c->d_cl_cstart, cstart.data(), cstart.size()));
         TRY(dupload(c, &c->d_cl_cons, cons.data(), cons.size()));
         TRY(dupload(c, &c->d_cl_astart, astart.data(), astart.size()));

@@ -213,13 +213,190 @@ __global__ void shake_prepare(ClusterArgs c, const double *dref, int n_atoms) {
     if (c.lam_sum) c.lam_sum[k] = 0.0;
 }
 
-// A star cluster: NC constraints that all share one centre atom (a heavy
-// atom and its NC hydrogens), one cluster per thread with every value in a
-// register.  The operations are those of the general sweep in the same
-// order: each constraint's multiplier, then each atom's sum over its
-// constraints (the centre's in ascending constraint order, from 0.0).
-template <bool RATTLE, int NC>
-__device__ void cluster_star(const ClusterArgs &c, int cl, double *pos, double *vel, int n, bool phase2) {
+// Star clusters: 1-8 constraints that all share one centre atom (a heavy atom
+// and its H atoms; a single constraint is a star of one).  One constraint per
+// lane: a star has a group of 1, 2, 4 or 8 lanes, each with its own H atom and
+// multiplier in registers and a copy of the centre, which all of them update
+// alike from the group's shuffled terms.  The operations are those of the
+// general sweep in the same order: each constraint's multiplier, then each
+// atom's sum over its constraints (the centre's in ascending constraint order,
+// from 0.0).  Differences are taken centre minus H whichever atom is the
+// constraint's i: both signs flip in every product, so the values are the
+// same bits.
+// An iteration is one serial chain of ~25 FP64 operations (a division among
+// them) whatever the star's size.  With a thread per star it was that for every
+// constraint of the star, and the one warp holding the four-H stars of a
+// 20,011-atom chain ran 113 us while every other was done in 20.
+struct StarLane {
+    int cen, h, k, cl;           // atoms, constraint (-1: a lane past the star's last), cluster
+    double cx, cy, cz, hx, hy, hz;  // SHAKE: positions; RATTLE: velocities
+    double rx, ry, rz;           // reference (SHAKE) or current (RATTLE) vector, centre - H
+    double inv_c, inv_h, wq, dsq;
+    double lam, acc;             // the last multiplier; the total (keep_sum)
+    unsigned it;                 // iterations done (alike over the group)
+    bool ok;                     // converged in phase 1
+};
+
+struct LaneGroup {
+    int width, base;
+    unsigned mask;
+};
+
+__device__ __forceinline__ LaneGroup lane_group(const ClusterArgs &c, int warp) {
+    LaneGroup g;
+    const int lane = threadIdx.x & 31;
+    g.width = c.lane_width[warp];
+    g.base = lane & ~(g.width - 1);
+    g.mask = ((1u << g.width) - 1u) << g.base;
+    return g;
+}
+
+// The displacement (or velocity change) of multiplier s.lam, for the groups
+// with `run`; every lane of the warp calls.
+__device__ __forceinline__ void lane_apply(StarLane &s, const LaneGroup &g, bool run) {
+    const unsigned full = 0xffffffffu;
+    const double w = s.lam * s.inv_c;
+    const double tx = w * s.rx, ty = w * s.ry, tz = w * s.rz;
+    double ddx = 0.0, ddy = 0.0, ddz = 0.0;
+    if (g.width == 1) {
+        ddx -= tx; ddy -= ty; ddz -= tz;
+    } else {
+        for (int q = 0; q < g.width; q++) {
+            // a lane past the star's last sends 0
+            ddx -= __shfl_sync(full, tx, g.base + q);
+            ddy -= __shfl_sync(full, ty, g.base + q);
+            ddz -= __shfl_sync(full, tz, g.base + q);
+        }
+    }
+    const double wh = s.lam * s.inv_h;
+    const double ux = wh * s.rx, uy = wh * s.ry, uz = wh * s.rz;
+    if (run) {
+        s.cx += ddx; s.cy += ddy; s.cz += ddz;
+        s.hx += ux; s.hy += uy; s.hz += uz;
+    }
+}
+
+// Jacobi iterations of every group of the warp: phase 1 to the group's own
+// convergence (at most `stop`), phase 2 to `stop`.
+template <bool RATTLE>
+__device__ __forceinline__ void lane_iterate(const ClusterArgs &c, StarLane &s, const LaneGroup &g, unsigned stop,
+                                             bool phase1, bool keep_sum) {
+    const unsigned full = 0xffffffffu;
+    for (;;) {
+        const bool run = s.cl >= 0 && s.it < stop && !(phase1 && s.ok);
+        if (!__any_sync(full, run)) break;
+        double l = 0.0;
+        if (s.k >= 0) {
+            const double dx = RATTLE ? s.cx - s.hx : cdiff(c, s.cx, s.hx, 0);
+            const double dy = RATTLE ? s.cy - s.hy : cdiff(c, s.cy, s.hy, 1);
+            const double dz = RATTLE ? s.cz - s.hz : cdiff(c, s.cz, s.hz, 2);
+            const double dot = dx * s.rx + dy * s.ry + dz * s.rz;
+            if (RATTLE) {
+                l = s.wq == 0.0 ? 0.0 : dot / s.wq;
+            } else {
+                const double diff = dx * dx + dy * dy + dz * dz - s.dsq;
+                const double denom = s.wq * dot;
+                l = denom == 0.0 ? 0.0 : diff / denom;
+            }
+        }
+        if (run) {
+            s.lam = l;
+            if (keep_sum) s.acc += l;
+        }
+        lane_apply(s, g, run);
+        // max |lambda| < tol over the group; a NaN counts as 0, as in the
+        // sequential sweep's strict comparison
+        const unsigned small = __ballot_sync(full, !(fabs(l) >= c.tol));
+        if (run) {
+            s.it++;
+            if (phase1) s.ok = (small & g.mask) == g.mask;
+        }
+    }
+}
+
+// The group's lane: atoms and constants.  `v`: the array that the solve
+// changes; RATTLE's vectors come from pos, SHAKE's from rvec.
+template <bool RATTLE>
+__device__ __forceinline__ void lane_constants(const ClusterArgs &c, int warp, StarLane &s) {
+    const int4 t = c.lanes[warp * 32 + (threadIdx.x & 31)];
+    s.cen = t.x; s.h = t.y; s.k = t.z; s.cl = t.w;
+    s.cx = s.cy = s.cz = s.hx = s.hy = s.hz = 0.0;
+    s.rx = s.ry = s.rz = s.inv_c = s.inv_h = s.wq = s.dsq = 0.0;
+    s.lam = s.acc = 0.0;
+    s.it = 0;
+    s.ok = false;
+    if (s.cl < 0) return;
+    s.inv_c = c.inv_mass[s.cen];
+    if (s.k >= 0) {
+        s.inv_h = c.inv_mass[s.h];
+        if (!RATTLE) {
+            s.dsq = c.constr_dsq[s.k];
+            s.wq = 2.0 * (s.inv_c + s.inv_h);
+        }
+    }
+}
+// RATTLE: the bond vector of the fixed positions and (1/m_i + 1/m_j) r^2
+__device__ __forceinline__ void lane_bond(const ClusterArgs &c, const double *pos, int n, StarLane &s) {
+    if (s.k < 0) return;
+    s.rx = cdiff(c, pos[s.cen], pos[s.h], 0);
+    s.ry = cdiff(c, pos[n + s.cen], pos[n + s.h], 1);
+    s.rz = cdiff(c, pos[2 * n + s.cen], pos[2 * n + s.h], 2);
+    const double rsq = s.rx * s.rx + s.ry * s.ry + s.rz * s.rz;
+    s.wq = (s.inv_c + s.inv_h) * rsq;
+}
+
+// The worst constraint of the group's last iteration (the first in ascending
+// order, a NaN never wins), alike over the group.
+__device__ __forceinline__ void lane_worst(const StarLane &s, const LaneGroup &g, double &mx, int &worst) {
+    const unsigned full = 0xffffffffu;
+    const double la = fabs(s.lam) > 0.0 ? fabs(s.lam) : 0.0;
+    mx = la;
+    for (int o = 1; o < 8; o <<= 1) {
+        const double m = __shfl_xor_sync(full, mx, o);
+        if (o < g.width) mx = fmax(mx, m);
+    }
+    const unsigned hit = __ballot_sync(full, s.k >= 0 && la == mx && mx > 0.0) & g.mask;
+    worst = __shfl_sync(full, s.k, hit ? __ffs(hit) - 1 : g.base);
+}
+
+// After phase 1: the clusters' counts and worst constraints, the failures and
+// the largest count (one atomic per warp).
+template <bool RATTLE>
+__device__ __forceinline__ void lane_report1(const ClusterArgs &c, const StarLane &s, const LaneGroup &g, unsigned *T) {
+    double mx;
+    int worst;
+    lane_worst(s, g, mx, worst);
+    const bool leader = s.cl >= 0 && (int)(threadIdx.x & 31) == g.base;
+    if (leader) {
+        c.cl_iters[s.cl] = (int)s.it;
+        c.cl_worst[s.cl] = mx;
+        c.cl_worst_idx[s.cl] = worst;
+        if (!s.ok) {
+            atomicOr(&c.status->error, RATTLE ? (unsigned)GM_DEV_RATTLE_FAIL : (unsigned)GM_DEV_SHAKE_FAIL);
+            atomicMin(&c.status->fail_step, c.status->step);
+        }
+    }
+    const unsigned it = __reduce_max_sync(0xffffffffu, leader ? s.it : 0u);
+    if ((threadIdx.x & 31) == 0 && it) atomicMax(T, it);
+}
+
+// After phase 2 of the groups that iterated (`ran`): counts, worst
+// constraints, and the check of the global stop rule.
+__device__ __forceinline__ void lane_report2(const ClusterArgs &c, const StarLane &s, const LaneGroup &g, unsigned T,
+                                             bool ran) {
+    double mx;
+    int worst;
+    lane_worst(s, g, mx, worst);
+    if (ran && s.cl >= 0 && (int)(threadIdx.x & 31) == g.base) {
+        c.cl_iters[s.cl] = (int)s.it;
+        c.cl_worst[s.cl] = mx;
+        c.cl_worst_idx[s.cl] = worst;
+        if (!(mx < c.tol) && T < c.max_iter) atomicOr(&c.status->error, (unsigned)GM_DEV_ITER_MISMATCH);
+    }
+}
+
+template <bool RATTLE>
+__device__ void star_phase(const ClusterArgs &c, int warp, double *pos, double *vel, int n, bool phase2) {
     const DevStatus *st = c.status;
     unsigned T = 0;
     if (!phase2) {
@@ -227,166 +404,46 @@ __device__ void cluster_star(const ClusterArgs &c, int cl, double *pos, double *
     } else {
         T = RATTLE ? st->rattle_T : st->shake_T;
         if ((st->error & ~(unsigned)(GM_DEV_SHAKE_FAIL | GM_DEV_RATTLE_FAIL)) != 0) return;
-        if ((unsigned)c.cl_iters[cl] >= T) return;
     }
-    const int c0 = c.cl_cstart[cl];
-    int kk[NC], hq[NC];
-    bool cen_i[NC];  // the centre is the constraint's i (it subtracts)
-    {
-        const int k0 = c.cl_cons[c0], k1 = c.cl_cons[c0 + 1];
-        const int i0 = c.constr_i[k0], j0 = c.constr_j[k0];
-        const int cen_ = (i0 == c.constr_i[k1] || i0 == c.constr_j[k1]) ? i0 : j0;
-#pragma unroll
-        for (int q = 0; q < NC; q++) {
-            const int k = c.cl_cons[c0 + q];
-            kk[q] = k;
-            const int i = c.constr_i[k];
-            cen_i[q] = i == cen_;
-            hq[q] = cen_i[q] ? c.constr_j[k] : i;
-        }
-        // centre
-        const int cen = cen_;
-        const double inv_c = c.inv_mass[cen];
-        double *v = RATTLE ? vel : pos;
-        double cx = v[cen], cy = v[n + cen], cz = v[2 * n + cen];
-        double hx[NC], hy[NC], hz[NC], inv_h[NC], rx[NC], ry[NC], rz[NC], wq[NC], dsq[NC], acc[NC];
-        const int ncst = c.n_constr;
-#pragma unroll
-        for (int q = 0; q < NC; q++) {
-            const int h = hq[q];
-            hx[q] = v[h]; hy[q] = v[n + h]; hz[q] = v[2 * n + h];
-            inv_h[q] = c.inv_mass[h];
-            const int k = kk[q];
-            const double inv_mi = cen_i[q] ? inv_c : inv_h[q], inv_mj = cen_i[q] ? inv_h[q] : inv_c;
-            if (!RATTLE) {
-                dsq[q] = c.constr_dsq[k];
-                rx[q] = c.rvec[k]; ry[q] = c.rvec[ncst + k]; rz[q] = c.rvec[2 * ncst + k];
-                wq[q] = 2.0 * (inv_mi + inv_mj);
-            } else {
-                const int i = cen_i[q] ? cen : h, j = cen_i[q] ? h : cen;
-                rx[q] = cdiff(c, pos[i], pos[j], 0);
-                ry[q] = cdiff(c, pos[n + i], pos[n + j], 1);
-                rz[q] = cdiff(c, pos[2 * n + i], pos[2 * n + j], 2);
-                const double rsq = rx[q] * rx[q] + ry[q] * ry[q] + rz[q] * rz[q];
-                wq[q] = (inv_mi + inv_mj) * rsq;
-                dsq[q] = 0.0;
-            }
-            acc[q] = 0.0;
-        }
-        const bool keep_sum = !RATTLE && c.lam_sum;
-        double lam[NC];
-        unsigned it;
-        double mx;
-        int worst;
-        bool apply_first = false;
-        if (!phase2) {
-            it = 0;
-            mx = 0.0;
-            worst = 0;
-            if (!RATTLE && c.lam0) {
-#pragma unroll
-                for (int q = 0; q < NC; q++) { acc[q] = c.lam0[kk[q]]; lam[q] = acc[q]; }
-                apply_first = true;
-            }
-        } else {
-            it = (unsigned)c.cl_iters[cl];
-            mx = c.cl_worst[cl];
-            worst = c.cl_worst_idx[cl];
-            if (keep_sum)
-#pragma unroll
-                for (int q = 0; q < NC; q++) acc[q] = c.lam_sum[kk[q]];
-        }
-        bool ok = false;
-        const unsigned stop = phase2 ? T : c.max_iter;
-        while (true) {
-            if (!apply_first) {
-                if (it >= stop) break;
-                double m_ = 0.0;
-                int w_ = kk[0];
-#pragma unroll
-                for (int q = 0; q < NC; q++) {
-                    // the constraint's i minus its j
-                    const double xi = cen_i[q] ? cx : hx[q], yi = cen_i[q] ? cy : hy[q], zi = cen_i[q] ? cz : hz[q];
-                    const double xj = cen_i[q] ? hx[q] : cx, yj = cen_i[q] ? hy[q] : cy, zj = cen_i[q] ? hz[q] : cz;
-                    double l_;
-                    if (RATTLE) {
-                        const double dvx = xi - xj;
-                        const double dvy = yi - yj;
-                        const double dvz = zi - zj;
-                        const double rel_vel = dvx * rx[q] + dvy * ry[q] + dvz * rz[q];
-                        l_ = wq[q] == 0.0 ? 0.0 : rel_vel / wq[q];
-                    } else {
-                        const double dx = cdiff(c, xi, xj, 0);
-                        const double dy = cdiff(c, yi, yj, 1);
-                        const double dz = cdiff(c, zi, zj, 2);
-                        const double diff = dx * dx + dy * dy + dz * dz - dsq[q];
-                        const double dot_new_old = dx * rx[q] + dy * ry[q] + dz * rz[q];
-                        const double denom = wq[q] * dot_new_old;
-                        l_ = denom == 0.0 ? 0.0 : diff / denom;
-                        if (keep_sum) acc[q] += l_;
-                    }
-                    lam[q] = l_;
-                    const double la = fabs(l_);
-                    if (la > m_) { m_ = la; w_ = kk[q]; }
-                }
-                mx = m_;
-                worst = w_;
-            }
-            // atoms: the centre over its constraints in ascending order, then each H
-            double ddx = 0.0, ddy = 0.0, ddz = 0.0;
-#pragma unroll
-            for (int q = 0; q < NC; q++) {
-                const double w = lam[q] * inv_c;
-                const double tx = w * rx[q], ty = w * ry[q], tz = w * rz[q];
-                if (cen_i[q]) { ddx -= tx; ddy -= ty; ddz -= tz; }
-                else { ddx += tx; ddy += ty; ddz += tz; }
-            }
-            cx += ddx; cy += ddy; cz += ddz;
-#pragma unroll
-            for (int q = 0; q < NC; q++) {
-                const double w = lam[q] * inv_h[q];
-                const double tx = w * rx[q], ty = w * ry[q], tz = w * rz[q];
-                double ex = 0.0, ey = 0.0, ez = 0.0;
-                if (cen_i[q]) { ex += tx; ey += ty; ez += tz; }
-                else { ex -= tx; ey -= ty; ez -= tz; }
-                hx[q] += ex; hy[q] += ey; hz[q] += ez;
-            }
-            if (apply_first) { apply_first = false; continue; }
-            it++;
-            if (!phase2 && mx < c.tol) { ok = true; break; }
-        }
-        v[cen] = cx; v[n + cen] = cy; v[2 * n + cen] = cz;
-#pragma unroll
-        for (int q = 0; q < NC; q++) {
-            const int h = hq[q];
-            v[h] = hx[q]; v[n + h] = hy[q]; v[2 * n + h] = hz[q];
-            if (keep_sum) c.lam_sum[kk[q]] = acc[q];
-        }
-        c.cl_iters[cl] = (int)it;
-        c.cl_worst[cl] = mx;
-        c.cl_worst_idx[cl] = worst;
-        if (!phase2) {
-            if (!ok) {
-                atomicOr(&c.status->error, RATTLE ? (unsigned)GM_DEV_RATTLE_FAIL : (unsigned)GM_DEV_SHAKE_FAIL);
-                atomicMin(&c.status->fail_step, c.status->step);
-            }
-            atomicMax(RATTLE ? &c.status->rattle_T : &c.status->shake_T, it);
-        } else if (!(mx < c.tol) && T < c.max_iter) {
-            atomicOr(&c.status->error, (unsigned)GM_DEV_ITER_MISMATCH);
+    const LaneGroup g = lane_group(c, warp);
+    StarLane s;
+    lane_constants<RATTLE>(c, warp, s);
+    if (phase2) {
+        s.it = s.cl >= 0 ? (unsigned)c.cl_iters[s.cl] : T;
+        if (!__any_sync(0xffffffffu, s.it < T)) return;
+    }
+    const bool ran = s.it < T;
+    double *v = RATTLE ? vel : pos;
+    const int ncst = c.n_constr;
+    if (s.cl >= 0) { s.cx = v[s.cen]; s.cy = v[n + s.cen]; s.cz = v[2 * n + s.cen]; }
+    if (s.k >= 0) {
+        s.hx = v[s.h]; s.hy = v[n + s.h]; s.hz = v[2 * n + s.h];
+        if (!RATTLE) {
+            // rvec is i - j
+            const bool flip = c.constr_i[s.k] != s.cen;
+            s.rx = c.rvec[s.k]; s.ry = c.rvec[ncst + s.k]; s.rz = c.rvec[2 * ncst + s.k];
+            if (flip) { s.rx = -s.rx; s.ry = -s.ry; s.rz = -s.rz; }
         }
     }
-}
-
-template <bool RATTLE>
-__device__ void cluster_star_any(const ClusterArgs &c, int cl, double *pos, double *vel, int n, bool phase2) {
-    switch (c.cl_cstart[cl + 1] - c.cl_cstart[cl]) {
-        case 2: cluster_star<RATTLE, 2>(c, cl, pos, vel, n, phase2); break;
-        case 3: cluster_star<RATTLE, 3>(c, cl, pos, vel, n, phase2); break;
-        case 4: cluster_star<RATTLE, 4>(c, cl, pos, vel, n, phase2); break;
-        case 5: cluster_star<RATTLE, 5>(c, cl, pos, vel, n, phase2); break;
-        case 6: cluster_star<RATTLE, 6>(c, cl, pos, vel, n, phase2); break;
-        case 7: cluster_star<RATTLE, 7>(c, cl, pos, vel, n, phase2); break;
-        default: cluster_star<RATTLE, 8>(c, cl, pos, vel, n, phase2); break;
+    if (RATTLE) lane_bond(c, pos, n, s);
+    const bool keep_sum = !RATTLE && c.lam_sum;
+    if (!phase2) {
+        if (!RATTLE && c.lam0) {
+            if (s.k >= 0) s.acc = s.lam = c.lam0[s.k];
+            lane_apply(s, g, s.cl >= 0);
+        }
+        lane_iterate<RATTLE>(c, s, g, c.max_iter, true, keep_sum);
+        lane_report1<RATTLE>(c, s, g, RATTLE ? &c.status->rattle_T : &c.status->shake_T);
+    } else {
+        if (keep_sum && s.k >= 0) s.acc = c.lam_sum[s.k];
+        lane_iterate<RATTLE>(c, s, g, T, false, keep_sum);
+        lane_report2(c, s, g, T, ran);
+        if (!ran) return;
+    }
+    if (s.cl >= 0 && (int)(threadIdx.x & 31) == g.base) { v[s.cen] = s.cx; v[n + s.cen] = s.cy; v[2 * n + s.cen] = s.cz; }
+    if (s.k >= 0) {
+        v[s.h] = s.hx; v[n + s.h] = s.hy; v[2 * n + s.h] = s.hz;
+        if (keep_sum) c.lam_sum[s.k] = s.acc;
     }
 }
 
@@ -569,135 +626,21 @@ __device__ void cluster_warp(const ClusterArgs &c, int cl, double *pos, double *
     }
 }
 
-// The per-atom update of a one-constraint cluster for multiplier l: atom i
-// subtracts, atom j adds, each sum starting from 0.0.
-__device__ __forceinline__ void single_apply(double l, double inv_mi, double inv_mj, double rx, double ry, double rz,
-                                             double &xi, double &yi, double &zi, double &xj, double &yj, double &zj) {
-    const double wi = l * inv_mi;
-    double ddx = 0.0, ddy = 0.0, ddz = 0.0;
-    ddx -= wi * rx; ddy -= wi * ry; ddz -= wi * rz;
-    const double wj = l * inv_mj;
-    double edx = 0.0, edy = 0.0, edz = 0.0;
-    edx += wj * rx; edy += wj * ry; edz += wj * rz;
-    xi += ddx; yi += ddy; zi += ddz;
-    xj += edx; yj += edy; zj += edz;
-}
-
-// A cluster of one constraint (one heavy atom and one H: most H-bond
-// clusters) entirely in scalar registers.  The operations are those of the
-// general path in the same order, including the per-atom sums that start
-// from 0.0, so the bits are the same.
-template <bool RATTLE>
-__device__ void cluster_single(const ClusterArgs &c, int cl, double *pos, double *vel, int n, bool phase2) {
-    const DevStatus *st = c.status;
-    unsigned T = 0;
-    if (!phase2) {
-        if (st->error) return;
-    } else {
-        T = RATTLE ? st->rattle_T : st->shake_T;
-        if ((st->error & ~(unsigned)(GM_DEV_SHAKE_FAIL | GM_DEV_RATTLE_FAIL)) != 0) return;
-        if ((unsigned)c.cl_iters[cl] >= T) return;
-    }
-    const int k = c.cl_cons[c.cl_cstart[cl]];
-    const int i = c.constr_i[k], j = c.constr_j[k];
-    const double inv_mi = c.inv_mass[i], inv_mj = c.inv_mass[j];
-    double *v = RATTLE ? vel : pos;
-    double xi = v[i], yi = v[n + i], zi = v[2 * n + i];
-    double xj = v[j], yj = v[n + j], zj = v[2 * n + j];
-    const int ncst = c.n_constr;
-    double rx, ry, rz, wq, dsq = 0.0;
-    if (!RATTLE) {
-        dsq = c.constr_dsq[k];
-        rx = c.rvec[k]; ry = c.rvec[ncst + k]; rz = c.rvec[2 * ncst + k];
-        wq = 2.0 * (inv_mi + inv_mj);
-    } else {
-        rx = cdiff(c, pos[i], pos[j], 0);
-        ry = cdiff(c, pos[n + i], pos[n + j], 1);
-        rz = cdiff(c, pos[2 * n + i], pos[2 * n + j], 2);
-        const double rsq = rx * rx + ry * ry + rz * rz;
-        wq = (inv_mi + inv_mj) * rsq;
-    }
-    const bool keep_sum = !RATTLE && c.lam_sum;
-    double acc = 0.0;
-    unsigned it;
-    double mx;
-    int worst;
-    if (!phase2) {
-        it = 0;
-        mx = 0.0;
-        worst = 0;
-        if (!RATTLE && c.lam0) {
-            acc = c.lam0[k];
-            single_apply(acc, inv_mi, inv_mj, rx, ry, rz, xi, yi, zi, xj, yj, zj);
-        }
-    } else {
-        it = (unsigned)c.cl_iters[cl];
-        mx = c.cl_worst[cl];
-        worst = c.cl_worst_idx[cl];
-        if (keep_sum) acc = c.lam_sum[k];
-    }
-    bool ok = false;
-    const unsigned stop = phase2 ? T : c.max_iter;
-    while (it < stop) {
-        double l_;
-        if (RATTLE) {
-            const double dvx = xi - xj;
-            const double dvy = yi - yj;
-            const double dvz = zi - zj;
-            const double rel_vel = dvx * rx + dvy * ry + dvz * rz;
-            l_ = wq == 0.0 ? 0.0 : rel_vel / wq;
-        } else {
-            const double dx = cdiff(c, xi, xj, 0);
-            const double dy = cdiff(c, yi, yj, 1);
-            const double dz = cdiff(c, zi, zj, 2);
-            const double diff = dx * dx + dy * dy + dz * dz - dsq;
-            const double dot_new_old = dx * rx + dy * ry + dz * rz;
-            const double denom = wq * dot_new_old;
-            l_ = denom == 0.0 ? 0.0 : diff / denom;
-            if (keep_sum) acc += l_;
-        }
-        const double la = fabs(l_);
-        mx = 0.0;
-        worst = k;
-        if (la > mx) mx = la;
-        single_apply(l_, inv_mi, inv_mj, rx, ry, rz, xi, yi, zi, xj, yj, zj);
-        it++;
-        if (!phase2 && mx < c.tol) { ok = true; break; }
-    }
-    v[i] = xi; v[n + i] = yi; v[2 * n + i] = zi;
-    v[j] = xj; v[n + j] = yj; v[2 * n + j] = zj;
-    if (keep_sum) c.lam_sum[k] = acc;
-    c.cl_iters[cl] = (int)it;
-    c.cl_worst[cl] = mx;
-    c.cl_worst_idx[cl] = worst;
-    if (!phase2) {
-        if (!ok) {
-            atomicOr(&c.status->error, RATTLE ? (unsigned)GM_DEV_RATTLE_FAIL : (unsigned)GM_DEV_SHAKE_FAIL);
-            atomicMin(&c.status->fail_step, c.status->step);
-        }
-        atomicMax(RATTLE ? &c.status->rattle_T : &c.status->shake_T, it);
-    } else if (!(mx < c.tol) && T < c.max_iter) {
-        atomicOr(&c.status->error, (unsigned)GM_DEV_ITER_MISMATCH);
-    }
-}
-
 // Warm start: one displacement with the predicted multipliers lam0, by the
 // update of a Jacobi sweep (per-atom deltas over the atom's constraints in
 // ascending order from 0.0, then added), before the unchanged iterations.
 // The multiplier totals start from lam0.
-// Clusters come in four ranges, launched with 32-thread blocks:
-// [0, n_single) one constraint, one per thread; [n_single, n_star_end)
-// stars of 2-8 constraints, one per thread; [n_star_end, n_warp_end) other
+// Clusters come in three ranges, launched with 32-thread blocks: stars (a
+// constraint per lane, n_lane_warps blocks), [n_star_end, n_warp_end) other
 // clusters of 2-32 constraints, one per warp; the rest one per thread
 // through global memory.
 struct ClusterBlocks {
-    int single, star, warp, big;
+    int star, warp, big;
 };
 
 __host__ __device__ __forceinline__ ClusterBlocks cluster_block_ranges(const ClusterArgs &c) {
     ClusterBlocks b;
-    b.single = (c.n_single + 31) / 32;
-    b.star = (c.n_star_end - c.n_single + 31) / 32;
+    b.star = c.n_lane_warps;
     b.warp = c.n_warp_end - c.n_star_end;
     b.big = (c.n_clusters - c.n_warp_end + 31) / 32;
     return b;
@@ -705,7 +648,7 @@ __host__ __device__ __forceinline__ ClusterBlocks cluster_block_ranges(const Clu
 
 int cluster_blocks(const ClusterArgs &c) {
     const ClusterBlocks b = cluster_block_ranges(c);
-    return b.single + b.star + b.warp + b.big;
+    return b.star + b.warp + b.big;
 }
 
 // Runs the cluster of this thread (or warp) by its class; false for the
@@ -715,15 +658,8 @@ __device__ __forceinline__ bool cluster_dispatch(const ClusterArgs &c, double *p
                                                  int *cl) {
     const ClusterBlocks b = cluster_block_ranges(c);
     int blk = blockIdx.x;
-    if (blk < b.single) {
-        const int q = blk * 32 + threadIdx.x;
-        if (q < c.n_single) cluster_single<RATTLE>(c, q, pos, vel, n, phase2);
-        return true;
-    }
-    blk -= b.single;
     if (blk < b.star) {
-        const int q = c.n_single + blk * 32 + threadIdx.x;
-        if (q < c.n_star_end) cluster_star_any<RATTLE>(c, q, pos, vel, n, phase2);
+        star_phase<RATTLE>(c, blk, pos, vel, n, phase2);
         return true;
     }
     blk -= b.star;
@@ -739,7 +675,7 @@ __device__ __forceinline__ bool cluster_dispatch(const ClusterArgs &c, double *p
 __global__ void warm_start_apply(ClusterArgs c, double *pos, int n_atoms) {
     // big clusters only: the other paths apply the warm start themselves
     const ClusterBlocks b = cluster_block_ranges(c);
-    const int blk = (int)blockIdx.x - b.single - b.star - b.warp;
+    const int blk = (int)blockIdx.x - b.star - b.warp;
     if (blk < 0) return;
     const int cl = c.n_warp_end + blk * 32 + threadIdx.x;
     if (cl >= c.n_clusters || c.status->error) return;
