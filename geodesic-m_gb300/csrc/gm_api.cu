@@ -105,6 +105,10 @@ struct gm_ctx {
         *d_cl_atoms = nullptr, *d_cl_acstart = nullptr, *d_cl_acons = nullptr, *d_cl_iters = nullptr,
         *d_cl_worst_idx = nullptr;
     double *d_cdsq = nullptr, *d_lam = nullptr, *d_rvec = nullptr, *d_cl_worst = nullptr;
+    int n_free = 0;                // atoms of no constraint
+    int *d_free = nullptr;
+    SolveSync *d_solve = nullptr;  // SHAKE's and RATTLE's words of the fused constrained step
+    int solve_threads = 0, solve_blocks = -1;  // its grid (-1: not looked up; 0: the clusters do not fit it)
     std::vector<int> h_ci, h_cj;
     // constraint warm start (gm_mlp.cu)
     bool ws_on = false, ws_model = false;
@@ -430,6 +434,46 @@ int persistent_grid(gm_ctx *c);
 // too: the phase only evaluates forces.
 bool force_phase(const gm_ctx *c) { return c->step_form == GM_STEP_PERSISTENT && !c->fp64 && c->n > 0; }
 
+// Constrained resident steps run as two cooperative launches around the force
+// evaluation when every cluster is a star, their lanes are resident at once,
+// and no warm start needs the solve's own launches.
+bool fused_solve(gm_ctx *c) {
+    if (!c->n_clusters || c->n_star_end != c->n_clusters || c->ws_on || c->ws_rec_stride > 0) return false;
+    if (c->solve_blocks < 0) gm_solve_step_grid(cluster_args(c), c->n_free, &c->solve_threads, &c->solve_blocks);
+    return c->solve_blocks > 0;
+}
+
+// Before the steps of a call: the barrier and queue words start cleared (a
+// launch that gave up at its barrier leaves them set).
+int begin_constrained(gm_ctx *c) {
+    if (!c->n_clusters) return GM_OK;
+    GM_CUDA(c, cudaMemsetAsync(c->d_solve, 0, 2 * sizeof(SolveSync), c->stream));
+    GM_CUDA(c, cudaMemsetAsync(c->d_sync, 0, sizeof(StepSync), c->stream));
+    return GM_OK;
+}
+
+SolveStepArgs solve_args(gm_ctx *c, double dt, unsigned long long cond, int which) {
+    const double half_skin = (c->p.r_skin - c->p.r_cutoff) / 2.0;  // neighbor.rs:61-62
+    SolveStepArgs a{};
+    a.n = c->n;
+    a.n_free = c->n_free;
+    a.free_atoms = c->d_free;
+    a.pos = c->d_pos;
+    a.vel = c->d_vel;
+    a.dref = c->d_dref;
+    a.force = c->d_force;
+    a.ref = c->d_ref;
+    a.dt_half = dt / 2.0;
+    a.dt = dt;
+    a.inv_dt = 1.0 / dt;
+    a.thr_sq = half_skin * half_skin;
+    a.cond = cond;
+    a.atom_sys = c->d_atom_sys;
+    a.sys_flag = c->d_sys_flag;
+    a.sync = c->d_solve + which;
+    return a;
+}
+
 // Force evaluation at the resident positions: the persistent kernel's force
 // phase (force_phase), or the pair kernel with the bonded and 1-4 kernels.
 // With a branch stream those run on it beside the pair kernel: every force
@@ -447,7 +491,8 @@ int seq_forces(gm_ctx *c, cudaStream_t s, bool energy = true, cudaStream_t branc
         // / 1-4 blocks from one queue, one launch, the same sums and energy
         // partials as the kernels below; the queue words start cleared (a
         // step launch that gave up at its barrier leaves them set)
-        cudaMemsetAsync(c->d_sync, 0, sizeof(StepSync), s);
+        // (a constrained step's are cleared at the start of its call)
+        if (!(packed && c->n_clusters)) cudaMemsetAsync(c->d_sync, 0, sizeof(StepSync), s);
         gm_launch_forces_persistent(fa, c->d_sync, c->persist_blocks, s);
         if (energy) gm_launch_energy(fa, s);
         c->energy_stale = !energy;
@@ -807,6 +852,12 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
         *count += 1;
         return GM_OK;
     }
+    if (fused_solve(c)) {
+        gm_launch_shake_step(cluster_args(c), solve_args(c, dt, cond, 0), pack_args(c), c->solve_threads,
+                             c->solve_blocks, s);
+        *count += 1;
+        return GM_OK;
+    }
     gm_launch_half_kick(n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, s); k++;
     gm_launch_drift(n, c->d_pos, c->d_vel, c->d_dref, dt, false, c->d_status, s); k++;
     k += issue_shake(c, s, true);
@@ -820,8 +871,12 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
 
 int issue_step_tail(gm_ctx *c, cudaStream_t s, double dt, long long *count) {
     if (persistent_form(c)) return GM_OK;  // the next launch evaluates the forces
-    long long k = seq_forces(c, s, false, c->side, c->n_clusters == 0);
-    if (c->n_clusters) {
+    const bool fused = fused_solve(c);
+    long long k = seq_forces(c, s, false, c->side, c->n_clusters == 0 || fused);
+    if (fused) {
+        gm_launch_rattle_step(cluster_args(c), solve_args(c, dt, 0ull, 1), c->solve_threads, c->solve_blocks, s);
+        k++;
+    } else if (c->n_clusters) {
         gm_launch_half_kick(c->n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, s); k++;
         gm_launch_rattle(cluster_args(c), c->n, c->d_pos, c->d_vel, s); k += 3;
         gm_launch_step(c->d_status, s); k++;
@@ -908,7 +963,7 @@ int run_direct(gm_ctx *c, double dt, int64_t n_steps);
 // rest of the call evaluates forces and the closing half-kick).
 int launch_loop(gm_ctx *c, double dt, int64_t n_steps) {
     const bool pf = persistent_form(c) && n_steps > 0;
-    int rc = pf ? begin_persistent(c, true) : GM_OK;
+    int rc = pf ? begin_persistent(c, true) : begin_constrained(c);
     if (rc) return rc;
     if (!c->use_graph) {
         rc = run_direct(c, dt, n_steps);
@@ -1550,6 +1605,17 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
                 w[(size_t)k] = (float)inv_mass[(size_t)c->h_ci[(size_t)k]] + (float)inv_mass[(size_t)c->h_cj[(size_t)k]];
             TRY(dupload(c, &c->d_ws_w, w.data(), w.size()));
         }
+        {
+            std::vector<char> held((size_t)n, 0);
+            for (int k = 0; k < c->n_constr; k++) held[(size_t)c->h_ci[(size_t)k]] = held[(size_t)c->h_cj[(size_t)k]] = 1;
+            std::vector<int> free_atoms;
+            for (int i = 0; i < n; i++)
+                if (!held[(size_t)i]) free_atoms.push_back(i);
+            c->n_free = (int)free_atoms.size();
+            TRY(dupload(c, &c->d_free, free_atoms.data(), free_atoms.size()));
+            TRY(dalloc(c, &c->d_solve, 2));
+            if (cudaMemset(c->d_solve, 0, 2 * sizeof(SolveSync)) != cudaSuccess) return bail(GM_ERR_DEVICE);
+        }
         TRY(dalloc(c, &c->d_rvec, 3 * (size_t)c->n_constr));
         TRY(dalloc(c, &c->d_cl_iters, (size_t)c->n_clusters));
         TRY(dalloc(c, &c->d_cl_worst, (size_t)c->n_clusters));
@@ -1932,6 +1998,10 @@ int32_t gm_profile(gm_ctx *c, int32_t which, int32_t n_iter, double dt, double *
     ForceArgs fa = force_args(c);
     ListArgs la = list_args(c);
     const bool pf = which == 3 && persistent_form(c);
+    if (which == 3 && !pf) {
+        rc = begin_constrained(c);
+        if (rc) return rc;
+    }
     for (int k = 0; k < n_iter; k++) {
         if (pf) {
             rc = begin_persistent(c, false);  // the timed launch evaluates its forces
@@ -2017,7 +2087,7 @@ int32_t gm_time_steps(gm_ctx *c, double dt, uint64_t first_step, int64_t n_steps
     if (!rc && c->use_graph) rc = capture_graph(c, dt);
     // every timed persistent launch evaluates its forces
     const bool pf = persistent_form(c);
-    if (!rc && pf) rc = begin_persistent(c, false);
+    if (!rc) rc = pf ? begin_persistent(c, false) : begin_constrained(c);
     if (rc) return rc;
     std::vector<cudaEvent_t> ev((size_t)(2 * n_steps));
     for (auto &e : ev) GM_CUDA(c, cudaEventCreate(&e));

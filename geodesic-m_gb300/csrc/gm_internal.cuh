@@ -185,6 +185,48 @@ __device__ __forceinline__ void gm_pack_record(float4 *rec, double ox, double oy
     rec[1] = make_float4((float)(ox - (double)hx), (float)(oy - (double)hy), (float)(oz - (double)hz), qw.y);
 }
 
+__device__ __forceinline__ unsigned gm_ld_acquire(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// ~64 ns per poll: about a quarter of a second before a block gives up
+constexpr unsigned GM_BARRIER_POLLS = 1u << 22;
+
+// Grid-wide barrier of a cooperative launch (every block is resident).  The
+// generation is read before arriving, the last block to arrive resets the
+// count and advances the generation.  Returns false (and records the
+// timeout) when the generation did not advance within GM_BARRIER_POLLS polls.
+// All threads of the block call.
+__device__ __forceinline__ bool gm_grid_barrier(unsigned *arrive, unsigned *gen, DevStatus *st) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        const unsigned g = gm_ld_acquire(gen);
+        __threadfence();
+        if (atomicAdd(arrive, 1u) == gridDim.x - 1) {
+            atomicExch(arrive, 0u);
+            __threadfence();
+            atomicAdd(gen, 1u);
+        } else {
+            for (unsigned it = 0; gm_ld_acquire(gen) == g; it++) {
+                if (it >= GM_BARRIER_POLLS) {
+                    atomicOr(&st->error, (unsigned)GM_DEV_BARRIER_TIMEOUT);
+                    ok = 0;
+                    break;
+                }
+                __nanosleep(64);
+            }
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
 // ------------------------------------------------------- launcher exports
 
 struct ListArgs {
@@ -385,6 +427,33 @@ struct StepArgs {
     unsigned int *sys_flag;
     StepSync *sync;
 };
+// The constrained step's two cooperative kernels (star clusters only):
+//   shake: half-kick, drift, SHAKE, velocity resync, rebuild check, pack;
+//   rattle: half-kick, RATTLE, the step count.
+// Both phases of a solve run in one launch with a grid barrier between them.
+struct SolveSync {
+    unsigned int arrive, gen;  // grid barrier
+    unsigned int T;            // largest iteration count of phase 1
+    unsigned int fail;         // a cluster of phase 1 did not converge
+};
+struct SolveStepArgs {
+    int n, n_free;
+    const int *free_atoms;     // atoms of no constraint
+    double *pos, *vel, *dref;
+    long long *force;
+    const double *ref;
+    double dt_half, dt, inv_dt, thr_sq;
+    unsigned long long cond;
+    const int *atom_sys;
+    unsigned int *sys_flag;
+    SolveSync *sync;
+};
+// Threads per block and blocks (all co-resident) of both kernels; blocks 0
+// when the system's clusters do not fit.
+void gm_solve_step_grid(const ClusterArgs &c, int n_free, int *threads, int *blocks);
+void gm_launch_shake_step(const ClusterArgs &c, const SolveStepArgs &sa, const PackArgs &pk, int threads, int blocks,
+                          cudaStream_t s);
+void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int threads, int blocks, cudaStream_t s);
 // Blocks of the cooperative grid (all co-resident, no more than the work
 // items and atoms fill); 0 when the form does not apply.
 int gm_step_persistent_blocks(const ForceArgs &fa);

@@ -37,47 +37,6 @@ namespace {
 
 constexpr int kStepThreads = 128;
 constexpr int kStepMinBlocks = 6;  // 24 warps per SM: at most 80 registers a thread
-// ~64 ns per poll: about a quarter of a second before a block gives up
-constexpr unsigned kBarrierPolls = 1u << 22;
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid-wide barrier of a cooperative launch (every block is resident).  The
-// generation is read before arriving, the last block to arrive resets the
-// count and advances the generation.  Returns false (and records the
-// timeout) when the generation did not advance within kBarrierPolls polls.
-__device__ bool grid_barrier(StepSync *sy, DevStatus *st) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned g = ld_acquire(&sy->gen);
-        __threadfence();
-        if (atomicAdd(&sy->arrive, 1u) == gridDim.x - 1) {
-            atomicExch(&sy->arrive, 0u);
-            __threadfence();
-            atomicAdd(&sy->gen, 1u);
-        } else {
-            for (unsigned it = 0; ld_acquire(&sy->gen) == g; it++) {
-                if (it >= kBarrierPolls) {
-                    atomicOr(&st->error, (unsigned)GM_DEV_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 // A 64-term block of bonded terms (or 1-4 pairs) by one warp, two terms a
 // lane, with the energy partial and the per-system energies of term_block
 // (gm_force.cu): lane l holds terms l and l + 32, and the shuffle-down tree
@@ -184,10 +143,10 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
         return;
     }
     // ---- 2. every force is summed
-    if (!grid_barrier(sy, st)) return;
+    if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
     // ---- 3. kick, drift, pack, rebuild check (kick_drift_check_kernel's
     // operations, one atom at a time)
-    const bool err0 = ld_acquire(&st->error) != 0, tail0 = ld_acquire(&st->tail_pending) != 0;
+    const bool err0 = gm_ld_acquire(&st->error) != 0, tail0 = gm_ld_acquire(&st->tail_pending) != 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sy->ticket = 0;
         sy->fresh = 0;
