@@ -1712,7 +1712,10 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         int dev_sms = 0;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device);
         const int warps = 24 * std::max(dev_sms, 1);
-        c->split = std::max(1, std::min(GM_MAX_SPLIT, (8 * warps + c->n_groups - 1) / std::max(c->n_groups, 1)));
+        // The FP64 pair kernel is no queue and waits for one pipe: two items
+        // per warp (5,000 atoms: 1.54 ms for five steps, 1.90 with eight).
+        const int want = (c->fp64 ? 2 : 8) * warps, most = c->fp64 ? GM_SET_SPLIT : GM_MAX_SPLIT;
+        c->split = std::max(1, std::min(most, (want + c->n_groups - 1) / std::max(c->n_groups, 1)));
         const long long terms = (long long)c->n_bonds + c->n_angles + c->n_diheds + c->n14;
         c->term_chunk = terms > 32ll * warps ? 128 : 32;
     }
