@@ -12,6 +12,13 @@
  *            FMA, and RN(q + r y) is the correctly rounded quotient when y is
  *            the correctly rounded reciprocal (away from overflow and
  *            underflow).  Three FP64 operations instead of a division.
+ * gm_div_rcp: num / den correctly rounded from y = RN(1 / den), the same
+ *            correction for any den of ordinary size (2^-200 to 2^200, the
+ *            caller's to see); a numerator that is zero, tiny or huge takes
+ *            the division.
+ * gm_abs_ge: |v| >= t for a positive finite t, by integer comparison of the
+ *            bits (an FP64 comparison occupies the FP64 pipe like any other
+ *            FP64 instruction); false for a NaN.
  * gm_min_image: d - L round(d / L), round half away from zero, each operation
  *            rounded on its own: the reference's min_image
  *            (neighbor.rs:74-76).  Away from |d| = L/2 the rounded quotient
@@ -68,6 +75,34 @@ GM_HD int gm_hi_word(double v) {
 #endif
 }
 
+GM_HD double gm_div_by_dt(double num, double dt, double y) {
+    const double q = num * y;
+    const double r = fma(-q, dt, num);
+    return fma(r, y, q);
+}
+
+GM_HD int gm_ordinary(double v) { /* 2^-200 to 2^200 */
+    return (unsigned)((gm_hi_word(v) & 0x7fffffff) - ((1023 - 200) << 20)) < (unsigned)(400 << 20);
+}
+
+GM_HD double gm_div_rcp(double num, double den, double y) {
+    /* |num| in [2^-700, 2^700) */
+    if ((unsigned)((gm_hi_word(num) & 0x7fffffff) - ((1023 - 700) << 20)) >= (unsigned)(1400 << 20)) return num / den;
+    return gm_div_by_dt(num, den, y);
+}
+
+GM_HD int gm_abs_ge(double v, double t) {
+#ifdef __CUDA_ARCH__
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), tb = (unsigned long long)__double_as_longlong(t);
+#else
+    unsigned long long b, tb;
+    memcpy(&b, &v, sizeof b);
+    memcpy(&tb, &t, sizeof tb);
+#endif
+    const unsigned long long a = b & 0x7fffffffffffffffull;
+    return a >= tb && a <= 0x7ff0000000000000ull;
+}
+
 GM_HD double gm_min_image(double d, double L) {
     const int hd = gm_hi_word(d) & 0x7fffffff, hl = gm_hi_word(L);
     if (hd < hl - 0x101000) return d; /* |d| < L/2 (1 - 2^-8) */
@@ -80,10 +115,5 @@ GM_HD double gm_min_image(double d, double L) {
 #endif
 }
 
-GM_HD double gm_div_by_dt(double num, double dt, double y) {
-    const double q = num * y;
-    const double r = fma(-q, dt, num);
-    return fma(r, y, q);
-}
 
 #endif

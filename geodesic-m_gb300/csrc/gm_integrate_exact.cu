@@ -223,8 +223,11 @@ __global__ void shake_prepare(ClusterArgs c, const double *dref, int n_atoms) {
 // from 0.0).  Differences are taken centre minus H whichever atom is the
 // constraint's i: both signs flip in every product, so the values are the
 // same bits.
-// An iteration is one serial chain of ~25 FP64 operations (a division among
-// them) whatever the star's size.  With a thread per star it was that for every
+// An iteration is one serial chain of FP64 operations whatever the star's
+// size, ~50 cycles each on this part, so what need not be FP64 is not: the
+// convergence and zero tests compare bits, RATTLE's division by its constant
+// denominator is three operations from the reciprocal, and the centre's sum
+// starts from the first term.  With a thread per star it was that for every
 // constraint of the star, and the one warp holding the four-H stars of a
 // 20,011-atom chain ran 113 us while every other was done in 20.
 struct StarLane {
@@ -232,6 +235,7 @@ struct StarLane {
     double cx, cy, cz, hx, hy, hz;  // SHAKE: positions; RATTLE: velocities
     double rx, ry, rz;           // reference (SHAKE) or current (RATTLE) vector, centre - H
     double inv_c, inv_h, wq, dsq;
+    double rcp;                  // RATTLE: 1 / wq (0 where wq is not of ordinary size)
     double lam, acc;             // the last multiplier; the total (keep_sum)
     unsigned it;                 // iterations done (alike over the group)
     bool ok;                     // converged in phase 1
@@ -257,12 +261,16 @@ __device__ __forceinline__ void lane_apply(StarLane &s, const LaneGroup &g, bool
     const unsigned full = 0xffffffffu;
     const double w = s.lam * s.inv_c;
     const double tx = w * s.rx, ty = w * s.ry, tz = w * s.rz;
-    double ddx = 0.0, ddy = 0.0, ddz = 0.0;
+    // 0.0 - t_0 - t_1 - ..., the first difference as a negation (a lane past
+    // the star's last sends 0)
+    double ddx, ddy, ddz;
     if (g.width == 1) {
-        ddx -= tx; ddy -= ty; ddz -= tz;
+        ddx = -tx; ddy = -ty; ddz = -tz;
     } else {
-        for (int q = 0; q < g.width; q++) {
-            // a lane past the star's last sends 0
+        ddx = -__shfl_sync(full, tx, g.base);
+        ddy = -__shfl_sync(full, ty, g.base);
+        ddz = -__shfl_sync(full, tz, g.base);
+        for (int q = 1; q < g.width; q++) {
             ddx -= __shfl_sync(full, tx, g.base + q);
             ddy -= __shfl_sync(full, ty, g.base + q);
             ddz -= __shfl_sync(full, tz, g.base + q);
@@ -292,11 +300,12 @@ __device__ __forceinline__ void lane_iterate(const ClusterArgs &c, StarLane &s, 
             const double dz = RATTLE ? s.cz - s.hz : cdiff(c, s.cz, s.hz, 2);
             const double dot = dx * s.rx + dy * s.ry + dz * s.rz;
             if (RATTLE) {
-                l = s.wq == 0.0 ? 0.0 : dot / s.wq;
+                if (s.rcp != 0.0) l = gm_div_rcp(dot, s.wq, s.rcp);
+                else l = s.wq == 0.0 ? 0.0 : dot / s.wq;
             } else {
                 const double diff = dx * dx + dy * dy + dz * dz - s.dsq;
                 const double denom = s.wq * dot;
-                l = denom == 0.0 ? 0.0 : diff / denom;
+                l = (__double_as_longlong(denom) << 1) == 0 ? 0.0 : diff / denom;
             }
         }
         if (run) {
@@ -306,7 +315,7 @@ __device__ __forceinline__ void lane_iterate(const ClusterArgs &c, StarLane &s, 
         lane_apply(s, g, run);
         // max |lambda| < tol over the group; a NaN counts as 0, as in the
         // sequential sweep's strict comparison
-        const unsigned small = __ballot_sync(full, !(fabs(l) >= c.tol));
+        const unsigned small = __ballot_sync(full, !gm_abs_ge(l, c.tol));
         if (run) {
             s.it++;
             if (phase1) s.ok = (small & g.mask) == g.mask;
@@ -321,7 +330,7 @@ __device__ __forceinline__ void lane_constants(const ClusterArgs &c, int warp, S
     const int4 t = c.lanes[warp * 32 + (threadIdx.x & 31)];
     s.cen = t.x; s.h = t.y; s.k = t.z; s.cl = t.w;
     s.cx = s.cy = s.cz = s.hx = s.hy = s.hz = 0.0;
-    s.rx = s.ry = s.rz = s.inv_c = s.inv_h = s.wq = s.dsq = 0.0;
+    s.rx = s.ry = s.rz = s.inv_c = s.inv_h = s.wq = s.dsq = s.rcp = 0.0;
     s.lam = s.acc = 0.0;
     s.it = 0;
     s.ok = false;
@@ -343,6 +352,7 @@ __device__ __forceinline__ void lane_bond(const ClusterArgs &c, const double *po
     s.rz = cdiff(c, pos[2 * n + s.cen], pos[2 * n + s.h], 2);
     const double rsq = s.rx * s.rx + s.ry * s.ry + s.rz * s.rz;
     s.wq = (s.inv_c + s.inv_h) * rsq;
+    s.rcp = gm_ordinary(s.wq) ? 1.0 / s.wq : 0.0;
 }
 
 // The worst constraint of the group's last iteration (the first in ascending
