@@ -83,6 +83,9 @@ struct gm_ctx {
     int term_chunk = 128;            // bonded terms per work item of the persistent kernel
     int pair_warps = 4, pair_grid = 0;  // FP32 pair kernel block size and grid (0: one item per warp)
     int *d_list = nullptr, *d_count = nullptr, *d_gmax = nullptr, *d_stage = nullptr;
+    int *d_count_in = nullptr, *d_gmax_in = nullptr;  // without the last distance bucket
+    unsigned int *d_sys_far = nullptr;                // see ForceArgs::sys_far
+    bool far_marked = false;                          // every system is marked far
     bool built = false;
     // exclusions
     int *d_excl_start = nullptr, *d_excl = nullptr;
@@ -246,6 +249,9 @@ ListArgs list_args(gm_ctx *c) {
     a.list = c->d_list;
     a.count = c->d_count;
     a.gmax = c->d_gmax;
+    a.count_in = c->d_count_in;
+    a.gmax_in = c->d_gmax_in;
+    a.sys_far = c->d_sys_far;
     a.ref = c->d_ref;
     a.force = c->d_force;
     a.grid = c->d_grid;
@@ -265,6 +271,14 @@ ListArgs list_args(gm_ctx *c) {
     a.group_sys = c->d_group_sys;
     a.sys_flag = c->d_sys_flag;
     return a;
+}
+
+// Squared displacement up to which a system's outer list bucket cannot reach
+// the cutoff: pairs beyond half the skin at the build (bucket bound rounded in
+// FP32) need two atoms to move a quarter of it each; 1e-3 A covers the rounding.
+double far_sq(const gm_ctx *c) {
+    const double d = std::max((c->p.r_skin - c->p.r_cutoff) / 4.0 - 1e-3, 0.0);
+    return d * d;
 }
 
 // periodic && bonded_min_image: bonded, 1-4 and constraint differences at the
@@ -291,6 +305,9 @@ ForceArgs force_args(gm_ctx *c) {
     a.list = c->d_list;
     a.count = c->d_count;
     a.gmax = c->d_gmax;
+    a.count_in = c->d_count_in;
+    a.gmax_in = c->d_gmax_in;
+    a.sys_far = c->d_sys_far;
     a.ntypes = c->ntypes;
     a.tab32 = c->d_tab32;
     a.tab64 = c->d_tab64;
@@ -467,9 +484,11 @@ SolveStepArgs solve_args(gm_ctx *c, double dt, unsigned long long cond, int whic
     a.dt = dt;
     a.inv_dt = 1.0 / dt;
     a.thr_sq = half_skin * half_skin;
+    a.far_sq = far_sq(c);
     a.cond = cond;
     a.atom_sys = c->d_atom_sys;
     a.sys_flag = c->d_sys_flag;
+    a.sys_far = c->d_sys_far;
     a.sync = c->d_solve + which;
     return a;
 }
@@ -710,6 +729,7 @@ int do_build(gm_ctx *c, bool all = true) {
         if (rc) return rc;
         if (attempt == 0) r0 = c->h_status->n_rebuilds;
         c->launches += seq_rebuild(c, c->stream, all || attempt > 0);
+        c->far_marked = false;
         rc = check_status(c, nullptr);
         if (attempt == 0) counted = c->h_status->n_rebuilds - r0;
         // the build records the longest list and staged layer it met: on an
@@ -837,9 +857,11 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
         sa.dt = dt;
         sa.inv_dt = 1.0 / dt;
         sa.thr_sq = half_skin * half_skin;
+        sa.far_sq = far_sq(c);
         sa.cond = cond;
         sa.atom_sys = c->d_atom_sys;
         sa.sys_flag = c->d_sys_flag;
+        sa.sys_far = c->d_sys_far;
         sa.sync = c->d_sync;
         gm_launch_step_persistent(force_args(c), sa, pack_args(c), c->persist_blocks, s);
         *count += 1;
@@ -847,8 +869,8 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
     }
     if (!constrained) {
         gm_launch_kick_drift_check(n, c->d_pos, c->d_vel, c->d_dref, c->d_force, c->d_inv_mass, dt / 2.0, dt, c->d_ref,
-                                   half_skin * half_skin, c->d_status, cond, c->d_atom_sys, c->d_sys_flag,
-                                   pack_args(c), s);
+                                   half_skin * half_skin, far_sq(c), c->d_status, cond, c->d_atom_sys, c->d_sys_flag,
+                                   c->d_sys_far, pack_args(c), s);
         *count += 1;
         return GM_OK;
     }
@@ -862,8 +884,8 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
     gm_launch_drift(n, c->d_pos, c->d_vel, c->d_dref, dt, false, c->d_status, s); k++;
     k += issue_shake(c, s, true);
     gm_launch_resync(n, c->d_pos, c->d_vel, c->d_dref, dt, c->d_status, s); k++;
-    gm_launch_check(n, c->d_pos, c->d_ref, half_skin * half_skin, c->d_status, cond, gm_check_blocks(n), c->d_atom_sys,
-                    c->d_sys_flag, s);
+    gm_launch_check(n, c->d_pos, c->d_ref, half_skin * half_skin, far_sq(c), c->d_status, cond, gm_check_blocks(n),
+                    c->d_atom_sys, c->d_sys_flag, c->d_sys_far, s);
     k++;
     *count += k;
     return GM_OK;
@@ -962,6 +984,7 @@ int run_direct(gm_ctx *c, double dt, int64_t n_steps);
 // The steps themselves: after them the resident positions are final (the
 // rest of the call evaluates forces and the closing half-kick).
 int launch_loop(gm_ctx *c, double dt, int64_t n_steps) {
+    c->far_marked = false;  // a step may rebuild
     const bool pf = persistent_form(c) && n_steps > 0;
     int rc = pf ? begin_persistent(c, true) : begin_constrained(c);
     if (rc) return rc;
@@ -1043,9 +1066,8 @@ int ensure_forces(gm_ctx *c) {
         int rc = reset_status(c);
         if (rc) return rc;
         const double half_skin = (c->p.r_skin - c->p.r_cutoff) / 2.0;
-        gm_launch_check(c->n, c->d_pos, c->d_ref, half_skin * half_skin, c->d_status, 0ull, gm_check_blocks(c->n),
-                        c->d_atom_sys, c->d_sys_flag,
-                        c->stream);
+        gm_launch_check(c->n, c->d_pos, c->d_ref, half_skin * half_skin, far_sq(c), c->d_status, 0ull,
+                        gm_check_blocks(c->n), c->d_atom_sys, c->d_sys_flag, c->d_sys_far, c->stream);
         c->launches++;
         rc = st_read(c);
         if (rc) return rc;
@@ -1670,6 +1692,8 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         TRY(dupload(c, &c->d_atom_sys, atom_sys.data(), atom_sys.size()));
         TRY(dupload(c, &c->d_group_sys, group_sys.data(), group_sys.size()));
         TRY(dalloc(c, &c->d_sys_flag, (size_t)n_sys));
+        TRY(dalloc(c, &c->d_sys_far, (size_t)n_sys));
+        cudaMemset(c->d_sys_far, 0xFF, sizeof(unsigned int) * (size_t)n_sys);
         TRY(dalloc(c, &c->d_e_sys, (size_t)n_sys));
         cudaMemset(c->d_sys_flag, 0, sizeof(unsigned int) * (size_t)n_sys);
         cudaMemset(c->d_e_sys, 0, sizeof(long long) * (size_t)n_sys);
@@ -1701,6 +1725,10 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
     cudaMemset(c->d_count, 0, sizeof(int) * ns_);  // padding slots keep count 0
     TRY(dalloc(c, &c->d_gmax, (size_t)c->n_groups));
     cudaMemset(c->d_gmax, 0, sizeof(int) * (size_t)c->n_groups);
+    TRY(dalloc(c, &c->d_count_in, ns_));
+    cudaMemset(c->d_count_in, 0, sizeof(int) * ns_);
+    TRY(dalloc(c, &c->d_gmax_in, (size_t)c->n_groups));
+    cudaMemset(c->d_gmax_in, 0, sizeof(int) * (size_t)c->n_groups);
     c->n_epart = c->n_groups * GM_MAX_SPLIT + c->bonded_blocks + c->blocks14;
     {
         // about eight work items per resident warp (24 per SM), so that the
@@ -1720,7 +1748,8 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         c->term_chunk = terms > 32ll * warps ? 128 : 32;
     }
     TRY(dalloc(c, &c->d_epart, (size_t)c->n_epart));
-    TRY(dalloc(c, &c->d_energy, 1));
+    TRY(dalloc(c, &c->d_energy, 2 + GM_SUM_BLOCKS));
+    if (cudaMemset(c->d_energy, 0, sizeof(double) * (2 + GM_SUM_BLOCKS)) != cudaSuccess) return bail(GM_ERR_DEVICE);
     TRY(dalloc(c, &c->d_kin_part, 256));
     TRY(dalloc(c, &c->d_ke, 1));
     TRY(dalloc(c, &c->d_status, 1));
@@ -1812,6 +1841,13 @@ int32_t gm_compute_forces(gm_ctx *c, const double *px, const double *py, const d
     if (rc) return poison(rc);
     rc = reset_status(c);
     if (rc) return poison(rc);
+    if (!c->far_marked) {
+        // nothing has compared these positions with the build's: whole columns
+        // until the next build
+        const cudaError_t e = cudaMemsetAsync(c->d_sys_far, 0xFF, sizeof(unsigned int) * (size_t)c->n_sys, c->stream);
+        if (e != cudaSuccess) return poison(cuda_status(c, e, "cudaMemsetAsync"));
+        c->far_marked = true;
+    }
     c->launches += seq_forces(c, c->stream);
     gm_launch_forces_out(c->n, c->d_force, c->d_fout, c->stream);
     c->launches++;
@@ -1835,8 +1871,8 @@ int32_t gm_needs_rebuild(gm_ctx *c, const double *px, const double *py, const do
     rc = reset_status(c);
     if (rc) return rc;
     const double half_skin = (c->p.r_skin - c->p.r_cutoff) / 2.0;
-    gm_launch_check(c->n, c->d_pos, c->d_ref, half_skin * half_skin, c->d_status, 0ull, gm_check_blocks(c->n),
-                    c->d_atom_sys, c->d_sys_flag, c->stream);
+    gm_launch_check(c->n, c->d_pos, c->d_ref, half_skin * half_skin, far_sq(c), c->d_status, 0ull,
+                    gm_check_blocks(c->n), c->d_atom_sys, c->d_sys_flag, c->d_sys_far, c->stream);
     rc = st_read(c);
     if (rc) return rc;
     *result = c->h_status->rebuild ? 1 : 0;
@@ -2001,6 +2037,7 @@ int32_t gm_profile(gm_ctx *c, int32_t which, int32_t n_iter, double dt, double *
     ForceArgs fa = force_args(c);
     ListArgs la = list_args(c);
     const bool pf = which == 3 && persistent_form(c);
+    c->far_marked = false;
     if (which == 3 && !pf) {
         rc = begin_constrained(c);
         if (rc) return rc;
@@ -2092,6 +2129,7 @@ int32_t gm_time_steps(gm_ctx *c, double dt, uint64_t first_step, int64_t n_steps
     const bool pf = persistent_form(c);
     if (!rc) rc = pf ? begin_persistent(c, false) : begin_constrained(c);
     if (rc) return rc;
+    c->far_marked = false;
     std::vector<cudaEvent_t> ev((size_t)(2 * n_steps));
     for (auto &e : ev) GM_CUDA(c, cudaEventCreate(&e));
     if (flush_buf && flush_bytes > 0)
@@ -2421,7 +2459,7 @@ int32_t gm_frames_enable(gm_ctx *c, int32_t frame_interval, int32_t capacity) {
         int rc = dalloc(c, &c->d_frame_xyz, (size_t)capacity * 3 * (size_t)std::max(c->n, 1));
         if (!rc) rc = dalloc(c, &c->d_frame_step, (size_t)capacity);
         if (!rc) rc = dalloc(c, &c->d_frame_energy, 2 * (size_t)capacity);
-        if (!rc) rc = dalloc(c, &c->d_frame_part, (size_t)GM_FRAME_BLOCKS);
+        if (!rc) rc = dalloc(c, &c->d_frame_part, 2 * (size_t)GM_FRAME_BLOCKS);
         if (rc) return rc;
         c->frame_interval = frame_interval;
         c->frame_cap = capacity;

@@ -27,7 +27,8 @@ template <bool PERIODIC, bool COULOMB, bool BATCH, int W>
 __global__ void __launch_bounds__(W * 32)
 pair_kernel_mixed(int n, int n_slots, int cap, int split, const float4 *__restrict__ coord,
                   const int *__restrict__ perm, const int *__restrict__ list, const int *__restrict__ count,
-                  const int *__restrict__ gmax, int ntypes, const float4 *__restrict__ tab, PairConst k,
+                  const int *__restrict__ gmax, const int *__restrict__ count_in, const int *__restrict__ gmax_in,
+                  const unsigned *__restrict__ sys_far, int ntypes, const float4 *__restrict__ tab, PairConst k,
                   long long *__restrict__ force, double *__restrict__ epart, DevStatus *st,
                   const int *__restrict__ group_sys, long long *e_sys) {
     extern __shared__ float4 s_tab[];
@@ -38,8 +39,8 @@ pair_kernel_mixed(int n, int n_slots, int cap, int split, const float4 *__restri
     const int lane = threadIdx.x & 31;
     const int n_work = (n_slots / 32) * split;
     for (int wid = blockIdx.x * W + (threadIdx.x >> 5); wid < n_work; wid += gridDim.x * W)
-        pair_item_mixed<PERIODIC, COULOMB, BATCH>(wid, lane, n, cap, split, coord, perm, list, count, gmax, ntypes,
-                                                  tab, s_tab, k, force, epart, st, group_sys, e_sys);
+        pair_item_mixed<PERIODIC, COULOMB, BATCH>(wid, lane, n, cap, split, coord, perm, list, count, gmax, count_in,
+                                                  gmax_in, sys_far, ntypes, tab, s_tab, k, force, epart, st, group_sys, e_sys);
 }
 
 // 1/sqrt(x) in FP64 from the MUFU seed: the seed's argument is x truncated to
@@ -225,12 +226,27 @@ __global__ void __launch_bounds__(GM_BONDED_THREADS) bonded_pair14_kernel(ForceA
     }
 }
 
-// Fixed-order sum of all energy partials (pair groups, bonded blocks, 1-4
+// Fixed-order sum of all energy partials (pair items, bonded blocks, 1-4
 // blocks) into the FP64 total: deterministic for a given launch shape.
 __global__ void __launch_bounds__(256) energy_kernel(const double *epart, int n, double *out) {
     __shared__ double s[256];
-    const double e = gm_block_sum256(epart, n, s);
-    if (threadIdx.x == 0) *out = e;
+    __shared__ bool last;
+    double *part = out + 1;
+    unsigned *arrived = reinterpret_cast<unsigned *>(part + GM_SUM_BLOCKS);
+    const double mine = gm_share_sum256(epart, n, s);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = mine;
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const double e = gm_blocks_sum256(part, s);
+    if (threadIdx.x == 0) {
+        *out = e;
+        *arrived = 0u;
+    }
 }
 
 }  // namespace
@@ -254,7 +270,8 @@ void gm_launch_pair(const ForceArgs &a, bool fp64, cudaStream_t s) {
         const size_t smem = gtab ? 0 : tab_bytes;
 #define GM_PAIRMW(P, Q, B, WW)                                                                              \
     pair_kernel_mixed<P, Q, B, WW><<<blocks32, WW * 32, smem, s>>>(                                          \
-        a.n, a.n_slots, a.cap, a.split, a.coord, a.perm, a.list, a.count, a.gmax, a.ntypes, a.tab32, a.pc,    \
+        a.n, a.n_slots, a.cap, a.split, a.coord, a.perm, a.list, a.count, a.gmax, a.count_in, a.gmax_in,      \
+        a.sys_far, a.ntypes, a.tab32, a.pc,                                                                    \
         a.force, a.epart, a.status, a.group_sys, a.e_sys)
 #define GM_PAIRM(P, Q, B) { if (W == 2) GM_PAIRMW(P, Q, B, 2); else if (W == 8) GM_PAIRMW(P, Q, B, 8); \
                             else GM_PAIRMW(P, Q, B, 4); }
@@ -336,5 +353,5 @@ void gm_launch_pair14(const ForceArgs &a, bool, cudaStream_t s) {
 }
 
 void gm_launch_energy(const ForceArgs &a, cudaStream_t s) {
-    energy_kernel<<<1, 256, 0, s>>>(a.epart, a.n_epart_total, a.energy);
+    energy_kernel<<<GM_SUM_BLOCKS, 256, 0, s>>>(a.epart, a.n_epart_total, a.energy);
 }

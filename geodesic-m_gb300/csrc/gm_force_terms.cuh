@@ -82,12 +82,15 @@ template <bool PERIODIC, bool COULOMB, bool BATCH, bool ENERGY = true>
 __device__ __forceinline__ void
 pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__restrict__ coord,
                 const int *__restrict__ perm, const int *__restrict__ list, const int *__restrict__ count,
-                const int *__restrict__ gmax, int ntypes, const float4 *__restrict__ tab, const float4 *s_tab,
+                const int *__restrict__ gmax, const int *__restrict__ count_in, const int *__restrict__ gmax_in,
+                const unsigned *__restrict__ sys_far, int ntypes, const float4 *__restrict__ tab, const float4 *s_tab,
                 const PairConst &k, long long *__restrict__ force, double *__restrict__ epart, DevStatus *st,
                 const int *__restrict__ group_sys, long long *e_sys) {
     const unsigned full = 0xffffffffu;
     const int group = wid / split, part = wid - group * split;
-    const int gm = gmax[group];
+    // without the outer half of the skin while nothing can have come in from it
+    const bool inner = sys_far && sys_far[group_sys[group]] == 0u;
+    const int gm = inner ? gmax_in[group] : gmax[group];
     const int per = ((gm + split - 1) / split + kChunk - 1) / kChunk * kChunk;
     const int e_begin = part * per, e_end = min(gm, e_begin + per);
     if (e_begin >= e_end) {  // no columns left for this part
@@ -101,7 +104,7 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
     const int self = valid ? s : 0;
     float4 mh, ml;
     gm_ld_coord(coord + 2 * self, mh, ml);
-    const int cnt = valid ? count[s] : 0;
+    const int cnt = valid ? (inner ? count_in : count)[s] : 0;
     const float4 *trow = (BATCH ? tab + (size_t)group_sys[group] * ntypes * ntypes : s_tab) +
                          (valid ? gm_slot_type(ml.w) : 0) * ntypes;
     const gm_df qi = gm_df_make(mh.w, ml.w);

@@ -66,8 +66,9 @@ __global__ void resync_kernel(int n, const double *pos, double *vel, const doubl
     for (int d = 0; d < 3; d++) vel[d * n + i] = gm_div_by_dt(pos[d * n + i] - dref[d * n + i], dt, inv_dt);
 }
 
-__global__ void check_kernel(int n, const double *pos, const double *ref, double thr_sq, DevStatus *st,
-                             unsigned long long cond, const int *atom_sys, unsigned int *sys_flag) {
+__global__ void check_kernel(int n, const double *pos, const double *ref, double thr_sq, double far_sq, DevStatus *st,
+                             unsigned long long cond, const int *atom_sys, unsigned int *sys_flag,
+                             unsigned int *sys_far) {
     // neighbor.rs:60-72 plus the run loop's finite-position guard (lib.rs:94-107);
     // the atom's system is marked for the rebuild
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,8 +77,10 @@ __global__ void check_kernel(int n, const double *pos, const double *ref, double
         const double x = pos[i], y = pos[n + i], z = pos[2 * n + i];
         bad = !(isfinite(x) && isfinite(y) && isfinite(z));
         const double dx = x - ref[i], dy = y - ref[n + i], dz = z - ref[2 * n + i];
-        need = dx * dx + dy * dy + dz * dz > thr_sq;
+        const double d2 = dx * dx + dy * dy + dz * dz;
+        need = d2 > thr_sq;
         if (need) sys_flag[atom_sys[i]] = 1u;
+        if (gm_moved_far(d2, far_sq)) sys_far[atom_sys[i]] = 1u;
     }
     need = __syncthreads_or(need);
     bad = __syncthreads_or(bad);
@@ -790,7 +793,9 @@ __device__ __forceinline__ void finish_atom(const SolveStepArgs &sa, const PackA
     for (int d = 0; d < 3; d++) sa.force[d * n + i] = 0;
     bad |= !(isfinite(x) && isfinite(y) && isfinite(z));
     const double dx = x - sa.ref[i], dy = y - sa.ref[n + i], dz = z - sa.ref[2 * n + i];
-    if (dx * dx + dy * dy + dz * dz > sa.thr_sq) {
+    const double d2 = dx * dx + dy * dy + dz * dz;
+    if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sy] = 1u;
+    if (d2 > sa.thr_sq) {
         sa.sys_flag[sy] = 1u;
         need = 1;
     }
@@ -1069,15 +1074,18 @@ __global__ void __launch_bounds__(256) frame_kernel(int n, const double *pos, co
         if (threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
         __syncthreads();
     }
+    if (threadIdx.x == 0) f.partial[blockIdx.x] = s[0];
+    __syncthreads();
+    const double share = gm_share_sum256(f.epart, f.n_epart, s);
     if (threadIdx.x == 0) {
-        f.partial[blockIdx.x] = s[0];
+        f.partial[GM_FRAME_BLOCKS + blockIdx.x] = share;
         __threadfence();
         last = atomicAdd(&st->blocks_done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const double e_pot = gm_block_sum256(f.epart, f.n_epart, s);
+    const double e_pot = gm_blocks_sum256(f.partial + GM_FRAME_BLOCKS, s);
     if (threadIdx.x == 0) {
         double sum = 0.0;
         for (int b = 0; b < (int)gridDim.x; b++) sum += ((volatile double *)f.partial)[b];
@@ -1146,8 +1154,9 @@ __global__ void forces_out_kernel(int n3, const long long *force, double *out) {
 // drift kernels do).
 __global__ void kick_drift_check_kernel(int n, double *pos, double *vel, double *dref, long long *force,
                                         const double *inv_mass, double dt_half, double dt, double inv_dt,
-                                        const double *ref, double thr_sq, DevStatus *st, unsigned long long cond,
-                                        const int *atom_sys, unsigned int *sys_flag, PackArgs pk) {
+                                        const double *ref, double thr_sq, double far_sq, DevStatus *st,
+                                        unsigned long long cond, const int *atom_sys, unsigned int *sys_flag,
+                                        unsigned int *sys_far, PackArgs pk) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int need = 0, bad = 0;
     // read by every block before the last block updates them
@@ -1185,8 +1194,10 @@ __global__ void kick_drift_check_kernel(int n, double *pos, double *vel, double 
         for (int d = 0; d < 3; d++) force[d * n + i] = 0;
         bad = !(isfinite(np[0]) && isfinite(np[1]) && isfinite(np[2]));
         const double dx = np[0] - ref[i], dy = np[1] - ref[n + i], dz = np[2] - ref[2 * n + i];
-        need = dx * dx + dy * dy + dz * dz > thr_sq;
+        const double d2 = dx * dx + dy * dy + dz * dz;
+        need = d2 > thr_sq;
         if (need) sys_flag[atom_sys[i]] = 1u;
+        if (gm_moved_far(d2, far_sq)) sys_far[atom_sys[i]] = 1u;
     }
     need = __syncthreads_or(need);
     bad = __syncthreads_or(bad);
@@ -1261,20 +1272,21 @@ void gm_launch_resync(int n, const double *pos, double *vel, const double *dref,
 void gm_launch_step(DevStatus *st, cudaStream_t s) { step_kernel<<<1, 1, 0, s>>>(st); }
 void gm_launch_kick_drift_check(int n, double *pos, double *vel, double *dref, long long *force,
                                 const double *inv_mass, double dt_half, double dt, const double *ref, double thr_sq,
-                                DevStatus *st, unsigned long long cond, const int *atom_sys, unsigned int *sys_flag,
-                                const PackArgs &pk, cudaStream_t s) {
+                                double far_sq, DevStatus *st, unsigned long long cond, const int *atom_sys,
+                                unsigned int *sys_flag, unsigned int *sys_far, const PackArgs &pk, cudaStream_t s) {
     kick_drift_check_kernel<<<gm_check_blocks(n), 256, 0, s>>>(n, pos, vel, dref, force, inv_mass, dt_half, dt,
-                                                              1.0 / dt, ref, thr_sq, st, cond, atom_sys, sys_flag,
-                                                              pk);
+                                                              1.0 / dt, ref, thr_sq, far_sq, st, cond, atom_sys,
+                                                              sys_flag, sys_far, pk);
 }
 void gm_launch_kick_tail(int n, double *vel, const long long *force, const double *inv_mass, double dt_half,
                          DevStatus *st, cudaStream_t s) {
     kick_tail_kernel<<<gm_check_blocks(n), 256, 0, s>>>(n, vel, force, inv_mass, dt_half, st);
 }
 
-void gm_launch_check(int n, const double *pos, const double *ref, double thr_sq, DevStatus *st,
-                     unsigned long long cond, int blocks, const int *atom_sys, unsigned int *sys_flag, cudaStream_t s) {
-    check_kernel<<<blocks, 256, 0, s>>>(n, pos, ref, thr_sq, st, cond, atom_sys, sys_flag);
+void gm_launch_check(int n, const double *pos, const double *ref, double thr_sq, double far_sq, DevStatus *st,
+                     unsigned long long cond, int blocks, const int *atom_sys, unsigned int *sys_flag,
+                     unsigned int *sys_far, cudaStream_t s) {
+    check_kernel<<<blocks, 256, 0, s>>>(n, pos, ref, thr_sq, far_sq, st, cond, atom_sys, sys_flag, sys_far);
 }
 
 void gm_launch_shake_prepare(const ClusterArgs &c, int n_atoms, const double *dref, cudaStream_t s) {

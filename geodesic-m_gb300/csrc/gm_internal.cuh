@@ -138,26 +138,37 @@ __device__ __forceinline__ void gm_add_sys_energy(long long *e_sys, int sy, doub
     }
 }
 
-// Sum of x[0..n) by a block of 256 threads: per-thread strided partial sums,
-// then a tree over the block (fixed order; every caller gets the same bits).
-__device__ __forceinline__ double gm_block_sum256(const double *x, int n, double *s) {
-    double acc = 0.0;
-    int i = threadIdx.x;
-    for (; i + 15 * 256 < n; i += 16 * 256) {  // 16 loads in flight, added in order
-        double v[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[k] = x[i + 256 * k];
-#pragma unroll
-        for (int k = 0; k < 16; k++) acc += v[k];
-    }
-    for (; i < n; i += 256) acc += x[i];
-    s[threadIdx.x] = acc;
+// Sum of x[0..n) over GM_SUM_BLOCKS blocks of 256 threads: this block's
+// consecutive share, per-thread strided partial sums, then a tree over the
+// block.  The last block to arrive (`last`, true for all its threads) adds the
+// blocks' sums in a tree of its own.  The order is fixed, so every kernel that
+// sums this way gets the same bits.  (One block alone took 13 us for the
+// 33,000 partials of a 50,000-atom system: an FP64 addition holds a scheduler
+// for 64 cycles.)
+constexpr int GM_SUM_BLOCKS = 64;
+__device__ __forceinline__ double gm_tree256(double v, double *s) {
+    s[threadIdx.x] = v;
     __syncthreads();
     for (int k = 128; k > 0; k >>= 1) {
         if (threadIdx.x < k) s[threadIdx.x] += s[threadIdx.x + k];
         __syncthreads();
     }
     return s[0];
+}
+__device__ __forceinline__ double gm_share_sum256(const double *x, int n, double *s) {
+    const int share = (n + GM_SUM_BLOCKS - 1) / GM_SUM_BLOCKS, b = blockIdx.x * share;
+    const int e = b + share < n ? b + share : n;
+    double acc = 0.0;
+    for (int i = b + threadIdx.x; i < e; i += 256) acc += x[i];
+    const double r = gm_tree256(acc, s);
+    __syncthreads();
+    return r;
+}
+// the blocks' sums, by one block (written before a __threadfence by the others)
+__device__ __forceinline__ double gm_blocks_sum256(const double *part, double *s) {
+    const double r = gm_tree256((int)threadIdx.x < GM_SUM_BLOCKS ? ((const volatile double *)part)[threadIdx.x] : 0.0, s);
+    __syncthreads();
+    return r;
 }
 
 // Both float4 of a slot's (hi, lo) coordinate pair in one 256-bit load
@@ -227,6 +238,12 @@ __device__ __forceinline__ bool gm_grid_barrier(unsigned *arrive, unsigned *gen,
     return s_ok != 0;
 }
 
+// d2 > far_sq for d2 >= 0, rounded towards yes (the high words: no FP64
+// comparison); a NaN counts as far.
+__device__ __forceinline__ bool gm_moved_far(double d2, double far_sq) {
+    return __double2hiint(d2) >= __double2hiint(far_sq);
+}
+
 // ------------------------------------------------------- launcher exports
 
 struct ListArgs {
@@ -250,6 +267,8 @@ struct ListArgs {
     const double *charge64;  // caller order (FP64 mode)
     const int *excl_start, *excl;   // caller-order CSR (both directions, sorted)
     int *list, *count, *gmax;
+    int *count_in, *gmax_in;        // the same without the last distance bucket (the outer half of the skin)
+    unsigned int *sys_far;          // nonzero: an atom of the system moved more than far_sq since its build (or nullptr)
     int *stage;              // [group][layer][entry][lane], cap_seg entries per layer
     double *ref;             // FP64 x|y|z copy at each system's build
     long long *force;        // zeroed with the pack
@@ -299,6 +318,14 @@ struct ForceArgs {
     const int *type_sorted;  // FP64 mode
     const int *perm;
     const int *list, *count, *gmax;
+    // While no atom of a system has moved more than a quarter of the skin (less
+    // 1e-3 A) since its build, pairs of the last distance bucket (beyond half
+    // the skin) cannot be inside the cutoff, and the columns end before them.
+    // sys_far[system] != 0 (or nullptr: unknown) takes the whole columns.  Mixed
+    // kernels only: an FP64 entry past the cutoff costs an FP32 test, less than
+    // the look at the flag (5,000 atoms: 2 % slower with it).
+    const int *count_in, *gmax_in;
+    const unsigned int *sys_far;
     int ntypes;
     const float4 *tab32;     // (sigma_ij^2, 24 epsilon_ij) per type pair, each a double-float (hi, lo)
     const double2 *tab64;    // (sigma_ij^2, 24 epsilon_ij)
@@ -328,7 +355,7 @@ struct ForceArgs {
     const double *sigma, *epsilon, *charge64;
     const double4 *p14par;   // per 1-4 pair: (sigma_ij, 4 eps_ij s_lj, 24 eps_ij s_lj, k_C q_i q_j s_coul)
     double *epart14; int blocks14;
-    double *energy;          // total
+    double *energy;          // total, then GM_SUM_BLOCKS block sums and the arrival count of their sum
     int n_epart_total;       // n_groups * split + bonded_blocks + blocks14 entries
 };
 
@@ -378,9 +405,9 @@ void gm_launch_drift(int n, double *pos, double *vel, double *dref, double dt, b
                      cudaStream_t s);
 void gm_launch_resync(int n, const double *pos, double *vel, const double *dref, double dt, const DevStatus *st,
                       cudaStream_t s);
-void gm_launch_check(int n, const double *pos, const double *ref, double thr_sq, DevStatus *st,
+void gm_launch_check(int n, const double *pos, const double *ref, double thr_sq, double far_sq, DevStatus *st,
                      unsigned long long cond_handle, int blocks, const int *atom_sys, unsigned int *sys_flag,
-                     cudaStream_t s);
+                     unsigned int *sys_far, cudaStream_t s);
 void gm_launch_shake(const ClusterArgs &c, int n_atoms, const double *dref, double *pos, cudaStream_t s);
 // the same solve in two halves, so the warm start can run in between:
 // prepare (reset T, reference vectors, multiplier sums) and the iterations
@@ -421,10 +448,10 @@ struct StepArgs {
     int n;
     double *pos, *vel, *dref;
     const double *inv_mass, *ref;
-    double dt_half, dt, inv_dt, thr_sq;
+    double dt_half, dt, inv_dt, thr_sq, far_sq;
     unsigned long long cond;   // graph conditional handle of the rebuild, or 0
     const int *atom_sys;
-    unsigned int *sys_flag;
+    unsigned int *sys_flag, *sys_far;
     StepSync *sync;
 };
 // The constrained step's two cooperative kernels (star clusters only):
@@ -442,10 +469,10 @@ struct SolveStepArgs {
     double *pos, *vel, *dref;
     long long *force;
     const double *ref;
-    double dt_half, dt, inv_dt, thr_sq;
+    double dt_half, dt, inv_dt, thr_sq, far_sq;
     unsigned long long cond;
     const int *atom_sys;
-    unsigned int *sys_flag;
+    unsigned int *sys_flag, *sys_far;
     SolveSync *sync;
 };
 // Threads per block and blocks (all co-resident) of both kernels; blocks 0
@@ -465,8 +492,8 @@ void gm_launch_step_persistent(const ForceArgs &fa, const StepArgs &sa, const Pa
 void gm_launch_forces_persistent(const ForceArgs &fa, StepSync *sync, int blocks, cudaStream_t s);
 void gm_launch_kick_drift_check(int n, double *pos, double *vel, double *dref, long long *force,
                                 const double *inv_mass, double dt_half, double dt, const double *ref, double thr_sq,
-                                DevStatus *st, unsigned long long cond, const int *atom_sys, unsigned int *sys_flag,
-                                const PackArgs &pk, cudaStream_t s);
+                                double far_sq, DevStatus *st, unsigned long long cond, const int *atom_sys,
+                                unsigned int *sys_flag, unsigned int *sys_far, const PackArgs &pk, cudaStream_t s);
 // Trajectory frames recorded on the device during resident steps.
 struct FrameArgs {
     int interval;                // a frame when the completed step count is a multiple (0: none)
@@ -474,11 +501,11 @@ struct FrameArgs {
     float *xyz;                  // [cap][3][n] positions as float32
     unsigned long long *step;    // [cap] step of each frame
     double *energy;              // [cap][2] potential and kinetic energy (kcal/mol)
-    double *partial;             // [kFrameBlocks] kinetic partial sums
+    double *partial;             // [2][GM_FRAME_BLOCKS] kinetic and potential partial sums
     const double *epart;         // energy partials of the last force evaluation
     int n_epart;
 };
-constexpr int GM_FRAME_BLOCKS = 64;  // the kinetic reduction's grid (as gm_kinetic_energy's)
+constexpr int GM_FRAME_BLOCKS = GM_SUM_BLOCKS;  // the kinetic reduction's grid (as gm_kinetic_energy's)
 // Records a frame when the step just completed is due: positions as float32,
 // the kinetic energy of the step's final velocities (its closing half-kick
 // applied when still pending, in the finalizer's arithmetic; the reduction of

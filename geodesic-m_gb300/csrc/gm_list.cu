@@ -194,6 +194,7 @@ __global__ void grid_kernel(ListArgs a, int blocks) {
         g->full[d] = a.periodic && nc[d] < 5;
     }
     g->ncell = nc[0] * nc[1] * nc[2];  // <= max_cells by construction
+    if (a.sys_far) a.sys_far[sys] = 0u;  // (the static build keeps no list)
     atomicAdd(&a.status->n_rebuilds, 1ull);
     s_ncell = min(g->ncell, max_cells);
     }
@@ -700,7 +701,7 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
     // this layer's first position in each bucket: the earlier buckets of all
     // layers, then this bucket of the earlier layers
     int off[GM_NBUCKET];
-    int total = 0;
+    int total = 0, inner = 0;  // inner: without the last bucket
 #pragma unroll
     for (int q = 0; q < GM_NBUCKET; q++) {
         int before = 0, all = 0;
@@ -711,6 +712,7 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
             all += ck;
         }
         off[q] = total + before;
+        inner = total;
         total += all;
     }
     int *my_list = a.list + (size_t)group * 32 * cap + lane;
@@ -749,16 +751,21 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
     }
     if (over && lane == 0) atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
     if (seg == 0) {
-        if (valid) a.count[s] = total < cap ? total : cap;
+        if (valid) {
+            a.count[s] = total < cap ? total : cap;
+            a.count_in[s] = inner < cap ? inner : cap;
+        }
         if (valid && total > cap) atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
         int c = valid ? (total < cap ? total : cap) : 0;
         int tm = valid ? total : 0;
+        const int ci = __reduce_max_sync(full, valid ? min(inner, cap) : 0);
         for (int o = 16; o > 0; o >>= 1) {
             c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
             tm = max(tm, __shfl_xor_sync(0xffffffffu, tm, o));
         }
         if (lane == 0) {
             a.gmax[group] = c;
+            a.gmax_in[group] = ci;
             atomicMax(&a.status->max_count, (unsigned)tm);
         }
     }

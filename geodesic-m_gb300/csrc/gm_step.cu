@@ -125,8 +125,8 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
                 // bonded tickets at or before t: min(q + 1, nbw)
                 const int item = t - min(q + 1, nbw);
                 pair_item_mixed<PERIODIC, COULOMB, BATCH, !STEP>(
-                    item, lane, fa.n, fa.cap, fa.split, fa.coord, fa.perm, fa.list, fa.count, fa.gmax, fa.ntypes,
-                    fa.tab32, s_tab, fa.pc, fa.force, fa.epart, st, fa.group_sys, STEP ? nullptr : fa.e_sys);
+                    item, lane, fa.n, fa.cap, fa.split, fa.coord, fa.perm, fa.list, fa.count, fa.gmax, fa.count_in,
+                    fa.gmax_in, fa.sys_far, fa.ntypes, fa.tab32, s_tab, fa.pc, fa.force, fa.epart, st, fa.group_sys, STEP ? nullptr : fa.e_sys);
             }
         }
     }
@@ -180,7 +180,9 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
         bad |= !(isfinite(np[0]) && isfinite(np[1]) && isfinite(np[2]));
         const double dx = __dsub_rn(np[0], sa.ref[i]), dy = __dsub_rn(np[1], sa.ref[n + i]),
                      dz = __dsub_rn(np[2], sa.ref[2 * n + i]);
-        const bool moved = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)) > sa.thr_sq;
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        const bool moved = d2 > sa.thr_sq;
+        if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sa.atom_sys[i]] = 1u;
         if (moved) {
             sa.sys_flag[sa.atom_sys[i]] = 1u;
             need = 1;
