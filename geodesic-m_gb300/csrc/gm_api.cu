@@ -561,7 +561,6 @@ int check_status(gm_ctx *c, gm_convergence *conv);
 // DevStatus travels through the pinned h_status on the context's own stream
 // (the stream is non-blocking, so legacy-stream copies would not be ordered).
 int st_read(gm_ctx *c) {
-    GM_CUDA(c, cudaStreamSynchronize(c->stream));
     GM_CUDA(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, c->stream));
     GM_CUDA(c, cudaStreamSynchronize(c->stream));
     return GM_OK;
@@ -573,30 +572,19 @@ int st_write(gm_ctx *c) {
     return GM_OK;
 }
 
-// Clears error and per-call fields; keeps the rebuild counter and the step.
+// Clears error and per-call fields on the device; keeps the counters, the
+// call's rebuild base and, unless a step is given, the step.  (Reading the
+// status word, clearing it on the host and writing it back waited for the
+// stream three times in every trait call.)
 int reset_status(gm_ctx *c) {
-    int rc = st_read(c);
-    if (rc) return rc;
-    DevStatus z{};
-    z.fail_step = ~0ull;
-    z.n_rebuilds = c->h_status->n_rebuilds;
-    z.step = c->h_status->step;
-    z.c_steps = c->h_status->c_steps;
-    z.shake_sum = c->h_status->shake_sum;
-    z.rattle_sum = c->h_status->rattle_sum;
-    z.rec_n = c->h_status->rec_n;
-    z.rebuild_base = c->h_status->rebuild_base;
-    z.frame_n = c->h_status->frame_n;
-    z.frame_lost = c->h_status->frame_lost;
-    *c->h_status = z;
-    return st_write(c);
+    gm_launch_status_reset(c->d_status, 0, 0, 1, c->stream);
+    GM_CUDA(c, cudaGetLastError());
+    return GM_OK;
 }
-
-int set_step(gm_ctx *c, uint64_t step) {
-    int rc = st_read(c);
-    if (rc) return rc;
-    c->h_status->step = step;
-    return st_write(c);
+int reset_status(gm_ctx *c, uint64_t step) {
+    gm_launch_status_reset(c->d_status, 1, step, 1, c->stream);
+    GM_CUDA(c, cudaGetLastError());
+    return GM_OK;
 }
 
 int fill_convergence(gm_ctx *c, bool rattle, gm_convergence *conv) {
@@ -660,10 +648,9 @@ int status_result(gm_ctx *c, gm_convergence *conv) {
 }
 
 int check_status(gm_ctx *c, gm_convergence *conv) {
-    GM_CUDA(c, cudaStreamSynchronize(c->stream));
-    GM_CUDA(c, cudaGetLastError());
     int rc0 = st_read(c);
     if (rc0) return rc0;
+    GM_CUDA(c, cudaGetLastError());
     return status_result(c, conv);
 }
 
@@ -723,15 +710,14 @@ int ensure_estimated_buffers(gm_ctx *c, const double *px, const double *py, cons
 int do_build(gm_ctx *c, bool all = true) {
     // list build on the resident positions (every system, or the flagged
     // ones), growing the capacity on overflow (then rebuilding every system)
-    unsigned long long r0 = 0, counted = 0;
+    unsigned long long counted = 0;
     for (int attempt = 0; attempt < 6; attempt++) {
         int rc = reset_status(c);
         if (rc) return rc;
-        if (attempt == 0) r0 = c->h_status->n_rebuilds;
         c->launches += seq_rebuild(c, c->stream, all || attempt > 0);
         c->far_marked = false;
         rc = check_status(c, nullptr);
-        if (attempt == 0) counted = c->h_status->n_rebuilds - r0;
+        if (attempt == 0) counted = c->h_status->n_rebuilds;
         // the build records the longest list and staged layer it met: on an
         // overflow, or (when every system was built) within 20 % of a
         // capacity, since a resident run cannot grow the list, grow that
@@ -750,7 +736,7 @@ int do_build(gm_ctx *c, bool all = true) {
         if (rc) return rc;
         if (attempt > 0) {
             // capacity rebuilds are not list rebuilds: count the first attempt's
-            c->h_status->n_rebuilds = r0 + counted;
+            c->h_status->n_rebuilds = counted;
             rc = st_write(c);
             if (rc) return rc;
         }
@@ -1878,7 +1864,7 @@ int32_t gm_needs_rebuild(gm_ctx *c, const double *px, const double *py, const do
     *result = c->h_status->rebuild ? 1 : 0;
     gm_launch_flags(list_args(c), false, c->stream);  // a query: leave no system marked
     c->launches += 2;
-    GM_CUDA(c, cudaStreamSynchronize(c->stream));
+    GM_CUDA(c, cudaGetLastError());
     return GM_OK;
 }
 
@@ -1889,8 +1875,7 @@ int32_t gm_geodesic_drift(gm_ctx *c, double *px, double *py, double *pz, double 
     int rc = upload3(c, c->d_pos, px, py, pz);
     if (!rc) rc = upload3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
-    rc = reset_status(c);
-    if (!rc) rc = set_step(c, step);
+    rc = reset_status(c, step);
     if (rc) return rc;
     const bool constrained = c->n_clusters > 0;
     gm_launch_drift(c->n, c->d_pos, c->d_vel, c->d_dref, dt, !constrained, c->d_status, c->stream);
@@ -1930,8 +1915,7 @@ int32_t gm_constrain_velocities(gm_ctx *c, const double *px, const double *py, c
     int rc = upload3(c, c->d_pos, px, py, pz);
     if (!rc) rc = upload3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
-    rc = reset_status(c);
-    if (!rc) rc = set_step(c, step);
+    rc = reset_status(c, step);
     if (rc) return rc;
     gm_launch_rattle(cluster_args(c), c->n, c->d_pos, c->d_vel, c->stream);
     c->launches += 3;
@@ -1947,8 +1931,9 @@ int32_t gm_kinetic_energy(gm_ctx *c, const double *vx, const double *vy, const d
     if (rc) return rc;
     gm_launch_kinetic(c->n, c->d_vel, c->d_mass, c->d_kin_part, 64, c->d_ke, c->stream);
     c->launches += 2;
-    GM_CUDA(c, cudaMemcpyAsync(ke, c->d_ke, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    GM_CUDA(c, cudaMemcpyAsync(c->h_energy, c->d_ke, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     GM_CUDA(c, cudaStreamSynchronize(c->stream));
+    *ke = *c->h_energy;
     return GM_OK;
 }
 
@@ -2109,8 +2094,7 @@ int32_t gm_forces_resident(gm_ctx *c) {
 int32_t gm_run_resident(gm_ctx *c, double dt, uint64_t first_step, int64_t n_steps) {
     if (!c || !(dt > 0) || n_steps < 0) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
-    int rc = reset_status(c);
-    if (!rc) rc = set_step(c, first_step);
+    int rc = reset_status(c, first_step);
     if (rc) return rc;
     rc = ensure_forces(c);
     if (rc) return rc;
@@ -2121,8 +2105,7 @@ int32_t gm_time_steps(gm_ctx *c, double dt, uint64_t first_step, int64_t n_steps
                       int64_t flush_bytes, double *total_ms) {
     if (!c || !(dt > 0) || n_steps <= 0 || !total_ms) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
-    int rc = reset_status(c);
-    if (!rc) rc = set_step(c, first_step);
+    int rc = reset_status(c, first_step);
     if (!rc) rc = ensure_forces(c);
     if (!rc && c->use_graph) rc = capture_graph(c, dt);
     // every timed persistent launch evaluates its forces
@@ -2191,7 +2174,7 @@ int32_t gm_steps(gm_ctx *c, double *px, double *py, double *pz, double *vx, doub
         int rc = ensure_estimated_buffers(c, px, py, pz);
         if (rc) return rc;
     }
-    gm_launch_status_reset(c->d_status, 1, first_step, c->stream);
+    gm_launch_status_reset(c->d_status, 1, first_step, 0, c->stream);
     c->launches++;
     // the velocities travel on the copy stream, after the work already on
     // the context's stream and beside the position check

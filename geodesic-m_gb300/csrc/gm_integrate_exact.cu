@@ -1123,7 +1123,7 @@ __global__ void differs_kernel(int n3, const double *a, const double *b, unsigne
     if (threadIdx.x == 0 && (d || bad)) atomicOr(flag, (d ? 1u : 0u) | (bad ? 2u : 0u));
 }
 
-__global__ void status_reset_kernel(DevStatus *st, int set_step, unsigned long long step) {
+__global__ void status_reset_kernel(DevStatus *st, int set_step, unsigned long long step, int keep_base) {
     DevStatus z{};
     z.fail_step = ~0ull;
     z.n_rebuilds = st->n_rebuilds;
@@ -1134,7 +1134,7 @@ __global__ void status_reset_kernel(DevStatus *st, int set_step, unsigned long l
     z.rec_n = st->rec_n;
     z.frame_n = st->frame_n;
     z.frame_lost = st->frame_lost;
-    z.rebuild_base = st->n_rebuilds;
+    z.rebuild_base = keep_base ? st->rebuild_base : st->n_rebuilds;
     *st = z;
 }
 
@@ -1373,8 +1373,8 @@ void gm_launch_frame(int n, const double *pos, const double *vel, const long lon
                      const double *mass, double dt_half, DevStatus *st, const FrameArgs &f, cudaStream_t s) {
     frame_kernel<<<GM_FRAME_BLOCKS, 256, 0, s>>>(n, pos, vel, force, inv_mass, mass, dt_half, st, f);
 }
-void gm_launch_status_reset(DevStatus *st, int set_step, unsigned long long step, cudaStream_t s) {
-    status_reset_kernel<<<1, 1, 0, s>>>(st, set_step, step);
+void gm_launch_status_reset(DevStatus *st, int set_step, unsigned long long step, int keep_base, cudaStream_t s) {
+    status_reset_kernel<<<1, 1, 0, s>>>(st, set_step, step, keep_base);
 }
 void gm_launch_differs(int n, const double *a, const double *b, unsigned int *flag, cudaStream_t s) {
     if (n) differs_kernel<<<(3 * n + 255) / 256, 256, 0, s>>>(3 * n, a, b, flag);

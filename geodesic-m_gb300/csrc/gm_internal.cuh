@@ -521,8 +521,9 @@ void gm_launch_kinetic(int n, const double *vel, const double *mass, double *par
 void gm_launch_forces_out(int n, const long long *force, double *out, cudaStream_t s);
 void gm_launch_differs(int n, const double *a, const double *b, unsigned int *flag, cudaStream_t s);
 // The per-call status reset on the device: counters kept, per-call fields
-// cleared, the step set when set_step, n_rebuilds noted as the call's base.
-void gm_launch_status_reset(DevStatus *st, int set_step, unsigned long long step, cudaStream_t s);
+// cleared, the step set when set_step, n_rebuilds noted as the call's base
+// unless keep_base.
+void gm_launch_status_reset(DevStatus *st, int set_step, unsigned long long step, int keep_base, cudaStream_t s);
 int gm_check_blocks(int n);
 
 // ---- constraint warm start (gm_mlp.cu) -----------------------------------
