@@ -106,8 +106,10 @@ __device__ __forceinline__ long long gm_to_fix(double v) { return __double2ll_rn
 
 // A float force contribution to fixed point; flags non-finite / overflow.
 __device__ __forceinline__ long long gm_to_fix_checked(float v, unsigned int &bad) {
-    if (!isfinite(v)) { bad |= GM_DEV_NONFINITE_FORCE; return 0; }
-    if (fabsf(v) >= (float)GM_FIX_LIMIT) { bad |= GM_DEV_FIX_OVERFLOW; return 0; }
+    if (!(fabsf(v) < (float)GM_FIX_LIMIT)) {
+        bad |= isfinite(v) ? GM_DEV_FIX_OVERFLOW : GM_DEV_NONFINITE_FORCE;
+        return 0;
+    }
     return gm_f2fix(v);
 }
 __device__ __forceinline__ long long gm_to_fix_checked(double v, unsigned int &bad) {
