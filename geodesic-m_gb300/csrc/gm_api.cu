@@ -281,6 +281,9 @@ double far_sq(const gm_ctx *c) {
     return d * d;
 }
 
+// 32-atom groups up to which the persistent kernel gives each pair item a block.
+constexpr int kQuadGroups = 100;
+
 // periodic && bonded_min_image: bonded, 1-4 and constraint differences at the
 // nearest periodic image
 bool bonded_min_image(const gm_ctx *c) { return c->p.periodic && c->p.bonded_min_image; }
@@ -296,6 +299,7 @@ ForceArgs force_args(gm_ctx *c) {
     a.cap = c->cap;
     a.split = c->split;
     a.term_chunk = c->term_chunk;
+    a.quad = c->n_sys == 1 && c->n_groups <= kQuadGroups;
     a.pair_warps = c->pair_warps;
     a.pair_grid = c->pair_grid;
     a.coord = c->d_coord;

@@ -39,6 +39,87 @@ __device__ __forceinline__ void image_df(float &dh, float &dl, float L, float Ll
     dh = q;
 }
 
+// Difference of two slot records (at the nearest image: `vote` is a warp vote,
+// so all lanes call) and its square r^2 as a double-float.
+template <bool PERIODIC>
+__device__ __forceinline__ gm_df pair_r2(const float4 &mh, const float4 &ml, const float4 &jh, const float4 &jl,
+                                         const PairConst &k, float *d_h, float *d_l) {
+    d_h[0] = jh.x - mh.x; d_h[1] = jh.y - mh.y; d_h[2] = jh.z - mh.z;
+    d_l[0] = jl.x - ml.x; d_l[1] = jl.y - ml.y; d_l[2] = jl.z - ml.z;
+    float S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));  // exact
+    if (PERIODIC) {
+        if (__any_sync(0xffffffffu, S > k.img2)) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) image_df(d_h[d], d_l[d], k.box[d], k.box_lo[d], k.inv_box[d]);
+            S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));
+        }
+    }
+    const float c = fmaf(d_l[2], fmaf(2.f, d_h[2], d_l[2]),
+                         fmaf(d_l[1], fmaf(2.f, d_h[1], d_l[1]), d_l[0] * fmaf(2.f, d_h[0], d_l[0])));
+    return gm_fast_sum(S, c);
+}
+
+// F_r / r (and with ENERGY the pair energy v) of a pair inside the cutoff:
+// R = r^2, p = (sigma^2, 24 epsilon) as double-floats.  Every rounding is
+// pinned: the kernels that inline this get the same bits.
+template <bool COULOMB, bool ENERGY>
+__device__ __forceinline__ void pair_terms(const gm_df R, const gm_df qi, const gm_df qj, const float4 p,
+                                           const PairConst &k, gm_df &G, float &v) {
+    // 1/r^2 = y (1 + rho - Rl y), rho = 1 - Rh y
+    const float y = rcp_approx(R.h);
+    const float rho = fmaf(-R.h, y, 1.f);
+    const gm_df inv = gm_df_make(y, y * fmaf(-R.l, y, rho));
+    // 1/r = z (1 - tau / 2), tau = (Rh + Rl) z^2 - 1 from exact products
+    const float z = rsqrt_approx(R.h);
+    const float rz = __fmul_rn(R.h, z), ez = fmaf(R.h, z, -rz);
+    const float tau = fmaf(R.l, y, fmaf(ez, z, fmaf(rz, z, -1.f)));
+    const gm_df rinv = gm_df_make(z, -0.5f * z * tau);
+    gm_df Vc = gm_df_make(0.f, 0.f), Gc = Vc;
+    if (COULOMB) {
+        Vc = gm_dmul(gm_dmul(qi, qj), rinv);  // k q_i q_j / r
+        Gc = gm_dmul(Vc, inv);                // (k q_i q_j / r^2) / r
+    }
+    if (R.h <= k.rsw2) {
+        const gm_df x = gm_dmul(gm_df_make(p.x, p.y), inv);  // (sigma / r)^2
+        const gm_df x3 = gm_dmul(gm_dsqr(x), x);
+        gm_df w2 = gm_two_sum(x3.h + x3.h, -1.f);  // 2 x3 - 1
+        w2.l = fmaf(2.f, x3.l, w2.l);
+        const gm_df g = gm_dmul(gm_dmul(gm_dmul(gm_df_make(p.z, p.w), x3), w2), inv);
+        G = gm_dadd(g, Gc);
+        if (ENERGY) v = fmaf(__fmul_rn(__fmul_rn(p.z, 1.f / 6.f), x3.h), x3.h - 1.f, Vc.h + Vc.l);
+    } else {
+        // LJ in FP32 (tiny here), then V S and F_r S - V dS/dr
+        // (products rounded where the compiler could otherwise fuse them
+        // into the sums that follow)
+        const float xs = p.x * y, x3 = __fmul_rn(__fmul_rn(xs, xs), xs);
+        const float vlj = p.z * (1.f / 6.f) * x3 * (x3 - 1.f);
+        const float glj = p.z * x3 * fmaf(2.f, x3, -1.f) * y;
+        const gm_df V = gm_dadd(Vc, gm_df_make(vlj, 0.f));
+        const gm_df G0 = gm_dadd(Gc, gm_df_make(glj, 0.f));
+        // r = r^2 / r, whose head and its error are rz and ez
+        gm_df u0 = gm_fast_sum(rz, -k.rsw);
+        u0.l += fmaf(R.l, z, fmaf(R.h, rinv.l, ez)) - k.rsw_lo;
+        const gm_df uu = gm_dmul(u0, gm_df_make(k.inv_w, k.inv_w_lo));
+        const gm_df u2 = gm_dsqr(uu), u3 = gm_dmul(u2, uu);
+        // S = 1 + u^3 (-10 + u (15 - 6 u))
+        const float p6 = __fmul_rn(6.f, uu.h), e6 = fmaf(6.f, uu.h, -p6);
+        gm_df t = gm_fast_sum(15.f, -p6);
+        t.l -= fmaf(6.f, uu.l, e6);
+        t = gm_dmul(uu, t);
+        gm_df t3 = gm_fast_sum(-10.f, t.h);
+        t3.l += t.l;
+        t = gm_dmul(u3, t3);
+        gm_df sw = gm_fast_sum(1.f, t.h);
+        sw.l += t.l;
+        // dS/dr = -30 u^2 (1 - u)^2 / w
+        gm_df om = gm_fast_sum(1.f, -uu.h);
+        om.l -= uu.l;
+        const gm_df ds = gm_dmul(gm_dmul(u2, gm_dsqr(om)), gm_df_make(k.mds, k.mds_lo));
+        G = gm_dadd(gm_dmul(G0, sw), gm_dneg(gm_dmul(gm_dmul(V, ds), rinv)));
+        if (ENERGY) v = __fmul_rn(V.h + V.l, sw.h + sw.l);
+    }
+}
+
 // One work item of the mixed-precision nonbonded kernel (force/nonbonded.rs:20-82
 // physics plus the switched Coulomb term): FP32 operations throughout, arranged as
 // double-float arithmetic so that each pair's force carries ~1e-10 relative
@@ -129,77 +210,16 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
 #pragma unroll
             for (int u = 0; u < kBatch; u++) {
                 const float4 jh = jhv[u], jl = jlv[u];
-                float d_h[3] = {jh.x - mh.x, jh.y - mh.y, jh.z - mh.z};
-                float d_l[3] = {jl.x - ml.x, jl.y - ml.y, jl.z - ml.z};
-                float S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));  // exact
-                if (PERIODIC) {
-                    if (__any_sync(full, S > k.img2)) {
-#pragma unroll
-                        for (int d = 0; d < 3; d++) image_df(d_h[d], d_l[d], k.box[d], k.box_lo[d], k.inv_box[d]);
-                        S = fmaf(d_h[2], d_h[2], fmaf(d_h[1], d_h[1], d_h[0] * d_h[0]));
-                    }
-                }
-                const float c = fmaf(d_l[2], fmaf(2.f, d_h[2], d_l[2]),
-                                     fmaf(d_l[1], fmaf(2.f, d_h[1], d_l[1]), d_l[0] * fmaf(2.f, d_h[0], d_l[0])));
-                const gm_df R = gm_fast_sum(S, c);  // r^2
+                float d_h[3], d_l[3];
+                const gm_df R = pair_r2<PERIODIC>(mh, ml, jh, jl, k, d_h, d_l);
                 const bool in = R.h <= k.rc2 && R.h > 0.f;
                 if (!__any_sync(full, in)) continue;  // warp-uniform: the shell beyond the cutoff
                 if (in) {
-                    // 1/r^2 = y (1 + rho - Rl y), rho = 1 - Rh y
-                    const float y = rcp_approx(R.h);
-                    const float rho = fmaf(-R.h, y, 1.f);
-                    const gm_df inv = gm_df_make(y, y * fmaf(-R.l, y, rho));
-                    // 1/r = z (1 - tau / 2), tau = (Rh + Rl) z^2 - 1 from exact products
-                    const float z = rsqrt_approx(R.h);
-                    const float rz = __fmul_rn(R.h, z), ez = fmaf(R.h, z, -rz);
-                    const float tau = fmaf(R.l, y, fmaf(ez, z, fmaf(rz, z, -1.f)));
-                    const gm_df rinv = gm_df_make(z, -0.5f * z * tau);
                     const float4 p = BATCH ? __ldg(trow + gm_slot_type(jl.w)) : trow[gm_slot_type(jl.w)];
-                    gm_df Vc = gm_df_make(0.f, 0.f), Gc = Vc;
-                    if (COULOMB) {
-                        Vc = gm_dmul(gm_dmul(qi, gm_df_make(jh.w, jl.w)), rinv);  // k q_i q_j / r
-                        Gc = gm_dmul(Vc, inv);                                     // (k q_i q_j / r^2) / r
-                    }
                     gm_df G;  // F_r / r
-                    if (R.h <= k.rsw2) {
-                        const gm_df x = gm_dmul(gm_df_make(p.x, p.y), inv);  // (sigma / r)^2
-                        const gm_df x3 = gm_dmul(gm_dsqr(x), x);
-                        gm_df w2 = gm_two_sum(x3.h + x3.h, -1.f);  // 2 x3 - 1
-                        w2.l = fmaf(2.f, x3.l, w2.l);
-                        const gm_df g = gm_dmul(gm_dmul(gm_dmul(gm_df_make(p.z, p.w), x3), w2), inv);
-                        G = gm_dadd(g, Gc);
-                        if (ENERGY) ev += p.z * (1.f / 6.f) * x3.h * (x3.h - 1.f) + (Vc.h + Vc.l);
-                    } else {
-                        // LJ in FP32 (tiny here), then V S and F_r S - V dS/dr
-                        // (products rounded where the compiler could otherwise fuse them
-                        // into the sums that follow)
-                        const float xs = p.x * y, x3 = __fmul_rn(__fmul_rn(xs, xs), xs);
-                        const float vlj = p.z * (1.f / 6.f) * x3 * (x3 - 1.f);
-                        const float glj = p.z * x3 * fmaf(2.f, x3, -1.f) * y;
-                        const gm_df V = gm_dadd(Vc, gm_df_make(vlj, 0.f));
-                        const gm_df G0 = gm_dadd(Gc, gm_df_make(glj, 0.f));
-                        // r = r^2 / r, whose head and its error are rz and ez
-                        gm_df u0 = gm_fast_sum(rz, -k.rsw);
-                        u0.l += fmaf(R.l, z, fmaf(R.h, rinv.l, ez)) - k.rsw_lo;
-                        const gm_df uu = gm_dmul(u0, gm_df_make(k.inv_w, k.inv_w_lo));
-                        const gm_df u2 = gm_dsqr(uu), u3 = gm_dmul(u2, uu);
-                        // S = 1 + u^3 (-10 + u (15 - 6 u))
-                        const float p6 = __fmul_rn(6.f, uu.h), e6 = fmaf(6.f, uu.h, -p6);
-                        gm_df t = gm_fast_sum(15.f, -p6);
-                        t.l -= fmaf(6.f, uu.l, e6);
-                        t = gm_dmul(uu, t);
-                        gm_df t3 = gm_fast_sum(-10.f, t.h);
-                        t3.l += t.l;
-                        t = gm_dmul(u3, t3);
-                        gm_df sw = gm_fast_sum(1.f, t.h);
-                        sw.l += t.l;
-                        // dS/dr = -30 u^2 (1 - u)^2 / w
-                        gm_df om = gm_fast_sum(1.f, -uu.h);
-                        om.l -= uu.l;
-                        const gm_df ds = gm_dmul(gm_dmul(u2, gm_dsqr(om)), gm_df_make(k.mds, k.mds_lo));
-                        G = gm_dadd(gm_dmul(G0, sw), gm_dneg(gm_dmul(gm_dmul(V, ds), rinv)));
-                        if (ENERGY) ev += __fmul_rn(V.h + V.l, sw.h + sw.l);
-                    }
+                    float v;
+                    pair_terms<COULOMB, ENERGY>(R, qi, gm_df_make(jh.w, jl.w), p, k, G, v);
+                    if (ENERGY) ev += v;
                     // F_i -= G d, each product with its exact error
 #pragma unroll
                     for (int d = 0; d < 3; d++) {
@@ -230,6 +250,117 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
     }
     bad = __reduce_or_sync(full, bad);
     if (bad && lane == 0) atomicOr(&st->error, bad);
+}
+
+// Transposes x over the 4 lanes of a quad: lane c of the quad gets x[c] of its
+// lanes 0..3, in order.
+__device__ __forceinline__ void quad_transpose(float x[4], int sub) {
+    const unsigned full = 0xffffffffu;
+    const bool b0 = sub & 1, b1 = sub & 2;
+    const float p = __shfl_xor_sync(full, b0 ? x[0] : x[1], 1), q = __shfl_xor_sync(full, b0 ? x[2] : x[3], 1);
+    if (b0) { x[0] = p; x[2] = q; }
+    else { x[1] = p; x[3] = q; }
+    const float r = __shfl_xor_sync(full, b1 ? x[0] : x[2], 2), t = __shfl_xor_sync(full, b1 ? x[1] : x[3], 2);
+    if (b1) { x[0] = r; x[1] = t; }
+    else { x[2] = r; x[3] = t; }
+}
+
+// The same work item by a block of four warps, for systems whose items do not
+// fill the chip: an item is then one warp's latency, 32 entries of ~1,300
+// cycles each (a dependent chain of ~200 FP32 operations).  Here a warp takes 8
+// of the group's atoms and four lanes an atom: the four evaluate four
+// consecutive entries at once, and after a transposition lane 0, 1, 2 of the
+// quad add the four products to the x, y, z sum one after the other (lane 3 the
+// energies), in the order and the arithmetic of pair_item_mixed, so every
+// sum has its bits.  All threads of the block call; `s_e`: 32 doubles.
+template <bool PERIODIC, bool COULOMB, bool ENERGY>
+__device__ __forceinline__ void
+pair_item_quad(int wid, int warp, int lane, const ForceArgs &fa, const float4 *s_tab, double *s_e) {
+    const unsigned full = 0xffffffffu;
+    const PairConst &k = fa.pc;
+    const int split = fa.split, group = wid / split, part = wid - group * split;
+    const bool inner = fa.sys_far && fa.sys_far[fa.group_sys[group]] == 0u;
+    const int gm = inner ? fa.gmax_in[group] : fa.gmax[group];
+    const int per = ((gm + split - 1) / split + kChunk - 1) / kChunk * kChunk;
+    const int e_begin = part * per, e_end = min(gm, e_begin + per);
+    if (e_begin >= e_end) {  // block-uniform: no columns left for this part
+        if (ENERGY && warp == 0 && lane == 0) fa.epart[wid] = 0.0;
+        return;
+    }
+    const int sub = lane & 3, l = warp * 8 + (lane >> 2);
+    const int s = group * 32 + l;
+    const int atom = fa.perm[s];
+    const bool valid = atom >= 0;
+    const int self = valid ? s : 0;
+    float4 mh, ml;
+    gm_ld_coord(fa.coord + 2 * self, mh, ml);
+    const int cnt = valid ? (inner ? fa.count_in : fa.count)[s] : 0;
+    const float4 *trow = s_tab + (valid ? gm_slot_type(ml.w) : 0) * fa.ntypes;
+    const gm_df qi = gm_df_make(mh.w, ml.w);
+    const int *L = fa.list + (size_t)group * 32 * fa.cap + l;
+    long long sum = 0;
+    double eacc = 0.0;
+    unsigned bad = 0;
+    for (int e0 = e_begin; e0 < e_end; e0 += kChunk) {
+        gm_df acc = gm_df_make(0.f, 0.f);
+        float ev = 0.f;
+        const int e1 = min(e0 + kChunk, e_end);
+        int jj[kChunk / 4];
+#pragma unroll
+        for (int t = 0; t < kChunk / 4; t++) {
+            const int e = e0 + 4 * t + sub;
+            jj[t] = e < cnt && e < e1 ? __ldg(L + (size_t)e * 32) : self;
+        }
+        float4 jh, jl, nh, nl;
+        gm_ld_coord(fa.coord + 2 * jj[0], nh, nl);
+#pragma unroll
+        for (int t = 0; t < kChunk / 4; t++) {
+            jh = nh;
+            jl = nl;
+            if (t + 1 < kChunk / 4) gm_ld_coord(fa.coord + 2 * jj[t + 1], nh, nl);  // beside this round's arithmetic
+            float d_h[3], d_l[3];
+            const gm_df R = pair_r2<PERIODIC>(mh, ml, jh, jl, k, d_h, d_l);
+            const bool in = R.h <= k.rc2 && R.h > 0.f;
+            if (!__any_sync(full, in)) continue;
+            // an entry outside adds zeros, which change no sum
+            float pr[4] = {0.f, 0.f, 0.f, 0.f}, er[4] = {0.f, 0.f, 0.f, 0.f};
+            if (in) {
+                gm_df G;
+                float v = 0.f;
+                pair_terms<COULOMB, ENERGY>(R, qi, gm_df_make(jh.w, jl.w), trow[gm_slot_type(jl.w)], k, G, v);
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    pr[d] = __fmul_rn(G.h, d_h[d]);
+                    er[d] = fmaf(G.h, d_l[d], fmaf(G.l, d_h[d], fmaf(G.h, d_h[d], -pr[d])));
+                }
+                if (ENERGY) pr[3] = v;
+            }
+            quad_transpose(pr, sub);
+            quad_transpose(er, sub);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                gm_df t2 = gm_two_sum(acc.h, -pr[q]);
+                t2.l += acc.l - er[q];
+                acc = t2;
+                if (ENERGY) ev += pr[q];
+            }
+        }
+        if (sub < 3) sum += gm_to_fix_checked(acc.h, bad) + gm_f2fix(acc.l);
+        else if (ENERGY) eacc += (double)ev;
+    }
+    if (valid && sub < 3) gm_atomic_fix_add(fa.force + (size_t)sub * fa.n + atom, sum);
+    if (ENERGY) {
+        __syncthreads();
+        if (sub == 3) s_e[l] = eacc;
+        __syncthreads();
+        if (warp == 0) {
+            double e = s_e[lane];
+            for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(full, e, o);
+            if (lane == 0) fa.epart[wid] = 0.5 * e;
+        }
+    }
+    bad = __reduce_or_sync(full, bad);
+    if (bad && lane == 0) atomicOr(&fa.status->error, bad);
 }
 
 // ----------------------------------------------------------------- bonded

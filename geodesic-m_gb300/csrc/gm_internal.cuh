@@ -312,6 +312,7 @@ struct ForceArgs {
     const int *group_sys, *atom_sys;
     long long *e_sys;        // per-system potential energy, fixed point 2^-32 kcal/mol (batches), or nullptr
     int split;               // warps per 32-atom group in the FP32 pair kernel
+    int quad;                // the persistent kernel gives a pair item a block (small systems)
     int term_chunk;          // bonded terms (or 1-4 pairs) per work item of the persistent kernel
     int pair_warps;          // warps per block of the FP32 pair kernel (2, 4, 8)
     int pair_grid;           // blocks of the FP32 pair kernel (0: one work item per warp; fewer: persistent)

@@ -70,11 +70,47 @@ __host__ __device__ __forceinline__ int pair14_tickets(const ForceArgs &fa, int 
     return (fa.n14 + chunk - 1) / chunk;
 }
 
+// The force phase of a small system (QUAD): a block per pair item
+// (pair_item_quad) or per 128 bonded terms, handed out by block index.  With a
+// warp per item and a queue the phase was the longest item: 45,000 cycles at
+// 1,536 atoms, while most of the chip was idle.
+template <bool PERIODIC, bool COULOMB, bool MI, bool STEP>
+__device__ __forceinline__ void quad_phase(const ForceArgs &fa, const float4 *s_tab) {
+    __shared__ double s_e[kStepThreads];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int cb = bonded_tickets(fa, kStepThreads), nbw = cb + pair14_tickets(fa, kStepThreads);
+    const int total = nbw + fa.n_groups * fa.split;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        if (t >= nbw) {
+            pair_item_quad<PERIODIC, COULOMB, !STEP>(t - nbw, warp, lane, fa, s_tab, s_e);
+            continue;
+        }
+        unsigned bad = 0;
+        int first = -1;
+        const bool b14 = t >= cb;
+        const int term = (b14 ? t - cb : t) * kStepThreads + (int)threadIdx.x;
+        const double e = b14 ? pair14_term<MI>(fa, term, bad, first) : bonded_term<MI>(fa, term, bad, first);
+        if (!STEP) {
+            // term_block's partial of each 64 terms: two warps hold its halves
+            __syncthreads();
+            s_e[threadIdx.x] = e;
+            __syncthreads();
+            double v = e + s_e[(threadIdx.x + 32) % kStepThreads];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            const int blk = term / GM_BONDED_THREADS;
+            if (lane == 0 && (warp & 1) == 0 && blk < (b14 ? fa.blocks14 : fa.bonded_blocks))
+                (b14 ? fa.epart14 : fa.epart_bonded)[blk] = v;
+        }
+        bad = __reduce_or_sync(0xffffffffu, bad);
+        if (bad && lane == 0) atomicOr(&fa.status->error, bad);
+    }
+}
+
 // STEP: one BAB step (phases 1-3 above, a cooperative launch).  !STEP: phase
 // 1 alone with energies (the pair items' partials, the 64-term blocks'
 // partials and the per-system energies of the force kernels, the same bits),
 // a plain launch; its last warp clears the queue words.
-template <bool PERIODIC, bool COULOMB, bool BATCH, bool MI, bool STEP>
+template <bool PERIODIC, bool COULOMB, bool BATCH, bool MI, bool STEP, bool QUAD>
 __global__ void __launch_bounds__(kStepThreads, kStepMinBlocks)
 step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
     extern __shared__ float4 s_tab[];
@@ -90,6 +126,9 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
             for (int t = threadIdx.x; t < fa.ntypes * fa.ntypes; t += blockDim.x) s_tab[t] = fa.tab32[t];
             __syncthreads();
         }
+        if constexpr (QUAD) {
+            quad_phase<PERIODIC, COULOMB, MI, STEP>(fa, s_tab);
+        } else {
         // tickets: n_pair pair items and nbw bonded tickets (chunk bonded
         // terms or 1-4 pairs each), the bonded ones at t = k * stride
         const int n_pair = fa.n_groups * fa.split;
@@ -126,11 +165,14 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
                 const int item = t - min(q + 1, nbw);
                 pair_item_mixed<PERIODIC, COULOMB, BATCH, !STEP>(
                     item, lane, fa.n, fa.cap, fa.split, fa.coord, fa.perm, fa.list, fa.count, fa.gmax, fa.count_in,
-                    fa.gmax_in, fa.sys_far, fa.ntypes, fa.tab32, s_tab, fa.pc, fa.force, fa.epart, st, fa.group_sys, STEP ? nullptr : fa.e_sys);
+                    fa.gmax_in, fa.sys_far, fa.ntypes, fa.tab32, s_tab, fa.pc, fa.force, fa.epart, st, fa.group_sys,
+                    STEP ? nullptr : fa.e_sys);
             }
+        }
         }
     }
     if (!STEP) {
+        if (QUAD) return;  // no queue
         // the last warp out leaves the queue words at zero for the next launch
         if (lane == 0) {
             __threadfence();
@@ -214,8 +256,9 @@ using StepKernel = void (*)(ForceArgs, StepArgs, PackArgs);
 
 template <bool STEP>
 StepKernel pick(const ForceArgs &fa, bool gtab) {
-#define GM_STEPK(P, Q, B, M) return step_persistent_kernel<P, Q, B, M, STEP>
-#define GM_STEPB(P, Q, M) { if (gtab) GM_STEPK(P, Q, true, M); else GM_STEPK(P, Q, false, M); }
+#define GM_STEPK(P, Q, B, M, D) return step_persistent_kernel<P, Q, B, M, STEP, D>
+#define GM_STEPB(P, Q, M) { if (gtab) GM_STEPK(P, Q, true, M, false); else if (fa.quad) GM_STEPK(P, Q, false, M, true); \
+                            else GM_STEPK(P, Q, false, M, false); }
 #define GM_STEPQ(P, M) { if (fa.coulomb) GM_STEPB(P, true, M) else GM_STEPB(P, false, M) }
     if (fa.bonded_mi) GM_STEPQ(true, true)
     if (fa.periodic) GM_STEPQ(true, false)
@@ -241,9 +284,10 @@ int gm_step_persistent_blocks(const ForceArgs &fa) {
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick<true>(fa, gtab), kStepThreads, smem) != cudaSuccess)
         return 0;
-    // no more blocks than the tickets (a warp each) or the atoms fill: a
+    // no more blocks than the tickets (a warp each, a block with quad) or the atoms fill: a
     // small system's barrier waits for fewer arrivals
-    const int chunk = ticket_terms<true>(fa), warps = kStepThreads / 32;
+    const bool quad = fa.quad && !gtab;
+    const int chunk = quad ? kStepThreads : ticket_terms<true>(fa), warps = quad ? 1 : kStepThreads / 32;
     const long long tickets = (long long)fa.n_groups * fa.split + bonded_tickets(fa, chunk) + pair14_tickets(fa, chunk);
     const long long fill = (tickets + warps - 1) / warps, atoms = ((long long)fa.n + kStepThreads - 1) / kStepThreads;
     const long long want = fill > atoms ? fill : atoms;
