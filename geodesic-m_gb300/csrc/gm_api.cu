@@ -142,6 +142,11 @@ struct gm_ctx {
     // graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
+    // the persistent form's runs: launches of several steps inside a WHILE node
+    cudaGraph_t loop_graph = nullptr;
+    cudaGraphExec_t loop_exec = nullptr;
+    double loop_dt = 0.0;
+    int loop_cap = -1;
     double graph_dt = 0.0;
     int graph_cap = -1;
     long long launches_per_step = 0;
@@ -658,6 +663,13 @@ int check_status(gm_ctx *c, gm_convergence *conv) {
     return status_result(c, conv);
 }
 
+void drop_graph(gm_ctx *c) {
+    for (cudaGraphExec_t *e : {&c->graph_exec, &c->loop_exec})
+        if (*e) { cudaGraphExecDestroy(*e); *e = nullptr; }
+    for (cudaGraph_t *g : {&c->graph, &c->loop_graph})
+        if (*g) { cudaGraphDestroy(*g); *g = nullptr; }
+}
+
 // The list (cap entries per atom) and the list build's staging area (GM_NSEG
 // z layers of cap_seg entries per atom).
 int ensure_list_buffers(gm_ctx *c, int cap, int cap_seg) {
@@ -677,8 +689,7 @@ int ensure_list_buffers(gm_ctx *c, int cap, int cap_seg) {
         if (rc) return rc;
     }
     // captured graphs hold the old pointer
-    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
-    if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
+    drop_graph(c);
     return GM_OK;
 }
 
@@ -801,18 +812,19 @@ int persistent_grid(gm_ctx *c) {
     return fail(c, GM_ERR_DEVICE, "persistent step kernel: no block fits on an SM");
 }
 
-int begin_persistent(gm_ctx *c, bool fresh) {
+// `todo`: the steps of the call (looping launches).
+int begin_persistent(gm_ctx *c, bool fresh, int64_t todo = 1) {
     int rc = persistent_grid(c);
     if (rc) return rc;
-    GM_CUDA(c, cudaMemsetAsync(c->d_sync, 0, sizeof(StepSync), c->stream));
+    gm_launch_step_begin(c->d_sync, fresh, todo, c->stream);
+    c->launches++;
     if (c->stall_barrier) {
         // the arrival count starts far past the grid: no block is the last to
         // arrive, every block waits out the poll limit and reports the timeout
         GM_CUDA(c, cudaMemsetAsync(&c->d_sync->arrive, 0x40, sizeof(unsigned int), c->stream));
         c->stall_barrier = false;
     }
-    if (fresh) GM_CUDA(c, cudaMemsetAsync(&c->d_sync->fresh, 1, 1, c->stream));
-    else GM_CUDA(c, cudaMemsetAsync(c->d_force, 0, sizeof(long long) * 3 * (size_t)c->n, c->stream));
+    if (!fresh) GM_CUDA(c, cudaMemsetAsync(c->d_force, 0, sizeof(long long) * 3 * (size_t)c->n, c->stream));
     return GM_OK;
 }
 
@@ -828,7 +840,9 @@ int end_persistent(gm_ctx *c) {
 // One BAB + RATTLE step (lib.rs:292-323) issued on stream s.  With a graph
 // conditional handle the rebuild runs inside an IF node; otherwise the check
 // result is read back on the host.
-int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, long long *count) {
+// `loop`: the handle of the WHILE node round the launch (persistent form).
+int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, long long *count,
+               unsigned long long loop = 0ull) {
     long long k = 0;
     const int n = c->n;
     const bool constrained = c->n_clusters > 0;
@@ -849,6 +863,7 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
         sa.thr_sq = half_skin * half_skin;
         sa.far_sq = far_sq(c);
         sa.cond = cond;
+        sa.loop = loop;
         sa.atom_sys = c->d_atom_sys;
         sa.sys_flag = c->d_sys_flag;
         sa.sys_far = c->d_sys_far;
@@ -914,21 +929,9 @@ int issue_step_tail(gm_ctx *c, cudaStream_t s, double dt, long long *count) {
     return GM_OK;
 }
 
-int capture_graph(gm_ctx *c, double dt) {
-    if (c->graph_exec && c->graph_dt == dt && c->graph_cap == c->cap) return GM_OK;
-    if (force_phase(c)) {
-        int rc = persistent_grid(c);  // the grid size goes into the captured launches
-        if (rc) return rc;
-    }
-    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
-    if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
-    cudaGraph_t g;
-    GM_CUDA(c, cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle h;
-    GM_CUDA(c, cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-    GM_CUDA(c, cudaStreamBeginCaptureToGraph(c->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    long long count = 0;
-    issue_step(c, c->stream, dt, (unsigned long long)h, &count);
+// After what c->stream has captured so far: the IF node `h` with the rebuild,
+// and the capture goes on after it.
+int capture_rebuild(gm_ctx *c, cudaGraphConditionalHandle h) {
     cudaStreamCaptureStatus cs;
     const cudaGraphNode_t *deps = nullptr;
     const cudaGraphEdgeData *edges = nullptr;
@@ -947,12 +950,68 @@ int capture_graph(gm_ctx *c, double dt) {
     seq_rebuild(c, c->side, false);
     GM_CUDA(c, cudaStreamEndCapture(c->side, &body));
     GM_CUDA(c, cudaStreamUpdateCaptureDependencies(c->stream, &cnode, nullptr, 1, cudaStreamSetCaptureDependencies));
+    return GM_OK;
+}
+
+int capture_graph(gm_ctx *c, double dt) {
+    if (c->graph_exec && c->graph_dt == dt && c->graph_cap == c->cap) return GM_OK;
+    if (force_phase(c)) {
+        int rc = persistent_grid(c);  // the grid size goes into the captured launches
+        if (rc) return rc;
+    }
+    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
+    if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
+    cudaGraph_t g;
+    GM_CUDA(c, cudaGraphCreate(&g, 0));
+    cudaGraphConditionalHandle h;
+    GM_CUDA(c, cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+    GM_CUDA(c, cudaStreamBeginCaptureToGraph(c->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    long long count = 0;
+    issue_step(c, c->stream, dt, (unsigned long long)h, &count);
+    int rc = capture_rebuild(c, h);
+    if (rc) return rc;
     issue_step_tail(c, c->stream, dt, &count);
     GM_CUDA(c, cudaStreamEndCapture(c->stream, &g));
     GM_CUDA(c, cudaGraphInstantiate(&c->graph_exec, g, 0));
     c->graph = g;
     c->graph_dt = dt;
     c->graph_cap = c->cap;
+    c->launches_per_step = count;
+    return GM_OK;
+}
+
+// The persistent form's run of a call as one graph: WHILE steps are left, a
+// launch of up to GM_LOOP_STEPS steps that ends early when the list has to be
+// rebuilt, and the IF node of the rebuild.
+int capture_loop(gm_ctx *c, double dt) {
+    if (c->loop_exec && c->loop_dt == dt && c->loop_cap == c->cap) return GM_OK;
+    int rc = persistent_grid(c);
+    if (rc) return rc;
+    if (c->loop_exec) { cudaGraphExecDestroy(c->loop_exec); c->loop_exec = nullptr; }
+    if (c->loop_graph) { cudaGraphDestroy(c->loop_graph); c->loop_graph = nullptr; }
+    cudaGraph_t g;
+    GM_CUDA(c, cudaGraphCreate(&g, 0));
+    c->loop_graph = g;
+    cudaGraphConditionalHandle hw, hi;
+    GM_CUDA(c, cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams wp{};
+    wp.type = cudaGraphNodeTypeConditional;
+    wp.conditional.handle = hw;
+    wp.conditional.type = cudaGraphCondTypeWhile;
+    wp.conditional.size = 1;
+    cudaGraphNode_t wnode;
+    GM_CUDA(c, cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp));
+    cudaGraph_t body = wp.conditional.phGraph_out[0];
+    GM_CUDA(c, cudaGraphConditionalHandleCreate(&hi, body, 0, cudaGraphCondAssignDefault));
+    GM_CUDA(c, cudaStreamBeginCaptureToGraph(c->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    long long count = 0;
+    issue_step(c, c->stream, dt, (unsigned long long)hi, &count, (unsigned long long)hw);
+    rc = capture_rebuild(c, hi);
+    if (rc) return rc;
+    GM_CUDA(c, cudaStreamEndCapture(c->stream, &body));
+    GM_CUDA(c, cudaGraphInstantiate(&c->loop_exec, g, 0));
+    c->loop_dt = dt;
+    c->loop_cap = c->cap;
     c->launches_per_step = count;
     return GM_OK;
 }
@@ -969,17 +1028,22 @@ int finish_steps(gm_ctx *c, double dt) {
 
 int run_direct(gm_ctx *c, double dt, int64_t n_steps);
 
-// n resident steps (one graph launch each, or direct launches), then the
+// n resident steps (one graph launch each, one for all of the persistent
+// form's, or direct launches), then the
 // closing half-kick; nothing waits for the device.
 // The steps themselves: after them the resident positions are final (the
 // rest of the call evaluates forces and the closing half-kick).
 int launch_loop(gm_ctx *c, double dt, int64_t n_steps) {
     c->far_marked = false;  // a step may rebuild
     const bool pf = persistent_form(c) && n_steps > 0;
-    int rc = pf ? begin_persistent(c, true) : begin_constrained(c);
+    int rc = pf ? begin_persistent(c, true, n_steps) : begin_constrained(c);
     if (rc) return rc;
     if (!c->use_graph) {
         rc = run_direct(c, dt, n_steps);
+    } else if (pf && gm_step_loops(force_args(c))) {
+        rc = capture_loop(c, dt);
+        if (rc) return rc;
+        GM_CUDA(c, cudaGraphLaunch(c->loop_exec, c->stream));  // (its launches are counted on the device)
     } else {
         rc = capture_graph(c, dt);
         if (rc) return rc;
@@ -1188,11 +1252,6 @@ void build_lanes(const gm_ctx *c, const std::vector<int> &cstart, const std::vec
 // ===================================================================== C ABI
 
 namespace {
-
-void drop_graph(gm_ctx *c) {
-    if (c->graph_exec) { cudaGraphExecDestroy(c->graph_exec); c->graph_exec = nullptr; }
-    if (c->graph) { cudaGraphDestroy(c->graph); c->graph = nullptr; }
-}
 
 int ws_alloc_model(gm_ctx *c) {
     if (c->d_ws_params) return GM_OK;
@@ -1769,8 +1828,7 @@ int32_t gm_destroy(gm_ctx *c) {
     if (!c) return GM_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-    if (c->graph) cudaGraphDestroy(c->graph);
+    drop_graph(c);
     for (void *ptr : c->allocs) cudaFree(ptr);
     if (c->h_status) cudaFreeHost(c->h_status);
     if (c->h_energy) cudaFreeHost(c->h_energy);
@@ -2237,7 +2295,7 @@ int32_t gm_counters(const gm_ctx *cc, int64_t *out, int64_t n) {
     int rc = st_read(c);
     if (rc) return rc;
     const DevStatus st = *c->h_status;
-    int64_t v[12] = {0, (int64_t)st.n_rebuilds, c->cap, c->launches, (int64_t)st.shake_T, (int64_t)st.rattle_T,
+    int64_t v[12] = {0, (int64_t)st.n_rebuilds, c->cap, c->launches + (int64_t)st.c_loops, (int64_t)st.shake_T, (int64_t)st.rattle_T,
                      c->launches_per_step, c->split, (int64_t)st.c_steps, (int64_t)st.shake_sum,
                      (int64_t)st.rattle_sum, (int64_t)st.rec_n};
     if (c->built && n > 0) {

@@ -293,7 +293,7 @@ pair_item_quad(int wid, int warp, int lane, const ForceArgs &fa, const float4 *s
     const bool valid = atom >= 0;
     const int self = valid ? s : 0;
     float4 mh, ml;
-    gm_ld_coord(fa.coord + 2 * self, mh, ml);
+    gm_ld_coord_rw(fa.coord + 2 * self, mh, ml);
     const int cnt = valid ? (inner ? fa.count_in : fa.count)[s] : 0;
     const float4 *trow = s_tab + (valid ? gm_slot_type(ml.w) : 0) * fa.ntypes;
     const gm_df qi = gm_df_make(mh.w, ml.w);
@@ -312,12 +312,12 @@ pair_item_quad(int wid, int warp, int lane, const ForceArgs &fa, const float4 *s
             jj[t] = e < cnt && e < e1 ? __ldg(L + (size_t)e * 32) : self;
         }
         float4 jh, jl, nh, nl;
-        gm_ld_coord(fa.coord + 2 * jj[0], nh, nl);
+        gm_ld_coord_rw(fa.coord + 2 * jj[0], nh, nl);
 #pragma unroll
         for (int t = 0; t < kChunk / 4; t++) {
             jh = nh;
             jl = nl;
-            if (t + 1 < kChunk / 4) gm_ld_coord(fa.coord + 2 * jj[t + 1], nh, nl);  // beside this round's arithmetic
+            if (t + 1 < kChunk / 4) gm_ld_coord_rw(fa.coord + 2 * jj[t + 1], nh, nl);  // beside this round's arithmetic
             float d_h[3], d_l[3];
             const gm_df R = pair_r2<PERIODIC>(mh, ml, jh, jl, k, d_h, d_l);
             const bool in = R.h <= k.rc2 && R.h > 0.f;

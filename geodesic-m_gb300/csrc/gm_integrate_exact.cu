@@ -1132,6 +1132,7 @@ __global__ void status_reset_kernel(DevStatus *st, int set_step, unsigned long l
     z.shake_sum = st->shake_sum;
     z.rattle_sum = st->rattle_sum;
     z.rec_n = st->rec_n;
+    z.c_loops = st->c_loops;
     z.frame_n = st->frame_n;
     z.frame_lost = st->frame_lost;
     z.rebuild_base = keep_base ? st->rebuild_base : st->n_rebuilds;

@@ -87,6 +87,7 @@ struct DevStatus {
     unsigned long long rebuild_base;  // n_rebuilds when the current call's status was reset
     unsigned int frame_n;          // trajectory frames recorded since they were last taken
     unsigned int frame_lost;       // frames due while the ring was full
+    unsigned long long c_loops;    // looping step launches run
 };
 
 struct GridInfo {
@@ -180,6 +181,13 @@ __device__ __forceinline__ void gm_ld_coord(const float4 *p, float4 &h, float4 &
         : "=f"(h.x), "=f"(h.y), "=f"(h.z), "=f"(h.w), "=f"(l.x), "=f"(l.y), "=f"(l.z), "=f"(l.w)
         : "l"(p));
 }
+// The same where the launch itself writes the records (a launch of several
+// steps reads what other blocks wrote before its last grid barrier).
+__device__ __forceinline__ void gm_ld_coord_rw(const float4 *p, float4 &h, float4 &l) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(h.x), "=f"(h.y), "=f"(h.z), "=f"(h.w), "=f"(l.x), "=f"(l.y), "=f"(l.z), "=f"(l.w)
+                 : "l"(p));
+}
 
 // A slot's atom type, kept in the low 8 bits of its Q_lo (the low part of a
 // double-float charge; those bits are below 2^-39 of Q).
@@ -207,6 +215,19 @@ __device__ __forceinline__ unsigned gm_ld_acquire(const unsigned *p) {
 // ~64 ns per poll: about a quarter of a second before a block gives up
 constexpr unsigned GM_BARRIER_POLLS = 1u << 22;
 
+// Waits (one thread) until the barrier generation has left `g`; false, with the
+// timeout recorded, when it did not within GM_BARRIER_POLLS polls.
+__device__ __forceinline__ bool gm_wait_generation(const unsigned *gen, unsigned g, DevStatus *st) {
+    for (unsigned it = 0; gm_ld_acquire(gen) == g; it++) {
+        if (it >= GM_BARRIER_POLLS) {
+            atomicOr(&st->error, (unsigned)GM_DEV_BARRIER_TIMEOUT);
+            return false;
+        }
+        __nanosleep(64);
+    }
+    return true;
+}
+
 // Grid-wide barrier of a cooperative launch (every block is resident).  The
 // generation is read before arriving, the last block to arrive resets the
 // count and advances the generation.  Returns false (and records the
@@ -224,14 +245,7 @@ __device__ __forceinline__ bool gm_grid_barrier(unsigned *arrive, unsigned *gen,
             __threadfence();
             atomicAdd(gen, 1u);
         } else {
-            for (unsigned it = 0; gm_ld_acquire(gen) == g; it++) {
-                if (it >= GM_BARRIER_POLLS) {
-                    atomicOr(&st->error, (unsigned)GM_DEV_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
+            ok = gm_wait_generation(gen, g, st);
         }
         __threadfence();
         s_ok = ok;
@@ -446,13 +460,19 @@ struct StepSync {
     unsigned int gen;     // barrier generation
     unsigned int ticket;  // next work item of the force phase
     unsigned int fresh;   // nonzero: the forces at the current positions are summed already (skip the phase)
+    unsigned int more;    // the launch goes on with another step
+    unsigned int pad;
+    long long todo;       // looping launches: steps left in the call
 };
+// Steps a looping launch runs at most before its graph's WHILE node asks again.
+constexpr int GM_LOOP_STEPS = 64;
 struct StepArgs {
     int n;
     double *pos, *vel, *dref;
     const double *inv_mass, *ref;
     double dt_half, dt, inv_dt, thr_sq, far_sq;
     unsigned long long cond;   // graph conditional handle of the rebuild, or 0
+    unsigned long long loop;   // handle of the WHILE node round a launch of up to GM_LOOP_STEPS steps; 0: one step
     const int *atom_sys;
     unsigned int *sys_flag, *sys_far;
     StepSync *sync;
@@ -492,6 +512,9 @@ void gm_launch_step_persistent(const ForceArgs &fa, const StepArgs &sa, const Pa
 // The persistent kernel's force phase alone, with energies (the force
 // kernels' partials, the same bits), as a plain launch: pair items and bonded
 // / 1-4 blocks from one queue.  The queue words must be zero.
+// Whether the step kernel of these arguments can run several steps a launch.
+bool gm_step_loops(const ForceArgs &a);
+void gm_launch_step_begin(StepSync *sync, bool fresh, long long todo, cudaStream_t s);
 void gm_launch_forces_persistent(const ForceArgs &fa, StepSync *sync, int blocks, cudaStream_t s);
 void gm_launch_kick_drift_check(int n, double *pos, double *vel, double *dref, long long *force,
                                 const double *inv_mass, double dt_half, double dt, const double *ref, double thr_sq,

@@ -118,138 +118,183 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
     StepSync *sy = sa.sync;
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
-    // read by every block before the barrier; block 0 clears it after
+    // read by every block before the first barrier; block 0 clears it after
     const bool fresh = STEP && sy->fresh != 0;
-    // ---- 1. forces at the current positions
-    if (!fresh) {
-        if (!BATCH) {
-            for (int t = threadIdx.x; t < fa.ntypes * fa.ntypes; t += blockDim.x) s_tab[t] = fa.tab32[t];
-            __syncthreads();
-        }
-        if constexpr (QUAD) {
-            quad_phase<PERIODIC, COULOMB, MI, STEP>(fa, s_tab);
-        } else {
-        // tickets: n_pair pair items and nbw bonded tickets (chunk bonded
-        // terms or 1-4 pairs each), the bonded ones at t = k * stride
-        const int n_pair = fa.n_groups * fa.split;
-        const int chunk = ticket_terms<STEP>(fa), cb = bonded_tickets(fa, chunk);
-        const int nbw = cb + pair14_tickets(fa, chunk), total = n_pair + nbw;
-        const int stride = nbw > 0 ? total / nbw : 1;
-        for (;;) {
-            int t = 0;
-            if (lane == 0) t = (int)atomicAdd(&sy->ticket, 1u);
-            t = __shfl_sync(full, t, 0);
-            if (t >= total) break;
-            const int q = t / stride, r = t - q * stride;
-            if (r == 0 && q < nbw) {
-                unsigned bad = 0;
-                const bool b14 = q >= cb;
-                if (STEP) {
-                    int first = -1;
-                    const int base = (b14 ? q - cb : q) * chunk + lane;
-                    for (int u = 0; u < chunk; u += 32) {
-                        if (b14) pair14_term<MI>(fa, base + u, bad, first);
-                        else bonded_term<MI>(fa, base + u, bad, first);
+    const bool loop = STEP && QUAD && sa.loop;
+    const long long todo = loop ? sy->todo : 1;
+    const int steps = (int)(todo < GM_LOOP_STEPS ? todo : GM_LOOP_STEPS);
+    if (loop && blockIdx.x == 0 && threadIdx.x == 0) {
+        // until the last step's bookkeeping says otherwise (a barrier that
+        // times out ends the WHILE node)
+        cudaGraphSetConditional((cudaGraphConditionalHandle)sa.loop, 0u);
+        cudaGraphSetConditional((cudaGraphConditionalHandle)sa.cond, 0u);
+    }
+    if (!BATCH && !(fresh && steps == 1)) {
+        for (int t = threadIdx.x; t < fa.ntypes * fa.ntypes; t += blockDim.x) s_tab[t] = fa.tab32[t];
+        __syncthreads();
+    }
+    for (int k = 0; k < steps; k++) {
+        // ---- 1. forces at the current positions
+        if (!fresh || k > 0) {
+            if constexpr (QUAD) {
+                quad_phase<PERIODIC, COULOMB, MI, STEP>(fa, s_tab);
+            } else {
+            // tickets: n_pair pair items and nbw bonded tickets (chunk bonded
+            // terms or 1-4 pairs each), the bonded ones at t = k * stride
+            const int n_pair = fa.n_groups * fa.split;
+            const int chunk = ticket_terms<STEP>(fa), cb = bonded_tickets(fa, chunk);
+            const int nbw = cb + pair14_tickets(fa, chunk), total = n_pair + nbw;
+            const int stride = nbw > 0 ? total / nbw : 1;
+            for (;;) {
+                int t = 0;
+                if (lane == 0) t = (int)atomicAdd(&sy->ticket, 1u);
+                t = __shfl_sync(full, t, 0);
+                if (t >= total) break;
+                const int q = t / stride, r = t - q * stride;
+                if (r == 0 && q < nbw) {
+                    unsigned bad = 0;
+                    const bool b14 = q >= cb;
+                    if (STEP) {
+                        int first = -1;
+                        const int base = (b14 ? q - cb : q) * chunk + lane;
+                        for (int u = 0; u < chunk; u += 32) {
+                            if (b14) pair14_term<MI>(fa, base + u, bad, first);
+                            else bonded_term<MI>(fa, base + u, bad, first);
+                        }
+                    } else {
+                        const int blk0 = (b14 ? q - cb : q) * (chunk / GM_BONDED_THREADS);
+                        for (int h = 0; h < chunk / GM_BONDED_THREADS; h++) {
+                            if (b14) term_block_warp<MI, true>(fa, blk0 + h, lane, bad);
+                            else term_block_warp<MI, false>(fa, blk0 + h, lane, bad);
+                        }
                     }
+                    bad = __reduce_or_sync(full, bad);
+                    if (bad && lane == 0) atomicOr(&st->error, bad);
                 } else {
-                    const int blk0 = (b14 ? q - cb : q) * (chunk / GM_BONDED_THREADS);
-                    for (int h = 0; h < chunk / GM_BONDED_THREADS; h++) {
-                        if (b14) term_block_warp<MI, true>(fa, blk0 + h, lane, bad);
-                        else term_block_warp<MI, false>(fa, blk0 + h, lane, bad);
+                    // bonded tickets at or before t: min(q + 1, nbw)
+                    const int item = t - min(q + 1, nbw);
+                    pair_item_mixed<PERIODIC, COULOMB, BATCH, !STEP>(
+                        item, lane, fa.n, fa.cap, fa.split, fa.coord, fa.perm, fa.list, fa.count, fa.gmax, fa.count_in,
+                        fa.gmax_in, fa.sys_far, fa.ntypes, fa.tab32, s_tab, fa.pc, fa.force, fa.epart, st, fa.group_sys,
+                        STEP ? nullptr : fa.e_sys);
+                }
+            }
+            }
+        }
+        if (!STEP) {
+            if (QUAD) return;  // no queue
+            // the last warp out leaves the queue words at zero for the next launch
+            if (lane == 0) {
+                __threadfence();
+                const unsigned warps = gridDim.x * (blockDim.x / 32);
+                if (atomicAdd(&sy->arrive, 1u) == warps - 1) {
+                    atomicExch(&sy->ticket, 0u);
+                    atomicExch(&sy->arrive, 0u);
+                }
+            }
+            return;
+        }
+        // ---- 2. every force is summed
+        if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
+        // ---- 3. kick, drift, pack, rebuild check (kick_drift_check_kernel's
+        // operations, one atom at a time)
+        const bool err0 = gm_ld_acquire(&st->error) != 0, tail0 = gm_ld_acquire(&st->tail_pending) != 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            sy->ticket = 0;
+            sy->fresh = 0;
+        }
+        const int n = sa.n;
+        int need = 0, bad = 0;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            double np[3];
+            if (!err0) {
+                const double inv_m = sa.inv_mass[i];
+                for (int d = 0; d < 3; d++) {
+                    const double f = __dmul_rn((double)__ldcg(fa.force + d * n + i), GM_FIX_INV);
+                    const double kick = __dmul_rn(__dmul_rn(__dmul_rn(sa.dt_half, f), inv_m), GM_FORCE_TO_ACCEL);
+                    double v = sa.vel[d * n + i];
+                    if (tail0) v = __dadd_rn(v, kick);
+                    v = __dadd_rn(v, kick);
+                    const double p = sa.pos[d * n + i];
+                    sa.dref[d * n + i] = p;
+                    np[d] = __dadd_rn(p, __dmul_rn(sa.dt, v));
+                    sa.pos[d * n + i] = np[d];
+                    sa.vel[d * n + i] = gm_div_by_dt(__dsub_rn(np[d], p), sa.dt, sa.inv_dt);
+                }
+            } else {
+                for (int d = 0; d < 3; d++) np[d] = sa.pos[d * n + i];
+            }
+            const int sl = pk.slot_of[i];
+            const GridInfo *g = pk.grid + sa.atom_sys[i];
+            gm_pack_record(pk.coord + 2 * sl, __dsub_rn(np[0], g->origin[0]), __dsub_rn(np[1], g->origin[1]),
+                           __dsub_rn(np[2], g->origin[2]), pk.qw[i]);
+            for (int d = 0; d < 3; d++) fa.force[d * n + i] = 0;
+            bad |= !(isfinite(np[0]) && isfinite(np[1]) && isfinite(np[2]));
+            const double dx = __dsub_rn(np[0], sa.ref[i]), dy = __dsub_rn(np[1], sa.ref[n + i]),
+                         dz = __dsub_rn(np[2], sa.ref[2 * n + i]);
+            const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+            const bool moved = d2 > sa.thr_sq;
+            if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sa.atom_sys[i]] = 1u;
+            if (moved) {
+                sa.sys_flag[sa.atom_sys[i]] = 1u;
+                need = 1;
+            }
+        }
+        need = __syncthreads_or(need);
+        bad = __syncthreads_or(bad);
+        // ---- 4. the last block's bookkeeping; with steps left, a second barrier
+        // whose last block decides for all whether to go on (no block reads the
+        // error or rebuild words themselves, which a faster block may set already)
+        const bool last_step = !QUAD || k + 1 == steps;
+        __shared__ int s_more;
+        if (threadIdx.x == 0) {
+            if (need) atomicOr(&st->rebuild, 1u);
+            if (bad) atomicOr(&st->bad_pending, 1u);
+            const unsigned gen = QUAD ? gm_ld_acquire(&sy->gen) : 0u;
+            __threadfence();
+            const unsigned done = atomicAdd(&st->blocks_done, 1u);
+            if (done == gridDim.x - 1) {
+                __threadfence();
+                const unsigned r = atomicOr(&st->rebuild, 0u);
+                st->blocks_done = 0;
+                if (atomicExch(&st->bad_pending, 0u)) atomicOr(&st->error, (unsigned)GM_DEV_NONFINITE_POS);
+                const unsigned e = atomicOr(&st->error, 0u);
+                const bool more = !last_step && !r && !e;
+                if (!more) {
+                    if (sa.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)sa.cond, (r && !e) ? 1u : 0u);
+                    if (loop) {
+                        const long long left = todo - (k + 1);
+                        sy->todo = left;
+                        st->c_loops += 1;
+                        cudaGraphSetConditional((cudaGraphConditionalHandle)sa.loop, (left > 0 && !e) ? 1u : 0u);
                     }
                 }
-                bad = __reduce_or_sync(full, bad);
-                if (bad && lane == 0) atomicOr(&st->error, bad);
+                if (!err0) {
+                    if (tail0) st->step += 1;
+                    st->tail_pending = 1u;
+                }
+                if (loop) {
+                    sy->more = more;
+                    __threadfence();
+                    atomicAdd(&sy->gen, 1u);
+                }
+                s_more = more;
             } else {
-                // bonded tickets at or before t: min(q + 1, nbw)
-                const int item = t - min(q + 1, nbw);
-                pair_item_mixed<PERIODIC, COULOMB, BATCH, !STEP>(
-                    item, lane, fa.n, fa.cap, fa.split, fa.coord, fa.perm, fa.list, fa.count, fa.gmax, fa.count_in,
-                    fa.gmax_in, fa.sys_far, fa.ntypes, fa.tab32, s_tab, fa.pc, fa.force, fa.epart, st, fa.group_sys,
-                    STEP ? nullptr : fa.e_sys);
+                s_more = !last_step && gm_wait_generation(&sy->gen, gen, st) && gm_ld_acquire(&sy->more) != 0;
             }
-        }
-        }
-    }
-    if (!STEP) {
-        if (QUAD) return;  // no queue
-        // the last warp out leaves the queue words at zero for the next launch
-        if (lane == 0) {
             __threadfence();
-            const unsigned warps = gridDim.x * (blockDim.x / 32);
-            if (atomicAdd(&sy->arrive, 1u) == warps - 1) {
-                atomicExch(&sy->ticket, 0u);
-                atomicExch(&sy->arrive, 0u);
-            }
         }
-        return;
+        if (!loop) return;
+        __syncthreads();
+        if (!s_more) return;
     }
-    // ---- 2. every force is summed
-    if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
-    // ---- 3. kick, drift, pack, rebuild check (kick_drift_check_kernel's
-    // operations, one atom at a time)
-    const bool err0 = gm_ld_acquire(&st->error) != 0, tail0 = gm_ld_acquire(&st->tail_pending) != 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        sy->ticket = 0;
-        sy->fresh = 0;
-    }
-    const int n = sa.n;
-    int need = 0, bad = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double np[3];
-        if (!err0) {
-            const double inv_m = sa.inv_mass[i];
-            for (int d = 0; d < 3; d++) {
-                const double f = __dmul_rn((double)__ldcg(fa.force + d * n + i), GM_FIX_INV);
-                const double kick = __dmul_rn(__dmul_rn(__dmul_rn(sa.dt_half, f), inv_m), GM_FORCE_TO_ACCEL);
-                double v = sa.vel[d * n + i];
-                if (tail0) v = __dadd_rn(v, kick);
-                v = __dadd_rn(v, kick);
-                const double p = sa.pos[d * n + i];
-                sa.dref[d * n + i] = p;
-                np[d] = __dadd_rn(p, __dmul_rn(sa.dt, v));
-                sa.pos[d * n + i] = np[d];
-                sa.vel[d * n + i] = gm_div_by_dt(__dsub_rn(np[d], p), sa.dt, sa.inv_dt);
-            }
-        } else {
-            for (int d = 0; d < 3; d++) np[d] = sa.pos[d * n + i];
-        }
-        const int sl = pk.slot_of[i];
-        const GridInfo *g = pk.grid + sa.atom_sys[i];
-        gm_pack_record(pk.coord + 2 * sl, __dsub_rn(np[0], g->origin[0]), __dsub_rn(np[1], g->origin[1]),
-                       __dsub_rn(np[2], g->origin[2]), pk.qw[i]);
-        for (int d = 0; d < 3; d++) fa.force[d * n + i] = 0;
-        bad |= !(isfinite(np[0]) && isfinite(np[1]) && isfinite(np[2]));
-        const double dx = __dsub_rn(np[0], sa.ref[i]), dy = __dsub_rn(np[1], sa.ref[n + i]),
-                     dz = __dsub_rn(np[2], sa.ref[2 * n + i]);
-        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-        const bool moved = d2 > sa.thr_sq;
-        if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sa.atom_sys[i]] = 1u;
-        if (moved) {
-            sa.sys_flag[sa.atom_sys[i]] = 1u;
-            need = 1;
-        }
-    }
-    need = __syncthreads_or(need);
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) {
-        if (need) atomicOr(&st->rebuild, 1u);
-        if (bad) atomicOr(&st->bad_pending, 1u);
-        __threadfence();
-        const unsigned done = atomicAdd(&st->blocks_done, 1u);
-        if (done == gridDim.x - 1) {
-            __threadfence();
-            const unsigned r = atomicOr(&st->rebuild, 0u);
-            st->blocks_done = 0;
-            if (atomicExch(&st->bad_pending, 0u)) atomicOr(&st->error, (unsigned)GM_DEV_NONFINITE_POS);
-            const unsigned e = atomicOr(&st->error, 0u);
-            if (sa.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)sa.cond, (r && !e) ? 1u : 0u);
-            if (!err0) {
-                if (tail0) st->step += 1;
-                st->tail_pending = 1u;
-            }
-        }
-    }
+}
+
+__global__ void step_begin_kernel(StepSync *sy, unsigned fresh, long long todo) {
+    StepSync z{};
+    z.fresh = fresh;
+    z.todo = todo;
+    *sy = z;
 }
 
 using StepKernel = void (*)(ForceArgs, StepArgs, PackArgs);
@@ -275,6 +320,8 @@ bool global_table(const ForceArgs &fa) {
 }
 
 }  // namespace
+
+bool gm_step_loops(const ForceArgs &fa) { return fa.quad && !global_table(fa); }
 
 int gm_step_persistent_blocks(const ForceArgs &fa) {
     const bool gtab = global_table(fa);
@@ -317,4 +364,8 @@ void gm_launch_forces_persistent(const ForceArgs &fa, StepSync *sync, int blocks
     PackArgs pk{};
     const size_t smem = gtab ? 0 : sizeof(float4) * (size_t)fa.ntypes * fa.ntypes;
     pick<false>(fa, gtab)<<<blocks, kStepThreads, smem, s>>>(fa, sa, pk);
+}
+
+void gm_launch_step_begin(StepSync *sync, bool fresh, long long todo, cudaStream_t s) {
+    step_begin_kernel<<<1, 1, 0, s>>>(sync, fresh ? 1u : 0u, todo);
 }
