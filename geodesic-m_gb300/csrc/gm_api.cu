@@ -448,8 +448,8 @@ int seq_rebuild(gm_ctx *c, cudaStream_t s, bool all) {
     gm_launch_build(a, s);
     gm_launch_flags(a, false, s);
     // [flags], wrap or bbox, grid (clears the cells), assign, scan, scatter,
-    // rank, pack, build, clear flags
-    return (all ? 1 : 0) + 9 + (a.periodic || a.n > 0 ? 1 : 0);
+    // rank, pack, build and its second kernel, clear flags
+    return (all ? 1 : 0) + 10 + (a.periodic || a.n > 0 ? 1 : 0);
 }
 
 bool persistent_form(const gm_ctx *c);

@@ -87,6 +87,7 @@ struct DevStatus {
     unsigned long long rebuild_base;  // n_rebuilds when the current call's status was reset
     unsigned int frame_n;          // trajectory frames recorded since they were last taken
     unsigned int frame_lost;       // frames due while the ring was full
+    unsigned int stage_over;       // list groups whose staged words did not fit (built by the second kernel)
     unsigned long long c_loops;    // looping step launches run
 };
 

@@ -423,6 +423,8 @@ constexpr int kRound = 256, kRoundY = 64;
 // Rows of 32 ints that 32 candidates (a word) take in the staging buffer: their
 // slots, then each lane's accept mask and the two bits of its bucket masks.
 constexpr int kWordRows = 4;
+// gmax of a group whose words did not fit the staging area
+constexpr int kStageOver = -1;
 // Groups (per system) up to which the build splits a layer's y rows over
 // warps: 162 groups 125 us against 191, 48 groups 66 against 144; 750 groups
 // 291 against 259, 3,072 groups 921 against 793 (partly filled words).
@@ -456,9 +458,13 @@ constexpr int kYSplitGroups = 300;
 // the switch band, the shell beyond the cutoff.  Within a bucket the entries
 // keep the single-warp sweep order.  The pair kernel's lanes then meet the
 // same kind of pair at the same entry and branch together.
-template <bool PERIODIC, int YS>
-__global__ void __launch_bounds__(GM_NSEG * YS * 32, YS == 1 ? 5 : 1)
-build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucket_r2) {
+//   * A warp that meets more words than its staging area holds (the area is
+//     sized from the mean density and the first lists, and a resident run
+//     cannot grow it) marks its group; the kernel after it (AGAIN) sweeps a
+//     marked group twice instead, to count and to write, in the same order.
+template <bool PERIODIC, int YS, bool AGAIN>
+__device__ __forceinline__ void build_group(const ListArgs &a, int group, float rl2_lo, float rl2_hi, double rl2_64,
+                                            float3 bucket_r2) {
     // the round's candidates: coordinates relative to the group's first atom
     // (FP32; the rounding, under 1e-5 A for candidates within a few list
     // radii, stays far inside the FP64 re-decision margin) and slot; the
@@ -468,11 +474,12 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
     __shared__ int s_cnt[NSEG][GM_NBUCKET][32];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int group = blockIdx.x, seg = wib;
+    const int seg = wib;
     const int gseg = group * NSEG + seg;
     if (group * 32 >= a.n_slots) return;
     const int sys = a.group_sys[group];
     if (!a.sys_flag[sys]) return;  // block-uniform: the system keeps its list
+    if (AGAIN && a.gmax[group] != kStageOver) return;
     const int soff = a.sys_slot_off[sys], coff = a.sys_cell_off[sys];
     const int ns = a.sys_atom_off[sys + 1] - a.sys_atom_off[sys];
     const int s = group * 32 + lane;
@@ -528,228 +535,251 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
     int nb[GM_NBUCKET] = {0, 0, 0, 0};  // accepted entries per bucket
     const double bx[3] = {a.box[0], a.box[1], a.box[2]};
     const float slack = 1e-3f + (PERIODIC ? 2e-7f * fmaxf(g.box[0], fmaxf(g.box[1], g.box[2])) : 0.f);
-    unsigned remaining = __ballot_sync(full, valid);
-    while (remaining) {
-        const int leader = __ffs(remaining) - 1;
-        const int R = __shfl_sync(full, row_id, leader);
-        bool mine = valid && row_id == R;
-        int ymin = R % g.nc[1], ymax = ymin;
-        const int zR = R / g.nc[1];
-        int xmin, xmax;
-        if (!PERIODIC) {
-            // Near a droplet's surface 32 atoms may lie in many short rows of
-            // one layer: one sweep over all of them when it visits fewer cells
-            // (a row's own box is about 5 x 6 cells).  Candidates keep their
-            // order; the extra ones are out of reach of the lanes they are
-            // new to.
-            const bool layer = valid && cz == zR && ((remaining >> lane) & 1u);
-            const unsigned peers = __match_any_sync(full, layer ? row_id : -1 - lane);
-            const int rows = __popc(__ballot_sync(full, layer && (peers & ((1u << lane) - 1u)) == 0));
-            ymin = __reduce_min_sync(full, layer ? cy : INT_MAX);
-            ymax = __reduce_max_sync(full, layer ? cy : INT_MIN);
-            xmin = __reduce_min_sync(full, layer ? cx : INT_MAX);
-            xmax = __reduce_max_sync(full, layer ? cx : INT_MIN);
-            if (rows > 1 && ymax - ymin < 28 && (xmax - xmin + 5) * (ymax - ymin + 5) <= 30 * rows) mine = layer;
-            else ymin = ymax = R % g.nc[1];
-        }
-        remaining &= ~__ballot_sync(full, mine);
-        xmin = __reduce_min_sync(full, mine ? cx : INT_MAX);
-        xmax = __reduce_max_sync(full, mine ? cx : INT_MIN);
-        Range rx = dim_range(xmin, xmax, g.nc[0], g.periodic, g.full[0]);
-        Range ry = dim_range(ymin, ymax, g.nc[1], g.periodic, g.full[1]);
-        Range rz = dim_range(zR, zR, g.nc[2], g.periodic, g.full[2]);
-        if (YS > 1) {
-            const int per = (ry.hi - ry.lo + YS) / YS;
-            ry.lo += seg % YS * per;
-            ry.hi = min(ry.hi, ry.lo + per - 1);
-        }
-        const int zz = rz.lo + seg / YS;
-        if (zz > rz.hi || ry.lo > ry.hi) continue;  // warp-uniform
-        const int z = rz.wrap ? wrapi(zz, g.nc[2]) : zz;
-        // the lanes' bounding box
-        const float lox = warp_min(mine ? mx : FLT_MAX), hix = warp_max(mine ? mx : -FLT_MAX);
-        const float loy = warp_min(mine ? my : FLT_MAX), hiy = warp_max(mine ? my : -FLT_MAX);
-        const float loz = warp_min(mine ? mz : FLT_MAX), hiz = warp_max(mine ? mz : -FLT_MAX);
-        const float bcx = 0.5f * (lox + hix), bcy = 0.5f * (loy + hiy), bcz = 0.5f * (loz + hiz);
-        // half extents, wider by the FP32 roundings of the tests below
-        const float bhx = 0.5f * (hix - lox) + slack, bhy = 0.5f * (hiy - loy) + slack, bhz = 0.5f * (hiz - loz) + slack;
-        // The x extent of each y row as one or two runs of consecutive cells
-        // (at most 32): lane r holds the slots [run_b, run_e) of run r.
-        int x0[2], x1[2], nrun = 1;
-        x0[0] = rx.lo; x1[0] = rx.hi; x0[1] = 0; x1[1] = -1;
-        if (rx.wrap && rx.lo < 0) { x0[0] = rx.lo + g.nc[0]; x1[0] = g.nc[0] - 1; x0[1] = 0; x1[1] = rx.hi; nrun = 2; }
-        else if (rx.wrap && rx.hi >= g.nc[0]) { x1[0] = g.nc[0] - 1; x0[1] = 0; x1[1] = rx.hi - g.nc[0]; nrun = 2; }
-        const int runs = (ry.hi - ry.lo + 1) * nrun;
-        int run_b = 0, run_e = 0;
-        if (lane < runs) {
-            const int yy = ry.lo + lane / nrun, sg = lane - lane / nrun * nrun;
-            const int row = (z * g.nc[1] + (ry.wrap ? wrapi(yy, g.nc[1]) : yy)) * g.nc[0];
-            run_b = soff + cell_start[row + x0[sg]];
-            run_e = soff + cell_start[row + x1[sg] + 1];
-        }
-        int run = 0, base = __shfl_sync(full, run_b, 0), end = __shfl_sync(full, run_e, 0);
-        int held = 0;               // candidates of the round
-        bool image = false;         // periodic: one of them may need the image
-        for (;;) {
-            while (base >= end && ++run < runs) {
-                base = __shfl_sync(full, run_b, run);
-                end = __shfl_sync(full, run_e, run);
-            }
-            const bool more = run < runs;
-            if (more) {
-                const int t = base + lane;
-                base += 32;
-                float4 c = make_float4(0.f, 0.f, 0.f, __int_as_float(t));
-                bool keep = false, far = false;
-                if (t < end) {
-                    float4 ch, cl;
-                    gm_ld_coord(a.coord + 2 * t, ch, cl);
-                    c.x = (ch.x - rh.x) + (cl.x - rl.x);
-                    c.y = (ch.y - rh.y) + (cl.y - rl.y);
-                    c.z = (ch.z - rh.z) + (cl.z - rl.z);
-                    float dx = c.x - bcx, dy = c.y - bcy, dz = c.z - bcz;
-                    if (PERIODIC) {
-                        // a raw difference below half the box from every lane
-                        // of the bounding box needs no image
-                        far = fabsf(dx) + bhx >= 0.49f * g.box[0] || fabsf(dy) + bhy >= 0.49f * g.box[1] ||
-                              fabsf(dz) + bhz >= 0.49f * g.box[2];
-                        dx = fmaf(-g.box[0], rintf(dx * g.inv_box[0]), dx);
-                        dy = fmaf(-g.box[1], rintf(dy * g.inv_box[1]), dy);
-                        dz = fmaf(-g.box[2], rintf(dz * g.inv_box[2]), dz);
-                    }
-                    keep = beyond2(dx, bhx) + beyond2(dy, bhy) + beyond2(dz, bhz) <= rl2_hi;
-                }
-                const unsigned kept = __ballot_sync(full, keep);
-                if (keep) s_rel[wib][held + __popc(kept & ((1u << lane) - 1u))] = c;
-                held += __popc(kept);
-                if (PERIODIC) image |= __any_sync(full, keep && far);
-            }
-            if (more && held <= ROUND - 32) continue;
-            if (held == 0) break;
-            // ---- a round: all lanes test, 32 candidates a word
-            __syncwarp();
-            for (int w0 = 0; w0 < held; w0 += 32) {
-                unsigned acc = 0, blo = 0, bhi = 0, look = 0;
-                auto test = [&](float r2, int k) {
-                    const bool in = r2 <= rl2_hi, far1 = r2 > bucket_r2.y;
-                    acc |= (in ? 1u : 0u) << k;
-                    bhi |= (far1 ? 1u : 0u) << k;
-                    blo |= (r2 > (far1 ? bucket_r2.z : bucket_r2.x) ? 1u : 0u) << k;
-                    look |= (in && (r2 > rl2_lo || r2 <= ex_r2) ? 1u : 0u) << k;
-                };
-                if (PERIODIC && image) {
-#pragma unroll
-                    for (int k = 0; k < 32; k++) test(rel_r2<true>(s_rel[wib][w0 + k], mx, my, mz, g), k);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 32; k++) test(rel_r2<false>(s_rel[wib][w0 + k], mx, my, mz, g), k);
-                }
-                const int m = held - w0;
-                const unsigned live = !mine ? 0u : m < 32 ? (1u << m) - 1u : full;
-                acc &= live;
-                look &= live;
-                while (look) {
-                    const int k = __ffs(look) - 1;
-                    look &= look - 1;
-                    const float4 c = s_rel[wib][w0 + k];
-                    const int slot = __float_as_int(c.w);
-                    const float r2 = rel_r2<PERIODIC>(c, mx, my, mz, g);
-                    bool drop = false;
-                    if (r2 > rl2_lo) {
-                        // the reference's own FP64 decision
-                        const int jo = a.perm[slot];
-                        double ex_ = gm_min_image(__dsub_rn(a.pos[jo], a.pos[my_orig]), bx[0]);
-                        double ey_ = gm_min_image(__dsub_rn(a.pos[n + jo], a.pos[n + my_orig]), bx[1]);
-                        double ez_ = gm_min_image(__dsub_rn(a.pos[2 * n + jo], a.pos[2 * n + my_orig]), bx[2]);
-                        double rr = __dadd_rn(__dadd_rn(__dmul_rn(ex_, ex_), __dmul_rn(ey_, ey_)), __dmul_rn(ez_, ez_));
-                        drop = !(rr <= rl2_64);
-                    }
-                    if (r2 <= ex_r2) {
-                        drop |= slot == s;
-#pragma unroll
-                        for (int q = 0; q < 8; q++) drop |= ex[q] == slot;
-                        for (int q = e0 + 8; q < e1; q++) drop |= a.slot_of[a.excl[q]] == slot;
-                    }
-                    if (drop) acc &= ~(1u << k);
-                }
-                if (n_words < cap_words) {  // (else flagged below, and not counted either)
-                    nb[0] += __popc(acc & ~(blo | bhi));
-                    nb[1] += __popc(acc & blo & ~bhi);
-                    nb[2] += __popc(acc & bhi & ~blo);
-                    nb[3] += __popc(acc & blo & bhi);
-                    int *row = stage + (size_t)n_words * (kWordRows * 32);
-                    row[0] = __float_as_int(s_rel[wib][w0 + lane].w);
-                    row[32] = (int)acc;
-                    row[64] = (int)blo;
-                    row[96] = (int)bhi;
-                }
-                n_words++;
-            }
-            __syncwarp();
-            held = 0;
-            image = false;
-            if (!more) break;
-        }
-    }
-    // the layers' entries go into the column one layer after the other
-    if (lane == 0) atomicMax(&a.status->max_layer, (unsigned)(n_words * kWordRows * YS));
-    const bool over = n_words > cap_words;
-    n_words = min(n_words, cap_words);
-#pragma unroll
-    for (int q = 0; q < GM_NBUCKET; q++) s_cnt[seg][q][lane] = nb[q];
-    __syncthreads();
-    // this layer's first position in each bucket: the earlier buckets of all
-    // layers, then this bucket of the earlier layers
+    int *my_list = a.list + (size_t)group * 32 * cap + lane;
     int off[GM_NBUCKET];
     int total = 0, inner = 0;  // inner: without the last bucket
-#pragma unroll
-    for (int q = 0; q < GM_NBUCKET; q++) {
-        int before = 0, all = 0;
-#pragma unroll
-        for (int k = 0; k < NSEG; k++) {
-            const int ck = s_cnt[k][q][lane];
-            before += k < seg ? ck : 0;
-            all += ck;
-        }
-        off[q] = total + before;
-        inner = total;
-        total += all;
-    }
-    int *my_list = a.list + (size_t)group * 32 * cap + lane;
-    constexpr int WB = ROUND / 32;  // words at a time: [row][word][lane]
-    int *buf = reinterpret_cast<int *>(s_rel[wib]);
-    for (int w0 = 0; w0 < n_words; w0 += WB) {
-        const int words = min(WB, n_words - w0);
-        __syncwarp();
-        const int *row = stage + (size_t)w0 * (kWordRows * 32);
-        int v[WB * kWordRows];
-#pragma unroll
-        for (int k = 0; k < WB * kWordRows; k++) v[k] = k < words * kWordRows ? row[k * 32] : 0;
-#pragma unroll
-        for (int k = 0; k < WB * kWordRows; k++) buf[((k % kWordRows) * WB + k / kWordRows) * 32 + lane] = v[k];
-        __syncwarp();
-        int w = 0;
-        unsigned acc = (unsigned)buf[WB * 32 + lane], blo = (unsigned)buf[2 * WB * 32 + lane],
-                 bhi = (unsigned)buf[3 * WB * 32 + lane];
-        for (;;) {
-            while (acc == 0 && ++w < words) {
-                acc = (unsigned)buf[(WB + w) * 32 + lane];
-                blo = (unsigned)buf[(2 * WB + w) * 32 + lane];
-                bhi = (unsigned)buf[(3 * WB + w) * 32 + lane];
+    for (int pass = 0;; pass++) {  // one sweep, or with AGAIN two
+        unsigned remaining = __ballot_sync(full, valid);
+        while (remaining) {
+            const int leader = __ffs(remaining) - 1;
+            const int R = __shfl_sync(full, row_id, leader);
+            bool mine = valid && row_id == R;
+            int ymin = R % g.nc[1], ymax = ymin;
+            const int zR = R / g.nc[1];
+            int xmin, xmax;
+            if (!PERIODIC) {
+                // Near a droplet's surface 32 atoms may lie in many short rows of
+                // one layer: one sweep over all of them when it visits fewer cells
+                // (a row's own box is about 5 x 6 cells).  Candidates keep their
+                // order; the extra ones are out of reach of the lanes they are
+                // new to.
+                const bool layer = valid && cz == zR && ((remaining >> lane) & 1u);
+                const unsigned peers = __match_any_sync(full, layer ? row_id : -1 - lane);
+                const int rows = __popc(__ballot_sync(full, layer && (peers & ((1u << lane) - 1u)) == 0));
+                ymin = __reduce_min_sync(full, layer ? cy : INT_MAX);
+                ymax = __reduce_max_sync(full, layer ? cy : INT_MIN);
+                xmin = __reduce_min_sync(full, layer ? cx : INT_MAX);
+                xmax = __reduce_max_sync(full, layer ? cx : INT_MIN);
+                if (rows > 1 && ymax - ymin < 28 && (xmax - xmin + 5) * (ymax - ymin + 5) <= 30 * rows) mine = layer;
+                else ymin = ymax = R % g.nc[1];
             }
-            if (acc == 0) break;
-            const int k = __ffs(acc) - 1;
-            acc &= acc - 1;
-            const int bk = ((blo >> k) & 1u) + 2 * ((bhi >> k) & 1u);
-            int pos = 0;
-#pragma unroll
-            for (int q = 0; q < GM_NBUCKET; q++) {
-                if (bk == q) { pos = off[q]; off[q]++; }
+            remaining &= ~__ballot_sync(full, mine);
+            xmin = __reduce_min_sync(full, mine ? cx : INT_MAX);
+            xmax = __reduce_max_sync(full, mine ? cx : INT_MIN);
+            Range rx = dim_range(xmin, xmax, g.nc[0], g.periodic, g.full[0]);
+            Range ry = dim_range(ymin, ymax, g.nc[1], g.periodic, g.full[1]);
+            Range rz = dim_range(zR, zR, g.nc[2], g.periodic, g.full[2]);
+            if (YS > 1) {
+                const int per = (ry.hi - ry.lo + YS) / YS;
+                ry.lo += seg % YS * per;
+                ry.hi = min(ry.hi, ry.lo + per - 1);
             }
-            if (pos < cap) my_list[(size_t)pos * 32] = buf[w * 32 + k];
+            const int zz = rz.lo + seg / YS;
+            if (zz > rz.hi || ry.lo > ry.hi) continue;  // warp-uniform
+            const int z = rz.wrap ? wrapi(zz, g.nc[2]) : zz;
+            // the lanes' bounding box
+            const float lox = warp_min(mine ? mx : FLT_MAX), hix = warp_max(mine ? mx : -FLT_MAX);
+            const float loy = warp_min(mine ? my : FLT_MAX), hiy = warp_max(mine ? my : -FLT_MAX);
+            const float loz = warp_min(mine ? mz : FLT_MAX), hiz = warp_max(mine ? mz : -FLT_MAX);
+            const float bcx = 0.5f * (lox + hix), bcy = 0.5f * (loy + hiy), bcz = 0.5f * (loz + hiz);
+            // half extents, wider by the FP32 roundings of the tests below
+            const float bhx = 0.5f * (hix - lox) + slack, bhy = 0.5f * (hiy - loy) + slack, bhz = 0.5f * (hiz - loz) + slack;
+            // The x extent of each y row as one or two runs of consecutive cells
+            // (at most 32): lane r holds the slots [run_b, run_e) of run r.
+            int x0[2], x1[2], nrun = 1;
+            x0[0] = rx.lo; x1[0] = rx.hi; x0[1] = 0; x1[1] = -1;
+            if (rx.wrap && rx.lo < 0) { x0[0] = rx.lo + g.nc[0]; x1[0] = g.nc[0] - 1; x0[1] = 0; x1[1] = rx.hi; nrun = 2; }
+            else if (rx.wrap && rx.hi >= g.nc[0]) { x1[0] = g.nc[0] - 1; x0[1] = 0; x1[1] = rx.hi - g.nc[0]; nrun = 2; }
+            const int runs = (ry.hi - ry.lo + 1) * nrun;
+            int run_b = 0, run_e = 0;
+            if (lane < runs) {
+                const int yy = ry.lo + lane / nrun, sg = lane - lane / nrun * nrun;
+                const int row = (z * g.nc[1] + (ry.wrap ? wrapi(yy, g.nc[1]) : yy)) * g.nc[0];
+                run_b = soff + cell_start[row + x0[sg]];
+                run_e = soff + cell_start[row + x1[sg] + 1];
+            }
+            int run = 0, base = __shfl_sync(full, run_b, 0), end = __shfl_sync(full, run_e, 0);
+            int held = 0;               // candidates of the round
+            bool image = false;         // periodic: one of them may need the image
+            for (;;) {
+                while (base >= end && ++run < runs) {
+                    base = __shfl_sync(full, run_b, run);
+                    end = __shfl_sync(full, run_e, run);
+                }
+                const bool more = run < runs;
+                if (more) {
+                    const int t = base + lane;
+                    base += 32;
+                    float4 c = make_float4(0.f, 0.f, 0.f, __int_as_float(t));
+                    bool keep = false, far = false;
+                    if (t < end) {
+                        float4 ch, cl;
+                        gm_ld_coord(a.coord + 2 * t, ch, cl);
+                        c.x = (ch.x - rh.x) + (cl.x - rl.x);
+                        c.y = (ch.y - rh.y) + (cl.y - rl.y);
+                        c.z = (ch.z - rh.z) + (cl.z - rl.z);
+                        float dx = c.x - bcx, dy = c.y - bcy, dz = c.z - bcz;
+                        if (PERIODIC) {
+                            // a raw difference below half the box from every lane
+                            // of the bounding box needs no image
+                            far = fabsf(dx) + bhx >= 0.49f * g.box[0] || fabsf(dy) + bhy >= 0.49f * g.box[1] ||
+                                  fabsf(dz) + bhz >= 0.49f * g.box[2];
+                            dx = fmaf(-g.box[0], rintf(dx * g.inv_box[0]), dx);
+                            dy = fmaf(-g.box[1], rintf(dy * g.inv_box[1]), dy);
+                            dz = fmaf(-g.box[2], rintf(dz * g.inv_box[2]), dz);
+                        }
+                        keep = beyond2(dx, bhx) + beyond2(dy, bhy) + beyond2(dz, bhz) <= rl2_hi;
+                    }
+                    const unsigned kept = __ballot_sync(full, keep);
+                    if (keep) s_rel[wib][held + __popc(kept & ((1u << lane) - 1u))] = c;
+                    held += __popc(kept);
+                    if (PERIODIC) image |= __any_sync(full, keep && far);
+                }
+                if (more && held <= ROUND - 32) continue;
+                if (held == 0) break;
+                // ---- a round: all lanes test, 32 candidates a word
+                __syncwarp();
+                for (int w0 = 0; w0 < held; w0 += 32) {
+                    unsigned acc = 0, blo = 0, bhi = 0, look = 0;
+                    auto test = [&](float r2, int k) {
+                        const bool in = r2 <= rl2_hi, far1 = r2 > bucket_r2.y;
+                        acc |= (in ? 1u : 0u) << k;
+                        bhi |= (far1 ? 1u : 0u) << k;
+                        blo |= (r2 > (far1 ? bucket_r2.z : bucket_r2.x) ? 1u : 0u) << k;
+                        look |= (in && (r2 > rl2_lo || r2 <= ex_r2) ? 1u : 0u) << k;
+                    };
+                    if (PERIODIC && image) {
+#pragma unroll
+                        for (int k = 0; k < 32; k++) test(rel_r2<true>(s_rel[wib][w0 + k], mx, my, mz, g), k);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 32; k++) test(rel_r2<false>(s_rel[wib][w0 + k], mx, my, mz, g), k);
+                    }
+                    const int m = held - w0;
+                    const unsigned live = !mine ? 0u : m < 32 ? (1u << m) - 1u : full;
+                    acc &= live;
+                    look &= live;
+                    while (look) {
+                        const int k = __ffs(look) - 1;
+                        look &= look - 1;
+                        const float4 c = s_rel[wib][w0 + k];
+                        const int slot = __float_as_int(c.w);
+                        const float r2 = rel_r2<PERIODIC>(c, mx, my, mz, g);
+                        bool drop = false;
+                        if (r2 > rl2_lo) {
+                            // the reference's own FP64 decision
+                            const int jo = a.perm[slot];
+                            double ex_ = gm_min_image(__dsub_rn(a.pos[jo], a.pos[my_orig]), bx[0]);
+                            double ey_ = gm_min_image(__dsub_rn(a.pos[n + jo], a.pos[n + my_orig]), bx[1]);
+                            double ez_ = gm_min_image(__dsub_rn(a.pos[2 * n + jo], a.pos[2 * n + my_orig]), bx[2]);
+                            double rr = __dadd_rn(__dadd_rn(__dmul_rn(ex_, ex_), __dmul_rn(ey_, ey_)), __dmul_rn(ez_, ez_));
+                            drop = !(rr <= rl2_64);
+                        }
+                        if (r2 <= ex_r2) {
+                            drop |= slot == s;
+#pragma unroll
+                            for (int q = 0; q < 8; q++) drop |= ex[q] == slot;
+                            for (int q = e0 + 8; q < e1; q++) drop |= a.slot_of[a.excl[q]] == slot;
+                        }
+                        if (drop) acc &= ~(1u << k);
+                    }
+                    if (AGAIN && pass == 1) {
+                        while (acc) {
+                            const int k = __ffs(acc) - 1;
+                            acc &= acc - 1;
+                            const int bk = ((blo >> k) & 1u) + 2 * ((bhi >> k) & 1u);
+                            int pos = 0;
+#pragma unroll
+                            for (int q = 0; q < GM_NBUCKET; q++) {
+                                if (bk == q) { pos = off[q]; off[q]++; }
+                            }
+                            if (pos < cap) my_list[(size_t)pos * 32] = __float_as_int(s_rel[wib][w0 + k].w);
+                        }
+                    } else if (AGAIN || n_words < cap_words) {  // (else the group is marked below)
+                        nb[0] += __popc(acc & ~(blo | bhi));
+                        nb[1] += __popc(acc & blo & ~bhi);
+                        nb[2] += __popc(acc & bhi & ~blo);
+                        nb[3] += __popc(acc & blo & bhi);
+                        if (!AGAIN) {
+                            int *row = stage + (size_t)n_words * (kWordRows * 32);
+                            row[0] = __float_as_int(s_rel[wib][w0 + lane].w);
+                            row[32] = (int)acc;
+                            row[64] = (int)blo;
+                            row[96] = (int)bhi;
+                        }
+                    }
+                    n_words++;
+                }
+                __syncwarp();
+                held = 0;
+                image = false;
+                if (!more) break;
+            }
         }
+        // the layers' entries go into the column one layer after the other
+        if (AGAIN && pass == 1) break;
+        if (!AGAIN && lane == 0) atomicMax(&a.status->max_layer, (unsigned)(n_words * kWordRows * YS));
+        const bool over = !AGAIN && n_words > cap_words;
+#pragma unroll
+        for (int q = 0; q < GM_NBUCKET; q++) s_cnt[seg][q][lane] = nb[q];
+        if (__syncthreads_or(over)) {
+            if (threadIdx.x == 0) {
+                a.gmax[group] = kStageOver;
+                atomicOr(&a.status->stage_over, 1u);
+            }
+            return;
+        }
+        // this layer's first position in each bucket: the earlier buckets of all
+        // layers, then this bucket of the earlier layers
+#pragma unroll
+        for (int q = 0; q < GM_NBUCKET; q++) {
+            int before = 0, all = 0;
+#pragma unroll
+            for (int k = 0; k < NSEG; k++) {
+                const int ck = s_cnt[k][q][lane];
+                before += k < seg ? ck : 0;
+                all += ck;
+            }
+            off[q] = total + before;
+            inner = total;
+            total += all;
+        }
+        if (AGAIN) continue;
+        constexpr int WB = ROUND / 32;  // words at a time: [row][word][lane]
+        int *buf = reinterpret_cast<int *>(s_rel[wib]);
+        for (int w0 = 0; w0 < n_words; w0 += WB) {
+            const int words = min(WB, n_words - w0);
+            __syncwarp();
+            const int *row = stage + (size_t)w0 * (kWordRows * 32);
+            int v[WB * kWordRows];
+#pragma unroll
+            for (int k = 0; k < WB * kWordRows; k++) v[k] = k < words * kWordRows ? row[k * 32] : 0;
+#pragma unroll
+            for (int k = 0; k < WB * kWordRows; k++) buf[((k % kWordRows) * WB + k / kWordRows) * 32 + lane] = v[k];
+            __syncwarp();
+            int w = 0;
+            unsigned acc = (unsigned)buf[WB * 32 + lane], blo = (unsigned)buf[2 * WB * 32 + lane],
+                     bhi = (unsigned)buf[3 * WB * 32 + lane];
+            for (;;) {
+                while (acc == 0 && ++w < words) {
+                    acc = (unsigned)buf[(WB + w) * 32 + lane];
+                    blo = (unsigned)buf[(2 * WB + w) * 32 + lane];
+                    bhi = (unsigned)buf[(3 * WB + w) * 32 + lane];
+                }
+                if (acc == 0) break;
+                const int k = __ffs(acc) - 1;
+                acc &= acc - 1;
+                const int bk = ((blo >> k) & 1u) + 2 * ((bhi >> k) & 1u);
+                int pos = 0;
+#pragma unroll
+                for (int q = 0; q < GM_NBUCKET; q++) {
+                    if (bk == q) { pos = off[q]; off[q]++; }
+                }
+                if (pos < cap) my_list[(size_t)pos * 32] = buf[w * 32 + k];
+            }
+        }
+        break;
     }
-    if (over && lane == 0) atomicOr(&a.status->error, (unsigned)GM_DEV_LIST_OVERFLOW);
     if (seg == 0) {
         if (valid) {
             a.count[s] = total < cap ? total : cap;
@@ -768,6 +798,24 @@ build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucke
             a.gmax_in[group] = ci;
             atomicMax(&a.status->max_count, (unsigned)tm);
         }
+    }
+}
+
+template <bool PERIODIC, int YS>
+__global__ void __launch_bounds__(GM_NSEG * YS * 32, YS == 1 ? 5 : 1)
+build_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucket_r2) {
+    build_group<PERIODIC, YS, false>(a, blockIdx.x, rl2_lo, rl2_hi, rl2_64, bucket_r2);
+}
+
+// The groups the build marked (usually none: one read of the status word).
+constexpr int kAgainBlocks = 304;
+template <bool PERIODIC>
+__global__ void __launch_bounds__(GM_NSEG * 32)
+build_again_kernel(ListArgs a, float rl2_lo, float rl2_hi, double rl2_64, float3 bucket_r2) {
+    if (a.status->stage_over == 0) return;
+    for (int group = blockIdx.x; group * 32 < a.n_slots; group += gridDim.x) {
+        build_group<PERIODIC, 1, true>(a, group, rl2_lo, rl2_hi, rl2_64, bucket_r2);
+        __syncthreads();
     }
 }
 
@@ -825,4 +873,7 @@ void gm_launch_build(const ListArgs &a, cudaStream_t s) {
     if (a.periodic) { if (ysplit) GM_BUILD(true, 5); else GM_BUILD(true, 1); }
     else { if (ysplit) GM_BUILD(false, 5); else GM_BUILD(false, 1); }
 #undef GM_BUILD
+    const int again = groups < kAgainBlocks ? groups : kAgainBlocks;
+    if (a.periodic) build_again_kernel<true><<<again, GM_NSEG * 32, 0, s>>>(a, lo, hi, rl2, bk);
+    else build_again_kernel<false><<<again, GM_NSEG * 32, 0, s>>>(a, lo, hi, rl2, bk);
 }

@@ -60,3 +60,28 @@ def test_pairs_equal_the_oracles(n, box, shape, r_list):
     (gi, gj), (ri, rj) = be.pairs(), ob.pairs()
     assert len(gi) == len(ri) and np.array_equal(gi, ri) and np.array_equal(gj, rj)
     be.close()
+
+
+@pytest.mark.parametrize("n,box,skin,steps", [(700, 45.0, 10.3, 190), (3200, 75.0, 10.5, 130)])
+def test_rebuilds_of_a_run_that_outgrow_the_staging_area(n, box, skin, steps):
+    """A droplet that condenses in a large periodic box: the staging area is
+    sized by the mean density and the first lists, and a resident run cannot
+    grow it.  The run ends, and the forces at its end are a fresh context's:
+    |dF| <= 1e-5 max(|F|, 1) per component."""
+    atoms, topo, state, _ = synth.generate(n, seed=11 + n, relax_iters=60)
+    pos = np.ascontiguousarray(state.pos - state.pos.mean(axis=1, keepdims=True))
+    vel = np.ascontiguousarray(state.vel).copy()
+    p = backend.SimParams(box_size=(box,) * 3, periodic=True, r_cutoff=10.0, r_skin=skin, r_switch=8.0, coulomb=True,
+                          bonded_min_image=True)
+    be = backend.CudaBackend(atoms, topo, p)
+    first = 0
+    for k in (3, 10, steps // 2, steps // 2):
+        _, _, f = be.steps(pos, vel, 0.002, k, first_step=first, want_forces=True)
+        first += k
+        other = backend.CudaBackend(atoms, topo, p)
+        q = pos.copy()
+        other.build_neighbor_list(q)
+        fr = other.compute_forces(q)
+        other.close()
+        assert np.max(np.abs(f - fr) / np.maximum(np.abs(fr), 1.0)) <= 1e-5, first
+    be.close()
