@@ -29,7 +29,9 @@ namespace {
 
 
 __device__ __forceinline__ double exact_wrap(double x, double L) {
-    // neighbor.rs:86-88: x - L * floor(x / L)
+    // neighbor.rs:86-88: x - L * floor(x / L); x itself inside the box (0 <= x <
+    // L by its bits, so the quotient rounds below 1; -0.0 goes the long way)
+    if ((unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(L)) return x;
     return __dsub_rn(x, __dmul_rn(L, floor(__ddiv_rn(x, L))));
 }
 
@@ -72,6 +74,22 @@ __device__ __forceinline__ int bbox_blocks_of(int n_atoms, int cap) {
     return b < 1 ? 1 : (b > cap ? cap : b);
 }
 
+// sm[0..8][t], t < width (a power of two): minima, maxima and sums over t, three
+// rows each, into column 0.  A level's 9 * k combinations are spread over the
+// block: an FP64 instruction holds its scheduler for 64 cycles whatever the
+// number of lanes, and with nine of them one after the other in every thread
+// the tree of 256 was 72 in a row (15 now).
+__device__ __forceinline__ void bbox_tree(double (*sm)[256], int width) {
+    for (int k = width / 2; k > 0; k >>= 1) {
+        for (int e = threadIdx.x; e < 9 * k; e += blockDim.x) {
+            const int v = e / k, t = e - v * k;
+            const double x = sm[v][t], y = sm[v][t + k];
+            sm[v][t] = v < 3 ? fmin(x, y) : (v < 6 ? fmax(x, y) : x + y);
+        }
+        __syncthreads();
+    }
+}
+
 // Per block and system: min x,y,z, max x,y,z and the sum x,y,z.
 __global__ void bbox_kernel(ListArgs a) {
     __shared__ double sm[9][256];
@@ -95,108 +113,97 @@ __global__ void bbox_kernel(ListArgs a) {
         sm[6 + d][threadIdx.x] = sum[d];
     }
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int d = 0; d < 3; d++) {
-                sm[d][threadIdx.x] = fmin(sm[d][threadIdx.x], sm[d][threadIdx.x + s]);
-                sm[3 + d][threadIdx.x] = fmax(sm[3 + d][threadIdx.x], sm[3 + d][threadIdx.x + s]);
-                sm[6 + d][threadIdx.x] += sm[6 + d][threadIdx.x + s];
-            }
-        __syncthreads();
-    }
+    bbox_tree(sm, 256);
     if (threadIdx.x < 9)
         a.bbox_scratch[((size_t)blockIdx.y * a.bbox_blocks + blockIdx.x) * 9 + threadIdx.x] = sm[threadIdx.x][0];
 }
 
-// One block per system: reduce its bbox partials, then lay out its grid.
-__global__ void grid_kernel(ListArgs a, int blocks) {
+// One block per system: reduce its bbox partials, then lay out its grid, a
+// dimension per lane (the FP64 divisions are most of the kernel: 1,536 atoms
+// 11.9 us with one thread for the three, 4.9 now).
+__global__ void __launch_bounds__(256) grid_kernel(ListArgs a, int blocks) {
     const int sys = blockIdx.x;
     if (!a.sys_flag[sys]) return;
     __shared__ double red[9][256];
-    const double *partial = a.bbox_scratch + (size_t)sys * blocks * 9;
-    const int nb = a.periodic ? 0 : bbox_blocks_of(a.sys_atom_off[sys + 1] - a.sys_atom_off[sys], 256);
-    for (int v = 0; v < 9; v++) {
-        double acc = v < 3 ? DBL_MAX : (v < 6 ? -DBL_MAX : 0.0);
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-            const double x = partial[b * 9 + v];
-            acc = v < 3 ? fmin(acc, x) : (v < 6 ? fmax(acc, x) : acc + x);
-        }
-        red[v][threadIdx.x] = acc;
-    }
-    __syncthreads();
     __shared__ int s_ncell;
-    for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-        if (threadIdx.x < k)
-            for (int v = 0; v < 9; v++) {
-                const double x = red[v][threadIdx.x + k];
-                red[v][threadIdx.x] = v < 3 ? fmin(red[v][threadIdx.x], x)
-                                            : (v < 6 ? fmax(red[v][threadIdx.x], x) : red[v][threadIdx.x] + x);
-            }
+    if (!a.periodic) {
+        const double *partial = a.bbox_scratch + (size_t)sys * blocks * 9;
+        const int nb = bbox_blocks_of(a.sys_atom_off[sys + 1] - a.sys_atom_off[sys], 256);
+        int width = 1;
+        while (width < nb) width *= 2;
+        if (threadIdx.x < width)
+            for (int v = 0; v < 9; v++)
+                red[v][threadIdx.x] = threadIdx.x < nb ? partial[threadIdx.x * 9 + v]
+                                                       : (v < 3 ? DBL_MAX : (v < 6 ? -DBL_MAX : 0.0));
         __syncthreads();
+        bbox_tree(red, width);
     }
-    if (threadIdx.x == 0) {
-    GridInfo *g = a.grid + sys;
-    const int n_atoms = a.sys_atom_off[sys + 1] - a.sys_atom_off[sys];
-    const int max_cells = a.sys_cell_off[sys + 1] - a.sys_cell_off[sys] - 1;
-    const double box[3] = {a.box[0], a.box[1], a.box[2]};
-    const double wmin = a.r_list * 0.5 * (1.0 + 1e-5) + 1e-6;
-    int nc[3];
-    double w[3], lo[3];
-    g->periodic = a.periodic;
-    for (int d = 0; d < 3; d++) {
-        g->box[d] = (float)box[d];
-        g->inv_box[d] = (float)(1.0 / box[d]);
-    }
-    if (a.periodic) {
-        for (int d = 0; d < 3; d++) {
-            nc[d] = (int)floor(box[d] / wmin);
-            if (nc[d] < 1) nc[d] = 1;
-            g->origin[d] = 0.5 * box[d];
-            lo[d] = -0.5 * box[d];
-        }
-    } else {
-        double mn[3], mx[3], sum[3];
-        for (int d = 0; d < 3; d++) { mn[d] = red[d][0]; mx[d] = red[3 + d][0]; sum[d] = red[6 + d][0]; }
-        // The grid covers a core cube around the mean position, at the finest
-        // cell width the allocation allows; atoms outside it (evaporated atoms
-        // of a droplet in vacuum) are clamped into the edge cells.  Clamping is
-        // 1-Lipschitz on cell indices, so the 5x5x5 stencil still finds every
-        // pair, and a few outliers no longer coarsen the whole grid.
-        const int per_dim = (int)floor(cbrt((double)max_cells));
-        for (int d = 0; d < 3; d++) {
-            double ext = mx[d] - mn[d];
-            if (!(ext == ext) || mx[d] < mn[d]) { ext = 0.0; mn[d] = mx[d] = 0.0; sum[d] = 0.0; }
+    if (threadIdx.x < 32) {
+        const unsigned full = 0xffffffffu;
+        const int d = min((int)threadIdx.x, 2);
+        const bool mine = threadIdx.x < 3;
+        GridInfo *g = a.grid + sys;
+        const int n_atoms = a.sys_atom_off[sys + 1] - a.sys_atom_off[sys];
+        const int max_cells = a.sys_cell_off[sys + 1] - a.sys_cell_off[sys] - 1;
+        const double box = a.box[d];
+        const double wmin = a.r_list * 0.5 * (1.0 + 1e-5) + 1e-6;
+        int nc;
+        double lo, origin;
+        if (a.periodic) {
+            nc = (int)floor(box / wmin);
+            if (nc < 1) nc = 1;
+            origin = 0.5 * box;
+            lo = -0.5 * box;
+        } else {
+            double mn = red[d][0], mx = red[3 + d][0], sum = red[6 + d][0];
+            // The grid covers a core cube around the mean position, at the finest
+            // cell width the allocation allows; atoms outside it (evaporated atoms
+            // of a droplet in vacuum) are clamped into the edge cells.  Clamping is
+            // 1-Lipschitz on cell indices, so the 5x5x5 stencil still finds every
+            // pair, and a few outliers no longer coarsen the whole grid.
+            const int per_dim = (int)floor(cbrt((double)max_cells));
+            double ext = mx - mn;
+            if (!(ext == ext) || mx < mn) { ext = 0.0; mn = mx = 0.0; sum = 0.0; }
             // min-image of the reference folds pairs farther apart than box/2;
             // the cell search assumes it never does
-            if (ext + a.r_list >= 0.5 * box[d]) atomicOr(&a.status->error, (unsigned)GM_DEV_EXTENT);
-            const double mean = n_atoms > 0 ? sum[d] / n_atoms : 0.0;
+            if (mine && ext + a.r_list >= 0.5 * box) atomicOr(&a.status->error, (unsigned)GM_DEV_EXTENT);
+            const double mean = n_atoms > 0 ? sum / n_atoms : 0.0;
             const double half = 0.5 * per_dim * wmin;
-            double lo_c = fmax(mn[d], mean - half), hi_c = fmin(mx[d], mean + half);
-            if (!(hi_c >= lo_c)) { lo_c = mn[d]; hi_c = mx[d]; }
+            double lo_c = fmax(mn, mean - half), hi_c = fmin(mx, mean + half);
+            if (!(hi_c >= lo_c)) { lo_c = mn; hi_c = mx; }
             const double pad = 1e-3 * (1.0 + (hi_c - lo_c));
-            g->origin[d] = 0.5 * (lo_c + hi_c);
-            lo[d] = (lo_c - g->origin[d]) - pad;
-            nc[d] = (int)floor((hi_c - lo_c + 2.0 * pad) / wmin);
-            if (nc[d] < 1) nc[d] = 1;
+            origin = 0.5 * (lo_c + hi_c);
+            lo = (lo_c - origin) - pad;
+            nc = (int)floor((hi_c - lo_c + 2.0 * pad) / wmin);
+            if (nc < 1) nc = 1;
         }
-    }
-    // keep the cell count within the allocation by coarsening the grid
-    // (coarser cells only widen the 5x5x5 search, never miss a pair)
-    while ((long long)nc[0] * nc[1] * nc[2] > max_cells) {
-        for (int d = 0; d < 3; d++) nc[d] = nc[d] > 1 ? (nc[d] * 3) / 4 : 1;
-    }
-    for (int d = 0; d < 3; d++) {
-        double span = a.periodic ? box[d] : -2.0 * lo[d];
-        w[d] = span / nc[d];
-        g->nc[d] = nc[d];
-        g->lo[d] = (float)lo[d];
-        g->inv_w[d] = (float)(1.0 / w[d]);
-        g->full[d] = a.periodic && nc[d] < 5;
-    }
-    g->ncell = nc[0] * nc[1] * nc[2];  // <= max_cells by construction
-    if (a.sys_far) a.sys_far[sys] = 0u;  // (the static build keeps no list)
-    atomicAdd(&a.status->n_rebuilds, 1ull);
-    s_ncell = min(g->ncell, max_cells);
+        // keep the cell count within the allocation by coarsening the grid
+        // (coarser cells only widen the 5x5x5 search, never miss a pair)
+        int n0, n1, n2;
+        for (;;) {
+            n0 = __shfl_sync(full, nc, 0), n1 = __shfl_sync(full, nc, 1), n2 = __shfl_sync(full, nc, 2);
+            const long long cells = (long long)n0 * n1 * n2;
+            if (cells <= max_cells || cells == 1) break;
+            nc = nc > 1 ? (nc * 3) / 4 : 1;
+        }
+        if (mine) {
+            const double span = a.periodic ? box : -2.0 * lo;
+            const double w = span / nc;
+            g->box[d] = (float)box;
+            g->inv_box[d] = (float)(1.0 / box);
+            g->origin[d] = origin;
+            g->nc[d] = nc;
+            g->lo[d] = (float)lo;
+            g->inv_w[d] = (float)(1.0 / w);
+            g->full[d] = a.periodic && nc < 5;
+        }
+        if (threadIdx.x == 0) {
+            g->periodic = a.periodic;
+            g->ncell = n0 * n1 * n2;  // <= max_cells by construction
+            if (a.sys_far) a.sys_far[sys] = 0u;  // (the static build keeps no list)
+            atomicAdd(&a.status->n_rebuilds, 1ull);
+            s_ncell = min(n0 * n1 * n2, max_cells);
+        }
     }
     // the cells the new grid uses (the only ones assign and the scan touch)
     __syncthreads();
