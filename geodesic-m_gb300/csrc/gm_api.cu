@@ -111,6 +111,7 @@ struct gm_ctx {
     int n_free = 0;                // atoms of no constraint
     int *d_free = nullptr;
     SolveSync *d_solve = nullptr;  // SHAKE's and RATTLE's words of the fused constrained step
+    bool solve_quads = false;  // four lanes a constraint
     int solve_threads = 0, solve_blocks = -1;  // its grid (-1: not looked up; 0: the clusters do not fit it)
     std::vector<int> h_ci, h_cj;
     // constraint warm start (gm_mlp.cu)
@@ -465,7 +466,8 @@ bool force_phase(const gm_ctx *c) { return c->step_form == GM_STEP_PERSISTENT &&
 // and no warm start needs the solve's own launches.
 bool fused_solve(gm_ctx *c) {
     if (!c->n_clusters || c->n_star_end != c->n_clusters || c->ws_on || c->ws_rec_stride > 0) return false;
-    if (c->solve_blocks < 0) gm_solve_step_grid(cluster_args(c), c->n_free, &c->solve_threads, &c->solve_blocks);
+    if (c->solve_blocks < 0) gm_solve_step_grid(cluster_args(c), c->n_free, &c->solve_threads, &c->solve_blocks,
+                                               &c->solve_quads);
     return c->solve_blocks > 0;
 }
 
@@ -881,7 +883,7 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
     }
     if (fused_solve(c)) {
         gm_launch_shake_step(cluster_args(c), solve_args(c, dt, cond, 0), pack_args(c), c->solve_threads,
-                             c->solve_blocks, s);
+                             c->solve_blocks, c->solve_quads, s);
         *count += 1;
         return GM_OK;
     }
@@ -901,7 +903,8 @@ int issue_step_tail(gm_ctx *c, cudaStream_t s, double dt, long long *count) {
     const bool fused = fused_solve(c);
     long long k = seq_forces(c, s, false, c->side, c->n_clusters == 0 || fused);
     if (fused) {
-        gm_launch_rattle_step(cluster_args(c), solve_args(c, dt, 0ull, 1), c->solve_threads, c->solve_blocks, s);
+        gm_launch_rattle_step(cluster_args(c), solve_args(c, dt, 0ull, 1), c->solve_threads, c->solve_blocks, c->solve_quads,
+                              s);
         k++;
     } else if (c->n_clusters) {
         gm_launch_half_kick(c->n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, s); k++;

@@ -833,6 +833,91 @@ __device__ __forceinline__ void lane_report_step(const ClusterArgs &c, const Sta
     if ((threadIdx.x & 31) == 0 && it) atomicMax(&sy->T, it);
 }
 
+// The first of a thread's atoms of no constraint: the threads past the `lanes`
+// solver lanes take them first.
+__device__ __forceinline__ int first_free(int tid, int threads, int lanes) {
+    return tid >= lanes ? tid - lanes : tid + threads - lanes;
+}
+
+// Kick, drift and what follows it for the atoms of no constraint; the kicked
+// velocity goes to dref for the case of a failed projection, which skips the
+// resync.
+__device__ __forceinline__ void free_drift(const ClusterArgs &c, const SolveStepArgs &sa, const PackArgs &pk, bool err0,
+                                           int free0, int threads, int &need, int &bad) {
+    const int n = sa.n;
+    for (int q = free0; q < sa.n_free; q += threads) {
+        const int i = sa.free_atoms[q];
+        double np[3];
+        const double inv_m = c.inv_mass[i];
+        for (int d = 0; d < 3; d++) {
+            const double p = sa.pos[d * n + i];
+            np[d] = p;
+            if (!err0) {
+                const double v = kicked(sa.vel[d * n + i], sa.force[d * n + i], inv_m, sa.dt_half);
+                np[d] = p + sa.dt * v;
+                sa.pos[d * n + i] = np[d];
+                sa.dref[d * n + i] = v;
+                sa.vel[d * n + i] = gm_div_by_dt(np[d] - p, sa.dt, sa.inv_dt);
+            }
+        }
+        finish_atom(sa, pk, i, np[0], np[1], np[2], need, bad);
+    }
+}
+__device__ __forceinline__ void free_kicked(const SolveStepArgs &sa, int free0, int threads) {
+    const int n = sa.n;
+    for (int q = free0; q < sa.n_free; q += threads) {
+        const int i = sa.free_atoms[q];
+        for (int d = 0; d < 3; d++) sa.vel[d * n + i] = sa.dref[d * n + i];
+    }
+}
+__device__ __forceinline__ void free_kick(const ClusterArgs &c, const SolveStepArgs &sa, int free0, int threads) {
+    const int n = sa.n;
+    for (int q = free0; q < sa.n_free; q += threads) {
+        const int i = sa.free_atoms[q];
+        const double inv_m = c.inv_mass[i];
+        for (int d = 0; d < 3; d++) sa.vel[d * n + i] = kicked(sa.vel[d * n + i], sa.force[d * n + i], inv_m, sa.dt_half);
+    }
+}
+
+// The ends of the two kernels: the last block's bookkeeping.
+__device__ __forceinline__ void shake_tail(const SolveStepArgs &sa, DevStatus *st, unsigned T, bool fail, int need,
+                                           int bad) {
+    SolveSync *sy = sa.sync;
+    need = __syncthreads_or(need);
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) {
+        if (need) atomicOr(&st->rebuild, 1u);
+        if (bad) atomicOr(&st->error, (unsigned)GM_DEV_NONFINITE_POS);
+        if (last_block(st)) {
+            st->shake_T = T;
+            if (fail) atomicOr(&st->error, (unsigned)GM_DEV_SHAKE_FAIL);
+            sy->T = 0;
+            sy->fail = 0;
+            const unsigned r = atomicOr(&st->rebuild, 0u), e = atomicOr(&st->error, 0u);
+            if (sa.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)sa.cond, (r && !e) ? 1u : 0u);
+        }
+    }
+}
+
+__device__ __forceinline__ void rattle_tail(const SolveStepArgs &sa, DevStatus *st, unsigned T, bool fail) {
+    SolveSync *sy = sa.sync;
+    __syncthreads();
+    if (threadIdx.x == 0 && last_block(st)) {
+        st->rattle_T = T;
+        if (fail) atomicOr(&st->error, (unsigned)GM_DEV_RATTLE_FAIL);
+        sy->T = 0;
+        sy->fail = 0;
+        if (atomicOr(&st->error, 0u) == 0) {  // step_kernel's count
+            st->step += 1;
+            if (st->shake_T || T) {
+                st->c_steps += 1;
+                st->shake_sum += st->shake_T;
+                st->rattle_sum += T;
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(128) shake_step_kernel(ClusterArgs c, SolveStepArgs sa, PackArgs pk) {
     DevStatus *st = c.status;
     SolveSync *sy = sa.sync;
@@ -873,28 +958,8 @@ __global__ void __launch_bounds__(128) shake_step_kernel(ClusterArgs c, SolveSte
             lane_report_step<false>(c, s, g, sy);
         }
     }
-    // atoms of no constraint, by the threads past the lanes first; the kicked
-    // velocity goes to dref for the case of a failed projection, which skips
-    // the resync
-    const int threads = gridDim.x * blockDim.x;
-    const int free0 = tid >= c.n_lane_warps * 32 ? tid - c.n_lane_warps * 32 : tid + threads - c.n_lane_warps * 32;
-    for (int q = free0; q < sa.n_free; q += threads) {
-        const int i = sa.free_atoms[q];
-        double np[3];
-        const double inv_m = c.inv_mass[i];
-        for (int d = 0; d < 3; d++) {
-            const double p = sa.pos[d * n + i];
-            np[d] = p;
-            if (!err0) {
-                const double v = kicked(sa.vel[d * n + i], sa.force[d * n + i], inv_m, sa.dt_half);
-                np[d] = p + sa.dt * v;
-                sa.pos[d * n + i] = np[d];
-                sa.dref[d * n + i] = v;
-                sa.vel[d * n + i] = gm_div_by_dt(np[d] - p, sa.dt, sa.inv_dt);
-            }
-        }
-        finish_atom(sa, pk, i, np[0], np[1], np[2], need, bad);
-    }
+    const int threads = gridDim.x * blockDim.x, free0 = first_free(tid, threads, c.n_lane_warps * 32);
+    free_drift(c, sa, pk, err0, free0, threads, need, bad);
     if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
     const unsigned T = gm_ld_acquire(&sy->T);
     const bool fail = gm_ld_acquire(&sy->fail) != 0;
@@ -929,25 +994,8 @@ __global__ void __launch_bounds__(128) shake_step_kernel(ClusterArgs c, SolveSte
             finish_atom(sa, pk, s.h, s.hx, s.hy, s.hz, need, bad);
         }
     }
-    if (!err0 && fail)
-        for (int q = free0; q < sa.n_free; q += threads) {
-            const int i = sa.free_atoms[q];
-            for (int d = 0; d < 3; d++) sa.vel[d * n + i] = sa.dref[d * n + i];
-        }
-    need = __syncthreads_or(need);
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) {
-        if (need) atomicOr(&st->rebuild, 1u);
-        if (bad) atomicOr(&st->error, (unsigned)GM_DEV_NONFINITE_POS);
-        if (last_block(st)) {
-            st->shake_T = T;
-            if (fail) atomicOr(&st->error, (unsigned)GM_DEV_SHAKE_FAIL);
-            sy->T = 0;
-            sy->fail = 0;
-            const unsigned r = atomicOr(&st->rebuild, 0u), e = atomicOr(&st->error, 0u);
-            if (sa.cond) cudaGraphSetConditional((cudaGraphConditionalHandle)sa.cond, (r && !e) ? 1u : 0u);
-        }
-    }
+    if (!err0 && fail) free_kicked(sa, free0, threads);
+    shake_tail(sa, st, T, fail, need, bad);
 }
 
 __global__ void __launch_bounds__(128) rattle_step_kernel(ClusterArgs c, SolveStepArgs sa) {
@@ -976,12 +1024,7 @@ __global__ void __launch_bounds__(128) rattle_step_kernel(ClusterArgs c, SolveSt
         lane_report_step<true>(c, s, g, sy);
     }
     const int threads = gridDim.x * blockDim.x;
-    const int free0 = tid >= c.n_lane_warps * 32 ? tid - c.n_lane_warps * 32 : tid + threads - c.n_lane_warps * 32;
-    for (int q = free0; q < sa.n_free && !err0; q += threads) {
-        const int i = sa.free_atoms[q];
-        const double inv_m = c.inv_mass[i];
-        for (int d = 0; d < 3; d++) sa.vel[d * n + i] = kicked(sa.vel[d * n + i], sa.force[d * n + i], inv_m, sa.dt_half);
-    }
+    if (!err0) free_kick(c, sa, first_free(tid, threads, c.n_lane_warps * 32), threads);
     if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
     const unsigned T = gm_ld_acquire(&sy->T);
     const bool fail = gm_ld_acquire(&sy->fail) != 0;
@@ -994,21 +1037,292 @@ __global__ void __launch_bounds__(128) rattle_step_kernel(ClusterArgs c, SolveSt
         }
         if (s.k >= 0) { sa.vel[s.h] = s.hx; sa.vel[n + s.h] = s.hy; sa.vel[2 * n + s.h] = s.hz; }
     }
-    __syncthreads();
-    if (threadIdx.x == 0 && last_block(st)) {
-        st->rattle_T = T;
-        if (fail) atomicOr(&st->error, (unsigned)GM_DEV_RATTLE_FAIL);
-        sy->T = 0;
-        sy->fail = 0;
-        if (atomicOr(&st->error, 0u) == 0) {  // step_kernel's count
-            st->step += 1;
-            if (st->shake_T || T) {
-                st->c_steps += 1;
-                st->shake_sum += st->shake_T;
-                st->rattle_sum += T;
-            }
+    rattle_tail(sa, st, T, fail);
+}
+
+// ---- the same step with four lanes a constraint ---------------------------
+//
+// For systems whose lanes leave schedulers without a warp: lane d of a quad
+// holds component d of the centre, the H atom and the vector (the fourth lane
+// repeats z and stores nothing), so a difference, a product or an update of
+// three components is one FP64 instruction of the warp instead of three; the
+// sums over components take the three products by shuffles and add them in the
+// order of the lane per constraint.  An iteration of a two-H star is 28 FP64
+// instructions in a row against 43 (SHAKE) and 14 against 28 (RATTLE).
+struct CompLane {
+    int cen, h, k, cl, d;    // atoms, constraint, cluster (as in StarLane); component
+    double x, y, r;          // centre, H atom (SHAKE: positions, RATTLE: velocities); the vector
+    double inv_c, inv_h, wq, dsq, rcp, lam, box;
+    unsigned it;
+    bool ok;
+};
+
+__device__ __forceinline__ double comp_dot(double p) {  // over the quad, every lane of the warp calls
+    const unsigned full = 0xffffffffu;
+    const double p0 = __shfl_sync(full, p, 0, 4), p1 = __shfl_sync(full, p, 1, 4), p2 = __shfl_sync(full, p, 2, 4);
+    return p0 + p1 + p2;
+}
+__device__ __forceinline__ double comp_diff(const ClusterArgs &c, const CompLane &s, double a, double b) {
+    const double v = a - b;
+    return c.mi ? gm_min_image(v, s.box) : v;
+}
+
+// The quad's constraint and constants; the group in lanes of the warp.
+template <bool RATTLE>
+__device__ __forceinline__ LaneGroup comp_init(const ClusterArgs &c, int warp, CompLane &s) {
+    const int lane = threadIdx.x & 31, q = warp * 8 + (lane >> 2);
+    LaneGroup g;
+    g.width = 4 * c.lane_width[q >> 5];
+    g.base = lane & ~(g.width - 1);
+    g.mask = g.width == 32 ? 0xffffffffu : ((1u << g.width) - 1u) << g.base;
+    const int4 t = c.lanes[q];
+    s.cen = t.x; s.h = t.y; s.k = t.z; s.cl = t.w;
+    s.d = min(lane & 3, 2);
+    s.box = s.d == 0 ? c.box64[0] : s.d == 1 ? c.box64[1] : c.box64[2];
+    s.x = s.y = s.r = s.inv_c = s.inv_h = s.wq = s.dsq = s.rcp = s.lam = 0.0;
+    s.it = 0;
+    s.ok = false;
+    if (s.cl >= 0) s.inv_c = c.inv_mass[s.cen];
+    if (s.k >= 0) {
+        s.inv_h = c.inv_mass[s.h];
+        if (!RATTLE) {
+            s.dsq = c.constr_dsq[s.k];
+            s.wq = 2.0 * (s.inv_c + s.inv_h);
         }
     }
+    return g;
+}
+
+// lane_iterate and lane_apply, a component per lane
+template <bool RATTLE>
+__device__ __forceinline__ void comp_iterate(const ClusterArgs &c, CompLane &s, const LaneGroup &g, unsigned stop,
+                                             bool phase1) {
+    const unsigned full = 0xffffffffu;
+    const int sub = threadIdx.x & 3;
+    for (;;) {
+        const bool run = s.cl >= 0 && s.it < stop && !(phase1 && s.ok);
+        if (!__any_sync(full, run)) break;
+        double l = 0.0;
+        const double dx = RATTLE ? s.x - s.y : comp_diff(c, s, s.x, s.y);
+        const double dot = comp_dot(dx * s.r);
+        if (RATTLE) {
+            if (s.k >= 0) {
+                if (s.rcp != 0.0) l = gm_div_rcp(dot, s.wq, s.rcp);
+                else l = s.wq == 0.0 ? 0.0 : dot / s.wq;
+            }
+        } else {
+            const double diff = comp_dot(dx * dx) - s.dsq;
+            if (s.k >= 0) {
+                const double denom = s.wq * dot;
+                l = (__double_as_longlong(denom) << 1) == 0 ? 0.0 : diff / denom;
+            }
+        }
+        if (run) s.lam = l;
+        const double w = s.lam * s.inv_c;
+        const double t = w * s.r;
+        double dd = -__shfl_sync(full, t, g.base + sub);
+        for (int q = 4; q < g.width; q += 4) dd -= __shfl_sync(full, t, g.base + q + sub);
+        const double wh = s.lam * s.inv_h;
+        const double u = wh * s.r;
+        if (run) {
+            s.x += dd;
+            s.y += u;
+        }
+        const unsigned small = __ballot_sync(full, !gm_abs_ge(l, c.tol));
+        if (run) {
+            s.it++;
+            if (phase1) s.ok = (small & g.mask) == g.mask;
+        }
+    }
+}
+
+// lane_worst, lane_report_step and lane_report2 over quads
+__device__ __forceinline__ void comp_worst(const CompLane &s, const LaneGroup &g, double &mx, int &worst) {
+    const unsigned full = 0xffffffffu;
+    const double la = fabs(s.lam) > 0.0 ? fabs(s.lam) : 0.0;
+    mx = la;
+    for (int o = 4; o < 32; o <<= 1) {
+        const double m = __shfl_xor_sync(full, mx, o);
+        if (o < g.width) mx = fmax(mx, m);
+    }
+    const unsigned hit = __ballot_sync(full, s.k >= 0 && la == mx && mx > 0.0) & g.mask;
+    worst = __shfl_sync(full, s.k, hit ? __ffs(hit) - 1 : g.base);
+}
+__device__ __forceinline__ void comp_report_step(const ClusterArgs &c, const CompLane &s, const LaneGroup &g,
+                                                 SolveSync *sy) {
+    double mx;
+    int worst;
+    comp_worst(s, g, mx, worst);
+    const bool leader = s.cl >= 0 && (int)(threadIdx.x & 31) == g.base;
+    if (leader) {
+        c.cl_iters[s.cl] = (int)s.it;
+        c.cl_worst[s.cl] = mx;
+        c.cl_worst_idx[s.cl] = worst;
+        if (!s.ok) {
+            atomicOr(&sy->fail, 1u);
+            atomicMin(&c.status->fail_step, c.status->step);
+        }
+    }
+    const unsigned it = __reduce_max_sync(0xffffffffu, leader ? s.it : 0u);
+    if ((threadIdx.x & 31) == 0 && it) atomicMax(&sy->T, it);
+}
+__device__ __forceinline__ void comp_report2(const ClusterArgs &c, const CompLane &s, const LaneGroup &g, unsigned T,
+                                             bool ran) {
+    double mx;
+    int worst;
+    comp_worst(s, g, mx, worst);
+    if (ran && s.cl >= 0 && (int)(threadIdx.x & 31) == g.base) {
+        c.cl_iters[s.cl] = (int)s.it;
+        c.cl_worst[s.cl] = mx;
+        c.cl_worst_idx[s.cl] = worst;
+        if (!(mx < c.tol) && T < c.max_iter) atomicOr(&c.status->error, (unsigned)GM_DEV_ITER_MISMATCH);
+    }
+}
+
+// finish_atom by a quad (with `on`): a component a lane, the fourth the charge;
+// every lane of the warp calls.
+__device__ __forceinline__ void comp_finish(const SolveStepArgs &sa, const PackArgs &pk, bool on, int i, int d, double x,
+                                            int &need, int &bad) {
+    const int n = sa.n, sub = threadIdx.x & 3;
+    int sy = 0;
+    double dx = 0.0;
+    if (on) {
+        const int sl = pk.slot_of[i];
+        sy = sa.atom_sys[i];
+        float *rec = reinterpret_cast<float *>(pk.coord + 2 * sl);
+        if (sub < 3) {
+            gm_pack_component(rec + sub, x - pk.grid[sy].origin[d]);
+            sa.force[d * n + i] = 0;
+            bad |= !isfinite(x);
+            dx = x - sa.ref[d * n + i];
+        } else {
+            const float2 qw = pk.qw[i];
+            rec[3] = qw.x;
+            rec[7] = qw.y;
+        }
+        if (pk.fp64) {
+            reinterpret_cast<double *>(pk.pos64s + sl)[sub] = sub < 3 ? x : pk.charge64[i];
+            if (sub == 3) pk.type_sorted[sl] = pk.type[i];
+        }
+    }
+    const double d2 = comp_dot(dx * dx);
+    if (on) {
+        if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sy] = 1u;
+        if (d2 > sa.thr_sq) {
+            sa.sys_flag[sy] = 1u;
+            need = 1;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(32) shake_comp_kernel(ClusterArgs c, SolveStepArgs sa, PackArgs pk) {
+    DevStatus *st = c.status;
+    SolveSync *sy = sa.sync;
+    const int n = sa.n, tid = blockIdx.x * blockDim.x + threadIdx.x, warp = tid >> 5, sub = tid & 3;
+    const bool err0 = gm_ld_acquire(&st->error) != 0;
+    const bool lanes = warp < 4 * c.n_lane_warps;
+    int need = 0, bad = 0;
+    CompLane s;
+    LaneGroup g;
+    double pc = 0.0, vc = 0.0, ph = 0.0, vh = 0.0;  // before the drift; after the kick
+    if (lanes) {
+        g = comp_init<false>(c, warp, s);
+        if (s.cl >= 0) {
+            const int q = s.d * n + s.cen;
+            pc = sa.pos[q];
+            vc = sa.vel[q];
+            if (!err0) vc = kicked(vc, sa.force[q], s.inv_c, sa.dt_half);
+        }
+        if (s.k >= 0) {
+            const int q = s.d * n + s.h;
+            ph = sa.pos[q];
+            vh = sa.vel[q];
+            if (!err0) vh = kicked(vh, sa.force[q], s.inv_h, sa.dt_half);
+        }
+        if (!err0) {
+            if (s.cl >= 0) s.x = pc + sa.dt * vc;
+            if (s.k >= 0) {
+                s.y = ph + sa.dt * vh;
+                s.r = comp_diff(c, s, pc, ph);
+            }
+            comp_iterate<false>(c, s, g, c.max_iter, true);
+            comp_report_step(c, s, g, sy);
+        }
+    }
+    const int threads = gridDim.x * blockDim.x, free0 = first_free(tid, threads, c.n_lane_warps * 128);
+    free_drift(c, sa, pk, err0, free0, threads, need, bad);
+    if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
+    const unsigned T = gm_ld_acquire(&sy->T);
+    const bool fail = gm_ld_acquire(&sy->fail) != 0;
+    if (lanes) {
+        if (!err0) {
+            const bool ran = s.cl >= 0 && s.it < T;
+            comp_iterate<false>(c, s, g, T, false);
+            comp_report2(c, s, g, T, ran);
+        } else {
+            s.x = pc;
+            s.y = ph;
+        }
+        const bool leader = s.cl >= 0 && (int)(threadIdx.x & 28) == g.base;
+        if (leader && !err0 && sub < 3) {
+            sa.pos[s.d * n + s.cen] = s.x;
+            sa.vel[s.d * n + s.cen] = fail ? vc : gm_div_by_dt(s.x - pc, sa.dt, sa.inv_dt);
+        }
+        comp_finish(sa, pk, leader, s.cen, s.d, s.x, need, bad);
+        if (s.k >= 0 && !err0 && sub < 3) {
+            sa.pos[s.d * n + s.h] = s.y;
+            sa.vel[s.d * n + s.h] = fail ? vh : gm_div_by_dt(s.y - ph, sa.dt, sa.inv_dt);
+        }
+        comp_finish(sa, pk, s.k >= 0, s.h, s.d, s.y, need, bad);
+    }
+    if (!err0 && fail) free_kicked(sa, free0, threads);
+    shake_tail(sa, st, T, fail, need, bad);
+}
+
+__global__ void __launch_bounds__(32) rattle_comp_kernel(ClusterArgs c, SolveStepArgs sa) {
+    DevStatus *st = c.status;
+    SolveSync *sy = sa.sync;
+    const int n = sa.n, tid = blockIdx.x * blockDim.x + threadIdx.x, warp = tid >> 5, sub = tid & 3;
+    const bool err0 = gm_ld_acquire(&st->error) != 0;
+    const bool lanes = warp < 4 * c.n_lane_warps;
+    CompLane s;
+    LaneGroup g;
+    if (lanes && !err0) {
+        g = comp_init<true>(c, warp, s);
+        double pc = 0.0, ph = 0.0;
+        if (s.cl >= 0) {
+            const int q = s.d * n + s.cen;
+            s.x = kicked(sa.vel[q], sa.force[q], s.inv_c, sa.dt_half);
+            pc = sa.pos[q];
+        }
+        if (s.k >= 0) {
+            const int q = s.d * n + s.h;
+            s.y = kicked(sa.vel[q], sa.force[q], s.inv_h, sa.dt_half);
+            ph = sa.pos[q];
+            s.r = comp_diff(c, s, pc, ph);
+        }
+        // lane_bond
+        const double rsq = comp_dot(s.r * s.r);
+        if (s.k >= 0) {
+            s.wq = (s.inv_c + s.inv_h) * rsq;
+            s.rcp = gm_ordinary(s.wq) ? 1.0 / s.wq : 0.0;
+        }
+        comp_iterate<true>(c, s, g, c.max_iter, true);
+        comp_report_step(c, s, g, sy);
+    }
+    const int threads = gridDim.x * blockDim.x;
+    if (!err0) free_kick(c, sa, first_free(tid, threads, c.n_lane_warps * 128), threads);
+    if (!gm_grid_barrier(&sy->arrive, &sy->gen, st)) return;
+    const unsigned T = gm_ld_acquire(&sy->T);
+    const bool fail = gm_ld_acquire(&sy->fail) != 0;
+    if (lanes && !err0) {
+        const bool ran = s.cl >= 0 && s.it < T;
+        comp_iterate<true>(c, s, g, T, false);
+        comp_report2(c, s, g, T, ran);
+        if (s.cl >= 0 && (int)(threadIdx.x & 28) == g.base && sub < 3) sa.vel[s.d * n + s.cen] = s.x;
+        if (s.k >= 0 && sub < 3) sa.vel[s.d * n + s.h] = s.y;
+    }
+    rattle_tail(sa, st, T, fail);
 }
 
 __global__ void reset_T(DevStatus *st, int rattle) {
@@ -1321,20 +1635,25 @@ void gm_launch_rattle(const ClusterArgs &c, int n_atoms, const double *pos, doub
     cluster_phase2<true><<<b, 32, 0, s>>>(c, const_cast<double *>(pos), vel, n_atoms);
 }
 
-void gm_solve_step_grid(const ClusterArgs &c, int n_free, int *threads, int *blocks) {
+void gm_solve_step_grid(const ClusterArgs &c, int n_free, int *threads, int *blocks, bool *quads) {
     *blocks = 0;
     int dev = 0, sms = 0, per1 = 0, per2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return;
+    // four lanes a constraint while every such warp has a scheduler of its own
+    const bool comp = c.n_lane_warps <= sms;
     // few constraints: a warp per block, so that every SM's FP64 pipe gets its share
     *threads = c.n_lane_warps <= 4 * sms ? 32 : 128;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, shake_step_kernel, *threads, 0) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, rattle_step_kernel, *threads, 0) != cudaSuccess)
-        return;
+    const cudaError_t e1 = comp ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, shake_comp_kernel, *threads, 0)
+                                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, shake_step_kernel, *threads, 0);
+    const cudaError_t e2 = comp ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, rattle_comp_kernel, *threads, 0)
+                                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, rattle_step_kernel, *threads, 0);
+    if (e1 != cudaSuccess || e2 != cudaSuccess) return;
     const int fit = (per1 < per2 ? per1 : per2) * sms, warps = *threads / 32;
-    const int need = (c.n_lane_warps + warps - 1) / warps;
+    const int need = comp ? 4 * c.n_lane_warps : (c.n_lane_warps + warps - 1) / warps;
     if (need > fit) return;
+    *quads = comp;
     // the free atoms take the rest of the SMs, one atom a thread while they last
     const int extra = (n_free + *threads - 1) / *threads;
     *blocks = need + extra < fit ? need + extra : fit;
@@ -1357,11 +1676,14 @@ void launch_cooperative(void (*kernel)(A...), int blocks, int threads, cudaStrea
 }  // namespace
 
 void gm_launch_shake_step(const ClusterArgs &c, const SolveStepArgs &sa, const PackArgs &pk, int threads, int blocks,
-                          cudaStream_t s) {
-    launch_cooperative<ClusterArgs, SolveStepArgs, PackArgs>(shake_step_kernel, blocks, threads, s, c, sa, pk);
+                          bool quads, cudaStream_t s) {
+    launch_cooperative<ClusterArgs, SolveStepArgs, PackArgs>(quads ? shake_comp_kernel : shake_step_kernel, blocks,
+                                                             threads, s, c, sa, pk);
 }
-void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int threads, int blocks, cudaStream_t s) {
-    launch_cooperative<ClusterArgs, SolveStepArgs>(rattle_step_kernel, blocks, threads, s, c, sa);
+void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int threads, int blocks, bool quads,
+                           cudaStream_t s) {
+    launch_cooperative<ClusterArgs, SolveStepArgs>(quads ? rattle_comp_kernel : rattle_step_kernel, blocks, threads, s,
+                                                   c, sa);
 }
 
 void gm_launch_kinetic(int n, const double *vel, const double *mass, double *partials, int blocks, double *out,

@@ -206,6 +206,12 @@ __device__ __forceinline__ void gm_pack_record(float4 *rec, double ox, double oy
     rec[0] = make_float4(hx, hy, hz, qw.x);
     rec[1] = make_float4((float)(ox - (double)hx), (float)(oy - (double)hy), (float)(oz - (double)hz), qw.y);
 }
+// One component of it: the grid value at rec[0], the remainder at rec[4].
+__device__ __forceinline__ void gm_pack_component(float *rec, double o) {
+    const float h = rintf((float)o * 256.f) * (1.f / 256.f);
+    rec[0] = h;
+    rec[4] = (float)(o - (double)h);
+}
 
 __device__ __forceinline__ unsigned gm_ld_acquire(const unsigned *p) {
     unsigned v;
@@ -501,10 +507,11 @@ struct SolveStepArgs {
 };
 // Threads per block and blocks (all co-resident) of both kernels; blocks 0
 // when the system's clusters do not fit.
-void gm_solve_step_grid(const ClusterArgs &c, int n_free, int *threads, int *blocks);
+void gm_solve_step_grid(const ClusterArgs &c, int n_free, int *threads, int *blocks, bool *quads);
 void gm_launch_shake_step(const ClusterArgs &c, const SolveStepArgs &sa, const PackArgs &pk, int threads, int blocks,
-                          cudaStream_t s);
-void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int threads, int blocks, cudaStream_t s);
+                          bool quads, cudaStream_t s);
+void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int threads, int blocks, bool quads,
+                           cudaStream_t s);
 // Blocks of the cooperative grid (all co-resident, no more than the work
 // items and atoms fill); 0 when the form does not apply.
 int gm_step_persistent_blocks(const ForceArgs &fa);

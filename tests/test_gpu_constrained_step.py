@@ -61,7 +61,9 @@ def system(sizes, n_free, seed):
 
 
 CASES = [([1], 0), ([2] * 5, 3), ([1] * 33, 100), ([3] * 9 + [4] * 8, 1), ([8] * 4 + [5, 6, 7], 40),
-         ([1] * 31 + [2] * 17 + [3] * 8 + [4] * 2 + [5] * 3 + [8], 700)]
+         ([1] * 31 + [2] * 17 + [3] * 8 + [4] * 2 + [5] * 3 + [8], 700),
+         # one star past a warp per scheduler with four lanes a constraint (152 SMs), and the last at it
+         ([2] * 2432, 5), ([2] * 2433, 5)]
 
 
 @pytest.mark.parametrize("precision", [backend.PRECISION_MIXED, backend.PRECISION_FP64])
