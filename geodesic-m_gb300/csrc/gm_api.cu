@@ -143,7 +143,7 @@ struct gm_ctx {
     // graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
-    // the persistent form's runs: launches of several steps inside a WHILE node
+    // the steps of a call inside a WHILE node
     cudaGraph_t loop_graph = nullptr;
     cudaGraphExec_t loop_exec = nullptr;
     double loop_dt = 0.0;
@@ -473,14 +473,15 @@ bool fused_solve(gm_ctx *c) {
 
 // Before the steps of a call: the barrier and queue words start cleared (a
 // launch that gave up at its barrier leaves them set).
-int begin_constrained(gm_ctx *c) {
+int begin_constrained(gm_ctx *c, int64_t todo = 1) {
     if (!c->n_clusters) return GM_OK;
-    GM_CUDA(c, cudaMemsetAsync(c->d_solve, 0, 2 * sizeof(SolveSync), c->stream));
+    gm_launch_solve_begin(c->d_solve, todo, c->stream);
+    c->launches++;
     GM_CUDA(c, cudaMemsetAsync(c->d_sync, 0, sizeof(StepSync), c->stream));
     return GM_OK;
 }
 
-SolveStepArgs solve_args(gm_ctx *c, double dt, unsigned long long cond, int which) {
+SolveStepArgs solve_args(gm_ctx *c, double dt, unsigned long long cond, int which, unsigned long long loop) {
     const double half_skin = (c->p.r_skin - c->p.r_cutoff) / 2.0;  // neighbor.rs:61-62
     SolveStepArgs a{};
     a.n = c->n;
@@ -497,6 +498,7 @@ SolveStepArgs solve_args(gm_ctx *c, double dt, unsigned long long cond, int whic
     a.thr_sq = half_skin * half_skin;
     a.far_sq = far_sq(c);
     a.cond = cond;
+    a.loop = loop;
     a.atom_sys = c->d_atom_sys;
     a.sys_flag = c->d_sys_flag;
     a.sys_far = c->d_sys_far;
@@ -842,7 +844,8 @@ int end_persistent(gm_ctx *c) {
 // One BAB + RATTLE step (lib.rs:292-323) issued on stream s.  With a graph
 // conditional handle the rebuild runs inside an IF node; otherwise the check
 // result is read back on the host.
-// `loop`: the handle of the WHILE node round the launch (persistent form).
+// `loop`: the handle of the WHILE node round the step (the forms that run in
+// one, see loops).
 int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, long long *count,
                unsigned long long loop = 0ull) {
     long long k = 0;
@@ -882,7 +885,7 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
         return GM_OK;
     }
     if (fused_solve(c)) {
-        gm_launch_shake_step(cluster_args(c), solve_args(c, dt, cond, 0), pack_args(c), c->solve_threads,
+        gm_launch_shake_step(cluster_args(c), solve_args(c, dt, cond, 0, loop), pack_args(c), c->solve_threads,
                              c->solve_blocks, c->solve_quads, s);
         *count += 1;
         return GM_OK;
@@ -898,13 +901,13 @@ int issue_step(gm_ctx *c, cudaStream_t s, double dt, unsigned long long cond, lo
     return GM_OK;
 }
 
-int issue_step_tail(gm_ctx *c, cudaStream_t s, double dt, long long *count) {
+int issue_step_tail(gm_ctx *c, cudaStream_t s, double dt, long long *count, unsigned long long loop = 0ull) {
     if (persistent_form(c)) return GM_OK;  // the next launch evaluates the forces
     const bool fused = fused_solve(c);
     long long k = seq_forces(c, s, false, c->side, c->n_clusters == 0 || fused);
     if (fused) {
-        gm_launch_rattle_step(cluster_args(c), solve_args(c, dt, 0ull, 1), c->solve_threads, c->solve_blocks, c->solve_quads,
-                              s);
+        gm_launch_rattle_step(cluster_args(c), solve_args(c, dt, 0ull, 1, loop), c->solve_threads, c->solve_blocks,
+                              c->solve_quads, s);
         k++;
     } else if (c->n_clusters) {
         gm_launch_half_kick(c->n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, s); k++;
@@ -983,12 +986,18 @@ int capture_graph(gm_ctx *c, double dt) {
     return GM_OK;
 }
 
-// The persistent form's run of a call as one graph: WHILE steps are left, a
-// launch of up to GM_LOOP_STEPS steps that ends early when the list has to be
-// rebuilt, and the IF node of the rebuild.
+// Whether a call's steps run as one graph (capture_loop): the forms whose last
+// kernel counts the steps and ends the WHILE node.
+bool loops(gm_ctx *c) {
+    return persistent_form(c) ? gm_step_loops(force_args(c)) : fused_solve(c);
+}
+
+// The steps of a call as one graph: WHILE steps are left, the step's launches
+// with the IF node of the rebuild.  In the persistent form a launch of up to
+// GM_LOOP_STEPS steps that ends early when the list has to be rebuilt.
 int capture_loop(gm_ctx *c, double dt) {
     if (c->loop_exec && c->loop_dt == dt && c->loop_cap == c->cap) return GM_OK;
-    int rc = persistent_grid(c);
+    int rc = force_phase(c) ? persistent_grid(c) : GM_OK;
     if (rc) return rc;
     if (c->loop_exec) { cudaGraphExecDestroy(c->loop_exec); c->loop_exec = nullptr; }
     if (c->loop_graph) { cudaGraphDestroy(c->loop_graph); c->loop_graph = nullptr; }
@@ -1011,6 +1020,7 @@ int capture_loop(gm_ctx *c, double dt) {
     issue_step(c, c->stream, dt, (unsigned long long)hi, &count, (unsigned long long)hw);
     rc = capture_rebuild(c, hi);
     if (rc) return rc;
+    issue_step_tail(c, c->stream, dt, &count, (unsigned long long)hw);
     GM_CUDA(c, cudaStreamEndCapture(c->stream, &body));
     GM_CUDA(c, cudaGraphInstantiate(&c->loop_exec, g, 0));
     c->loop_dt = dt;
@@ -1031,22 +1041,22 @@ int finish_steps(gm_ctx *c, double dt) {
 
 int run_direct(gm_ctx *c, double dt, int64_t n_steps);
 
-// n resident steps (one graph launch each, one for all of the persistent
-// form's, or direct launches), then the
-// closing half-kick; nothing waits for the device.
+// n resident steps (one graph launch for all, one each, or direct launches),
+// then the closing half-kick; nothing waits for the device.
 // The steps themselves: after them the resident positions are final (the
 // rest of the call evaluates forces and the closing half-kick).
 int launch_loop(gm_ctx *c, double dt, int64_t n_steps) {
     c->far_marked = false;  // a step may rebuild
     const bool pf = persistent_form(c) && n_steps > 0;
-    int rc = pf ? begin_persistent(c, true, n_steps) : begin_constrained(c);
+    int rc = pf ? begin_persistent(c, true, n_steps) : begin_constrained(c, n_steps);
     if (rc) return rc;
     if (!c->use_graph) {
         rc = run_direct(c, dt, n_steps);
-    } else if (pf && gm_step_loops(force_args(c))) {
+    } else if (n_steps > 1 && loops(c)) {
         rc = capture_loop(c, dt);
         if (rc) return rc;
-        GM_CUDA(c, cudaGraphLaunch(c->loop_exec, c->stream));  // (its launches are counted on the device)
+        GM_CUDA(c, cudaGraphLaunch(c->loop_exec, c->stream));
+        if (!pf) c->launches += c->launches_per_step * n_steps;  // (the persistent form's are counted on the device)
     } else {
         rc = capture_graph(c, dt);
         if (rc) return rc;

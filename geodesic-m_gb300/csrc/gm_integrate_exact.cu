@@ -879,6 +879,13 @@ __device__ __forceinline__ void free_kick(const ClusterArgs &c, const SolveStepA
     }
 }
 
+// The WHILE node round the step ends unless RATTLE's bookkeeping asks for
+// another step (a barrier that times out, in either launch, skips that).
+__device__ __forceinline__ void loop_off(const SolveStepArgs &sa) {
+    if (sa.loop && blockIdx.x == 0 && threadIdx.x == 0)
+        cudaGraphSetConditional((cudaGraphConditionalHandle)sa.loop, 0u);
+}
+
 // The ends of the two kernels: the last block's bookkeeping.
 __device__ __forceinline__ void shake_tail(const SolveStepArgs &sa, DevStatus *st, unsigned T, bool fail, int need,
                                            int bad) {
@@ -914,6 +921,11 @@ __device__ __forceinline__ void rattle_tail(const SolveStepArgs &sa, DevStatus *
                 st->shake_sum += st->shake_T;
                 st->rattle_sum += T;
             }
+            if (sa.loop) {
+                const long long left = sy->todo - 1;
+                sy->todo = left;
+                cudaGraphSetConditional((cudaGraphConditionalHandle)sa.loop, left > 0 ? 1u : 0u);
+            }
         }
     }
 }
@@ -923,6 +935,7 @@ __global__ void __launch_bounds__(128) shake_step_kernel(ClusterArgs c, SolveSte
     SolveSync *sy = sa.sync;
     const int n = sa.n, tid = blockIdx.x * blockDim.x + threadIdx.x, warp = tid >> 5;
     const bool err0 = gm_ld_acquire(&st->error) != 0;  // before any block may change it (the barrier)
+    loop_off(sa);
     const bool lanes = warp < c.n_lane_warps;            // warp-uniform
     int need = 0, bad = 0;
     StarLane s;
@@ -1222,6 +1235,7 @@ __global__ void __launch_bounds__(32) shake_comp_kernel(ClusterArgs c, SolveStep
     const bool err0 = gm_ld_acquire(&st->error) != 0;
     const bool lanes = warp < 4 * c.n_lane_warps;
     int need = 0, bad = 0;
+    loop_off(sa);
     CompLane s;
     LaneGroup g;
     double pc = 0.0, vc = 0.0, ph = 0.0, vh = 0.0;  // before the drift; after the kick
@@ -1323,6 +1337,13 @@ __global__ void __launch_bounds__(32) rattle_comp_kernel(ClusterArgs c, SolveSte
         if (s.k >= 0 && sub < 3) sa.vel[s.d * n + s.h] = s.y;
     }
     rattle_tail(sa, st, T, fail);
+}
+
+__global__ void solve_begin_kernel(SolveSync *two, long long todo) {
+    SolveSync z{};
+    two[0] = z;
+    z.todo = todo;
+    two[1] = z;
 }
 
 __global__ void reset_T(DevStatus *st, int rattle) {
@@ -1675,6 +1696,9 @@ void launch_cooperative(void (*kernel)(A...), int blocks, int threads, cudaStrea
 }
 }  // namespace
 
+void gm_launch_solve_begin(SolveSync *two, long long todo, cudaStream_t s) {
+    solve_begin_kernel<<<1, 1, 0, s>>>(two, todo);
+}
 void gm_launch_shake_step(const ClusterArgs &c, const SolveStepArgs &sa, const PackArgs &pk, int threads, int blocks,
                           bool quads, cudaStream_t s) {
     launch_cooperative<ClusterArgs, SolveStepArgs, PackArgs>(quads ? shake_comp_kernel : shake_step_kernel, blocks,

@@ -492,6 +492,7 @@ struct SolveSync {
     unsigned int arrive, gen;  // grid barrier
     unsigned int T;            // largest iteration count of phase 1
     unsigned int fail;         // a cluster of phase 1 did not converge
+    long long todo;            // RATTLE's: steps left in the call
 };
 struct SolveStepArgs {
     int n, n_free;
@@ -500,6 +501,7 @@ struct SolveStepArgs {
     long long *force;
     const double *ref;
     double dt_half, dt, inv_dt, thr_sq, far_sq;
+    unsigned long long loop;   // handle of the WHILE node round the step, or 0
     unsigned long long cond;
     const int *atom_sys;
     unsigned int *sys_flag, *sys_far;
@@ -508,6 +510,8 @@ struct SolveStepArgs {
 // Threads per block and blocks (all co-resident) of both kernels; blocks 0
 // when the system's clusters do not fit.
 void gm_solve_step_grid(const ClusterArgs &c, int n_free, int *threads, int *blocks, bool *quads);
+// Clears the two solves' words; `todo`: the steps of the call.
+void gm_launch_solve_begin(SolveSync *two, long long todo, cudaStream_t s);
 void gm_launch_shake_step(const ClusterArgs &c, const SolveStepArgs &sa, const PackArgs &pk, int threads, int blocks,
                           bool quads, cudaStream_t s);
 void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int threads, int blocks, bool quads,
