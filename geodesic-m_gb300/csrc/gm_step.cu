@@ -205,39 +205,88 @@ step_persistent_kernel(ForceArgs fa, StepArgs sa, PackArgs pk) {
         }
         const int n = sa.n;
         int need = 0, bad = 0;
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-            double np[3];
-            if (!err0) {
-                const double inv_m = sa.inv_mass[i];
-                for (int d = 0; d < 3; d++) {
-                    const double f = __dmul_rn((double)__ldcg(fa.force + d * n + i), GM_FIX_INV);
-                    const double kick = __dmul_rn(__dmul_rn(__dmul_rn(sa.dt_half, f), inv_m), GM_FORCE_TO_ACCEL);
-                    double v = sa.vel[d * n + i];
-                    if (tail0) v = __dadd_rn(v, kick);
-                    v = __dadd_rn(v, kick);
-                    const double p = sa.pos[d * n + i];
-                    sa.dref[d * n + i] = p;
-                    np[d] = __dadd_rn(p, __dmul_rn(sa.dt, v));
-                    sa.pos[d * n + i] = np[d];
-                    sa.vel[d * n + i] = gm_div_by_dt(__dsub_rn(np[d], p), sa.dt, sa.inv_dt);
+        if constexpr (QUAD) {
+            // a component per lane, the fourth lane the charge: an FP64
+            // instruction costs a scheduler the same for one lane as for 32,
+            // and a small system has schedulers to spare
+            for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ((4 * n + 31) & ~31); e += gridDim.x * blockDim.x) {
+                const int i = e >> 2, d = e & 3;
+                int sys = 0;
+                double dx = 0.0;
+                if (i < n) {
+                    sys = sa.atom_sys[i];
+                    float *rec = reinterpret_cast<float *>(pk.coord + 2 * pk.slot_of[i]);
+                    if (d < 3) {
+                        const double p = sa.pos[d * n + i];
+                        double np = p;
+                        if (!err0) {
+                            const double f = __dmul_rn((double)__ldcg(fa.force + d * n + i), GM_FIX_INV);
+                            const double kick =
+                                __dmul_rn(__dmul_rn(__dmul_rn(sa.dt_half, f), sa.inv_mass[i]), GM_FORCE_TO_ACCEL);
+                            double v = sa.vel[d * n + i];
+                            if (tail0) v = __dadd_rn(v, kick);
+                            v = __dadd_rn(v, kick);
+                            sa.dref[d * n + i] = p;
+                            np = __dadd_rn(p, __dmul_rn(sa.dt, v));
+                            sa.pos[d * n + i] = np;
+                            sa.vel[d * n + i] = gm_div_by_dt(__dsub_rn(np, p), sa.dt, sa.inv_dt);
+                        }
+                        gm_pack_component(rec + d, __dsub_rn(np, pk.grid[sys].origin[d]));
+                        fa.force[d * n + i] = 0;
+                        bad |= !isfinite(np);
+                        dx = __dsub_rn(np, sa.ref[d * n + i]);
+                    } else {
+                        const float2 qw = pk.qw[i];
+                        rec[3] = qw.x;
+                        rec[7] = qw.y;
+                    }
                 }
-            } else {
-                for (int d = 0; d < 3; d++) np[d] = sa.pos[d * n + i];
+                const double sq = __dmul_rn(dx, dx);
+                const double d2 = __dadd_rn(__dadd_rn(__shfl_sync(full, sq, 0, 4), __shfl_sync(full, sq, 1, 4)),
+                                            __shfl_sync(full, sq, 2, 4));
+                if (i < n) {
+                    if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sys] = 1u;
+                    if (d2 > sa.thr_sq) {
+                        sa.sys_flag[sys] = 1u;
+                        need = 1;
+                    }
+                }
             }
-            const int sl = pk.slot_of[i];
-            const GridInfo *g = pk.grid + sa.atom_sys[i];
-            gm_pack_record(pk.coord + 2 * sl, __dsub_rn(np[0], g->origin[0]), __dsub_rn(np[1], g->origin[1]),
-                           __dsub_rn(np[2], g->origin[2]), pk.qw[i]);
-            for (int d = 0; d < 3; d++) fa.force[d * n + i] = 0;
-            bad |= !(isfinite(np[0]) && isfinite(np[1]) && isfinite(np[2]));
-            const double dx = __dsub_rn(np[0], sa.ref[i]), dy = __dsub_rn(np[1], sa.ref[n + i]),
-                         dz = __dsub_rn(np[2], sa.ref[2 * n + i]);
-            const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-            const bool moved = d2 > sa.thr_sq;
-            if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sa.atom_sys[i]] = 1u;
-            if (moved) {
-                sa.sys_flag[sa.atom_sys[i]] = 1u;
-                need = 1;
+        } else {
+            for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+                double np[3];
+                if (!err0) {
+                    const double inv_m = sa.inv_mass[i];
+                    for (int d = 0; d < 3; d++) {
+                        const double f = __dmul_rn((double)__ldcg(fa.force + d * n + i), GM_FIX_INV);
+                        const double kick = __dmul_rn(__dmul_rn(__dmul_rn(sa.dt_half, f), inv_m), GM_FORCE_TO_ACCEL);
+                        double v = sa.vel[d * n + i];
+                        if (tail0) v = __dadd_rn(v, kick);
+                        v = __dadd_rn(v, kick);
+                        const double p = sa.pos[d * n + i];
+                        sa.dref[d * n + i] = p;
+                        np[d] = __dadd_rn(p, __dmul_rn(sa.dt, v));
+                        sa.pos[d * n + i] = np[d];
+                        sa.vel[d * n + i] = gm_div_by_dt(__dsub_rn(np[d], p), sa.dt, sa.inv_dt);
+                    }
+                } else {
+                    for (int d = 0; d < 3; d++) np[d] = sa.pos[d * n + i];
+                }
+                const int sl = pk.slot_of[i];
+                const GridInfo *g = pk.grid + sa.atom_sys[i];
+                gm_pack_record(pk.coord + 2 * sl, __dsub_rn(np[0], g->origin[0]), __dsub_rn(np[1], g->origin[1]),
+                               __dsub_rn(np[2], g->origin[2]), pk.qw[i]);
+                for (int d = 0; d < 3; d++) fa.force[d * n + i] = 0;
+                bad |= !(isfinite(np[0]) && isfinite(np[1]) && isfinite(np[2]));
+                const double dx = __dsub_rn(np[0], sa.ref[i]), dy = __dsub_rn(np[1], sa.ref[n + i]),
+                             dz = __dsub_rn(np[2], sa.ref[2 * n + i]);
+                const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+                const bool moved = d2 > sa.thr_sq;
+                if (gm_moved_far(d2, sa.far_sq)) sa.sys_far[sa.atom_sys[i]] = 1u;
+                if (moved) {
+                    sa.sys_flag[sa.atom_sys[i]] = 1u;
+                    need = 1;
+                }
             }
         }
         need = __syncthreads_or(need);
@@ -336,7 +385,7 @@ int gm_step_persistent_blocks(const ForceArgs &fa) {
     const bool quad = fa.quad && !gtab;
     const int chunk = quad ? kStepThreads : ticket_terms<true>(fa), warps = quad ? 1 : kStepThreads / 32;
     const long long tickets = (long long)fa.n_groups * fa.split + bonded_tickets(fa, chunk) + pair14_tickets(fa, chunk);
-    const long long fill = (tickets + warps - 1) / warps, atoms = ((long long)fa.n + kStepThreads - 1) / kStepThreads;
+    const long long fill = (tickets + warps - 1) / warps, atoms = ((long long)fa.n * (quad ? 4 : 1) + kStepThreads - 1) / kStepThreads;
     const long long want = fill > atoms ? fill : atoms;
     return (int)(want < (long long)per_sm * sms ? (want > 0 ? want : 1) : (long long)per_sm * sms);
 }
