@@ -15,7 +15,7 @@ CALLS = (1, 2, 63, 64, 65, 130)
 
 
 @pytest.mark.parametrize("n,box,skin", [(33, None, 12.0), (224, None, 10.2), (224, None, 12.0), (700, None, 10.3),
-                                        (700, 45.0, 12.0), (3200, None, 10.5)])
+                                        (700, 45.0, 12.0), (3200, None, 10.5), (3201, None, 12.0)])
 def test_calls_of_any_length_match_the_kernel_graph(n, box, skin):
     atoms, topo, state, _ = synth.generate(n, seed=11 + n, relax_iters=60)
     pos0 = np.ascontiguousarray(state.pos)
