@@ -1033,9 +1033,14 @@ int capture_loop(gm_ctx *c, double dt) {
 
 // After the last resident step of a call: the closing half-kick that the
 // unconstrained step leaves to the next step (nothing pending otherwise).
-int finish_steps(gm_ctx *c, double dt) {
+// `energy`: the same launch sums the energy partials (refresh_energy).
+int finish_steps(gm_ctx *c, double dt, bool energy = false) {
     if (c->n_clusters) return GM_OK;
-    gm_launch_kick_tail(c->n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, c->stream);
+    const ForceArgs fa = force_args(c);
+    const bool sum = energy && c->energy_stale;
+    gm_launch_kick_tail(c->n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, sum ? fa.epart : nullptr,
+                        fa.n_epart_total, fa.energy, c->stream);
+    if (sum) c->energy_stale = false;
     c->launches++;
     GM_CUDA(c, cudaGetLastError());
     return GM_OK;
@@ -1073,9 +1078,9 @@ int launch_loop(gm_ctx *c, double dt, int64_t n_steps) {
 
 // After launch_loop: the persistent form's forces at the final positions,
 // then the pending closing half-kick.
-int launch_end(gm_ctx *c, double dt, int64_t n_steps) {
+int launch_end(gm_ctx *c, double dt, int64_t n_steps, bool energy = false) {
     int rc = persistent_form(c) && n_steps > 0 ? end_persistent(c) : GM_OK;
-    return rc ? rc : finish_steps(c, dt);
+    return rc ? rc : finish_steps(c, dt, energy);
 }
 
 int launch_steps(gm_ctx *c, double dt, int64_t n_steps) {
@@ -2275,7 +2280,7 @@ int32_t gm_steps(gm_ctx *c, double *px, double *py, double *pz, double *vx, doub
     GM_CUDA(c, cudaStreamWaitEvent(c->xfer, c->ev_xfer_in, 0));
     rc = download3(c, c->d_pos, px, py, pz, c->xfer);
     if (!rc) GM_CUDA(c, cudaEventRecord(c->ev_xfer_out, c->xfer));
-    if (!rc) rc = launch_end(c, dt, n_steps);
+    if (!rc) rc = launch_end(c, dt, n_steps, energy != nullptr);
     if (!rc) GM_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_xfer_out, 0));
     if (rc) {
         cudaStreamSynchronize(c->xfer);

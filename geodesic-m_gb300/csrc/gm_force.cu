@@ -226,27 +226,9 @@ __global__ void __launch_bounds__(GM_BONDED_THREADS) bonded_pair14_kernel(ForceA
     }
 }
 
-// Fixed-order sum of all energy partials (pair items, bonded blocks, 1-4
-// blocks) into the FP64 total: deterministic for a given launch shape.
 __global__ void __launch_bounds__(256) energy_kernel(const double *epart, int n, double *out) {
     __shared__ double s[256];
-    __shared__ bool last;
-    double *part = out + 1;
-    unsigned *arrived = reinterpret_cast<unsigned *>(part + GM_SUM_BLOCKS);
-    const double mine = gm_share_sum256(epart, n, s);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = mine;
-        __threadfence();
-        last = atomicAdd(arrived, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    const double e = gm_blocks_sum256(part, s);
-    if (threadIdx.x == 0) {
-        *out = e;
-        *arrived = 0u;
-    }
+    gm_energy_block(epart, n, out, s);
 }
 
 }  // namespace

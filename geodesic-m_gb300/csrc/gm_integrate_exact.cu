@@ -1561,10 +1561,18 @@ __global__ void kick_drift_check_kernel(int n, double *pos, double *vel, double 
 }
 // The closing half-kick of the last unconstrained resident step and its step
 // count, when pending; the last block clears the flag after every block has
-// read it.
-__global__ void kick_tail_kernel(int n, double *vel, const long long *force, const double *inv_mass, double dt_half,
-                                 DevStatus *st) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// read it.  With `epart` the first GM_SUM_BLOCKS blocks sum the energy partials
+// instead (a launch of its own took 5-7 us of a one-step call).
+__global__ void __launch_bounds__(256) kick_tail_kernel(int n, double *vel, const long long *force,
+                                                        const double *inv_mass, double dt_half, DevStatus *st,
+                                                        const double *epart, int n_epart, double *energy) {
+    __shared__ double s[256];
+    const int first = epart ? GM_SUM_BLOCKS : 0;
+    if ((int)blockIdx.x < first) {
+        gm_energy_block(epart, n_epart, energy, s);
+        return;
+    }
+    int i = ((int)blockIdx.x - first) * blockDim.x + threadIdx.x;
     const bool go = st->tail_pending != 0 && st->error == 0;
     if (i < n && go) {
         const double inv_m = inv_mass[i];
@@ -1577,7 +1585,7 @@ __global__ void kick_tail_kernel(int n, double *vel, const long long *force, con
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned done = atomicAdd(&st->blocks_done, 1u);
-        if (done == gridDim.x - 1) {
+        if (done == gridDim.x - first - 1) {
             st->blocks_done = 0;
             if (go) st->step += 1;
             st->tail_pending = 0u;
@@ -1616,8 +1624,9 @@ void gm_launch_kick_drift_check(int n, double *pos, double *vel, double *dref, l
                                                               sys_flag, sys_far, pk);
 }
 void gm_launch_kick_tail(int n, double *vel, const long long *force, const double *inv_mass, double dt_half,
-                         DevStatus *st, cudaStream_t s) {
-    kick_tail_kernel<<<gm_check_blocks(n), 256, 0, s>>>(n, vel, force, inv_mass, dt_half, st);
+                         DevStatus *st, const double *epart, int n_epart, double *energy, cudaStream_t s) {
+    kick_tail_kernel<<<gm_check_blocks(n) + (epart ? GM_SUM_BLOCKS : 0), 256, 0, s>>>(n, vel, force, inv_mass, dt_half,
+                                                                                     st, epart, n_epart, energy);
 }
 
 void gm_launch_check(int n, const double *pos, const double *ref, double thr_sq, double far_sq, DevStatus *st,

@@ -175,6 +175,29 @@ __device__ __forceinline__ double gm_blocks_sum256(const double *part, double *s
     return r;
 }
 
+// Fixed-order sum of all energy partials (pair items, bonded blocks, 1-4
+// blocks) into the FP64 total: deterministic for a given launch shape.  Blocks
+// 0..GM_SUM_BLOCKS-1 of the launch call it, 256 threads each, `s` 256 doubles.
+__device__ __forceinline__ void gm_energy_block(const double *epart, int n, double *out, double *s) {
+    __shared__ bool last;
+    double *part = out + 1;
+    unsigned *arrived = reinterpret_cast<unsigned *>(part + GM_SUM_BLOCKS);
+    const double mine = gm_share_sum256(epart, n, s);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = mine;
+        __threadfence();
+        last = atomicAdd(arrived, 1u) == GM_SUM_BLOCKS - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const double e = gm_blocks_sum256(part, s);
+    if (threadIdx.x == 0) {
+        *out = e;
+        *arrived = 0u;
+    }
+}
+
 // Both float4 of a slot's (hi, lo) coordinate pair in one 256-bit load
 // through the read-only path (the pair is 32-byte aligned).
 __device__ __forceinline__ void gm_ld_coord(const float4 *p, float4 &h, float4 &l) {
@@ -552,8 +575,9 @@ void gm_launch_frame(int n, const double *pos, const double *vel, const long lon
                      const double *mass, double dt_half, DevStatus *st, const FrameArgs &f, cudaStream_t s);
 // The closing half-kick and step count of the last unconstrained resident
 // step, when one is pending (a no-op otherwise).
+// With `epart` the launch sums the n_epart energy partials into `energy` too.
 void gm_launch_kick_tail(int n, double *vel, const long long *force, const double *inv_mass, double dt_half,
-                         DevStatus *st, cudaStream_t s);
+                         DevStatus *st, const double *epart, int n_epart, double *energy, cudaStream_t s);
 void gm_launch_kinetic(int n, const double *vel, const double *mass, double *partials, int blocks, double *out,
                        cudaStream_t s);
 void gm_launch_forces_out(int n, const long long *force, double *out, cudaStream_t s);
