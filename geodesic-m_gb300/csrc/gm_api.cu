@@ -440,11 +440,12 @@ long long issue_shake(gm_ctx *c, cudaStream_t s, bool resident) {
 // ---- kernel sequences (each counted for gm_counters[3]) -------------------
 
 // The list rebuild of every system (all) or of the systems the rebuild check
-// flagged; the flags are cleared at the end.
-int seq_rebuild(gm_ctx *c, cudaStream_t s, bool all) {
+// flagged; the flags are cleared at the end.  `wrap`: the positions are wrapped
+// into the box first.
+int seq_rebuild(gm_ctx *c, cudaStream_t s, bool all, bool wrap = true) {
     ListArgs a = list_args(c);
     if (all) gm_launch_flags(a, true, s);
-    gm_launch_wrap(a, c->d_pos, s);
+    if (wrap) gm_launch_wrap(a, c->d_pos, s);
     gm_launch_grid(a, s);
     gm_launch_bin(a, s);
     gm_launch_pack(a, c->fp64, s);
@@ -735,7 +736,9 @@ int do_build(gm_ctx *c, bool all = true) {
     for (int attempt = 0; attempt < 6; attempt++) {
         int rc = reset_status(c);
         if (rc) return rc;
-        c->launches += seq_rebuild(c, c->stream, all || attempt > 0);
+        // a build wraps once (neighbor.rs:13-15): what the first attempt put
+        // exactly on a face must not become 0 in the next
+        c->launches += seq_rebuild(c, c->stream, all || attempt > 0, !(all && attempt > 0));
         c->far_marked = false;
         rc = check_status(c, nullptr);
         if (attempt == 0) counted = c->h_status->n_rebuilds;

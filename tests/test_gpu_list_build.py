@@ -85,3 +85,24 @@ def test_rebuilds_of_a_run_that_outgrow_the_staging_area(n, box, skin, steps):
         other.close()
         assert np.max(np.abs(f - fr) / np.maximum(np.abs(fr), 1.0)) <= 1e-5, first
     be.close()
+
+
+def test_wrap_at_the_faces():
+    """The wrap into the box is x - L floor(x / L) in FP64, bit for bit, at and
+    around the faces and the zeros."""
+    L = 40.0
+    x = np.array([0.0, -0.0, 5e-324, -5e-324, -1e-17, 1e-17, L, np.nextafter(L, 0), np.nextafter(L, 99), -L, 2 * L,
+                  np.nextafter(2 * L, 0), 3.25, -3.25, 97.5, -1e6 / 3])
+    n = 3 * len(x)
+    pos = np.stack([np.linspace(1, 39, n)] * 3)
+    for d in range(3):  # each value in each component, the atoms apart in another
+        pos[d, d * len(x):(d + 1) * len(x)] = x
+    pos = np.ascontiguousarray(pos)
+    atoms = amber.AtomData(np.full(n, 3.0), np.full(n, 0.1), np.full(n, 12.0), np.zeros(n), np.full(n, 1, np.uint8),
+                           np.zeros(n, np.uint32), [])
+    p = backend.SimParams(box_size=(L,) * 3, periodic=True, r_cutoff=8.0, r_skin=10.0, r_switch=7.0)
+    be = backend.CudaBackend(atoms, amber.BondedTopology.empty(), p)
+    want = pos - L * np.floor(pos / L)
+    be.build_neighbor_list(pos)
+    be.close()
+    assert np.array_equal(pos.view(np.uint64), want.view(np.uint64))
