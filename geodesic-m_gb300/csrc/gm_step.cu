@@ -360,10 +360,29 @@ __global__ void step_begin_kernel(StepSync *sy, unsigned fresh, long long todo) 
 
 using StepKernel = void (*)(ForceArgs, StepArgs, PackArgs);
 
+// Shared memory of a block without an opt-in.
+constexpr size_t kSharedLimit = 48 * 1024;
+// The QUAD kernels' static shared memory (quad_phase's s_e, the barrier's and
+// the step's words: 1,024 and 16 bytes), rounded up.
+constexpr size_t kQuadStatic = 2048;
+static_assert(sizeof(double) * kStepThreads + 256 <= kQuadStatic, "quad_phase's energies");
+
+size_t table_bytes(const ForceArgs &fa) { return sizeof(float4) * (size_t)fa.ntypes * fa.ntypes; }
+
+// A batch reads its [system][type][type] tables through L1, as does a single
+// system whose table passes 48 KB.
+bool global_table(const ForceArgs &fa) { return fa.e_sys != nullptr || table_bytes(fa) > kSharedLimit; }
+
+// A small system's block per pair item, where its table leaves room for the
+// kernel's own shared memory (up to 54 types; with 55 the table alone fits).
+bool quad_form(const ForceArgs &fa) {
+    return fa.quad && !global_table(fa) && table_bytes(fa) + kQuadStatic <= kSharedLimit;
+}
+
 template <bool STEP>
 StepKernel pick(const ForceArgs &fa, bool gtab) {
 #define GM_STEPK(P, Q, B, M, D) return step_persistent_kernel<P, Q, B, M, STEP, D>
-#define GM_STEPB(P, Q, M) { if (gtab) GM_STEPK(P, Q, true, M, false); else if (fa.quad) GM_STEPK(P, Q, false, M, true); \
+#define GM_STEPB(P, Q, M) { if (gtab) GM_STEPK(P, Q, true, M, false); else if (quad_form(fa)) GM_STEPK(P, Q, false, M, true); \
                             else GM_STEPK(P, Q, false, M, false); }
 #define GM_STEPQ(P, M) { if (fa.coulomb) GM_STEPB(P, true, M) else GM_STEPB(P, false, M) }
     if (fa.bonded_mi) GM_STEPQ(true, true)
@@ -374,27 +393,25 @@ StepKernel pick(const ForceArgs &fa, bool gtab) {
 #undef GM_STEPK
 }
 
-// A batch reads its [system][type][type] tables through L1, as does a single
-// system whose table passes 48 KB.
-bool global_table(const ForceArgs &fa) {
-    return fa.e_sys != nullptr || sizeof(float4) * (size_t)fa.ntypes * fa.ntypes > 48 * 1024;
-}
-
 }  // namespace
 
-bool gm_step_loops(const ForceArgs &fa) { return fa.quad && !global_table(fa); }
+bool gm_step_loops(const ForceArgs &fa) { return quad_form(fa); }
 
 int gm_step_persistent_blocks(const ForceArgs &fa) {
     const bool gtab = global_table(fa);
-    const size_t smem = gtab ? 0 : sizeof(float4) * (size_t)fa.ntypes * fa.ntypes;
-    int dev = 0, sms = 0, per_sm = 0;
+    const size_t smem = gtab ? 0 : table_bytes(fa);
+    int dev = 0, sms = 0, per_sm = 0, per_sm_forces = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick<true>(fa, gtab), kStepThreads, smem) != cudaSuccess)
         return 0;
+    // the force phase alone has more static shared memory than the step
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_forces, pick<false>(fa, gtab), kStepThreads, smem) !=
+            cudaSuccess || per_sm_forces == 0)
+        return 0;
     // no more blocks than the tickets (a warp each, a block with quad) or the atoms fill: a
     // small system's barrier waits for fewer arrivals
-    const bool quad = fa.quad && !gtab;
+    const bool quad = quad_form(fa);
     const int chunk = quad ? kStepThreads : ticket_terms<true>(fa), warps = quad ? 1 : kStepThreads / 32;
     const long long tickets = (long long)fa.n_groups * fa.split + bonded_tickets(fa, chunk) + pair14_tickets(fa, chunk);
     const long long fill = (tickets + warps - 1) / warps, atoms = ((long long)fa.n * (quad ? 4 : 1) + kStepThreads - 1) / kStepThreads;
@@ -408,7 +425,7 @@ void gm_launch_step_persistent(const ForceArgs &fa, const StepArgs &sa, const Pa
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(kStepThreads);
-    cfg.dynamicSmemBytes = gtab ? 0 : sizeof(float4) * (size_t)fa.ntypes * fa.ntypes;
+    cfg.dynamicSmemBytes = gtab ? 0 : table_bytes(fa);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
@@ -423,8 +440,7 @@ void gm_launch_forces_persistent(const ForceArgs &fa, StepSync *sync, int blocks
     StepArgs sa{};
     sa.sync = sync;
     PackArgs pk{};
-    const size_t smem = gtab ? 0 : sizeof(float4) * (size_t)fa.ntypes * fa.ntypes;
-    pick<false>(fa, gtab)<<<blocks, kStepThreads, smem, s>>>(fa, sa, pk);
+    pick<false>(fa, gtab)<<<blocks, kStepThreads, gtab ? 0 : table_bytes(fa), s>>>(fa, sa, pk);
 }
 
 void gm_launch_step_begin(StepSync *sync, bool fresh, long long todo, cudaStream_t s) {
