@@ -1115,6 +1115,27 @@ int stage_positions(gm_ctx *c, const double *px, const double *py, const double 
     return GM_OK;
 }
 
+// Caller positions for a call that reads them but evaluates no forces: into the
+// resident array, or, while the resident forces are current, beside it with a
+// comparison on the device (no wait of its own).  After the caller's read of
+// the status word settle_positions makes them resident if they differ, and the
+// forces stale with them.  The status word was reset on the stream before.
+int put_positions(gm_ctx *c, const double *px, const double *py, const double *pz, double **where) {
+    *where = c->forces_current ? c->d_dref : c->d_pos;
+    int rc = upload3(c, *where, px, py, pz);
+    if (rc || !c->forces_current) return rc;
+    gm_launch_differs(c->n, c->d_dref, c->d_pos, &c->d_status->differs, c->stream);
+    c->launches++;
+    return GM_OK;
+}
+int settle_positions(gm_ctx *c, const double *where) {
+    if (where == c->d_pos || !c->h_status->differs) return GM_OK;
+    c->forces_current = false;
+    GM_CUDA(c, cudaMemcpyAsync(c->d_pos, c->d_dref, sizeof(double) * 3 * (size_t)c->n, cudaMemcpyDeviceToDevice,
+                               c->stream));
+    return GM_OK;
+}
+
 // The step without a graph: same kernels on the stream, the rebuild decision
 // read back on the host after each check (profilers cannot look inside
 // graphs that hold conditional nodes).
@@ -1908,6 +1929,7 @@ int32_t gm_compute_forces(gm_ctx *c, const double *px, const double *py, const d
     };
     if (cudaSetDevice(c->device) != cudaSuccess) return poison(GM_ERR_DEVICE);
     if (!c->built) return poison(fail(c, GM_ERR_NOT_BUILT, "compute_forces before build_neighbor_list"));
+    c->forces_current = false;  // until the new ones are known to be sound
     int rc = upload3(c, c->d_pos, px, py, pz);
     if (rc) return poison(rc);
     rc = reset_status(c);
@@ -1937,14 +1959,16 @@ int32_t gm_needs_rebuild(gm_ctx *c, const double *px, const double *py, const do
     if (!c || !result) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
     if (!c->built) { *result = 1; return GM_OK; }
-    int rc = upload3(c, c->d_pos, px, py, pz);
+    int rc = reset_status(c);
     if (rc) return rc;
-    rc = reset_status(c);
+    double *pos;
+    rc = put_positions(c, px, py, pz, &pos);
     if (rc) return rc;
     const double half_skin = (c->p.r_skin - c->p.r_cutoff) / 2.0;
-    gm_launch_check(c->n, c->d_pos, c->d_ref, half_skin * half_skin, far_sq(c), c->d_status, 0ull,
+    gm_launch_check(c->n, pos, c->d_ref, half_skin * half_skin, far_sq(c), c->d_status, 0ull,
                     gm_check_blocks(c->n), c->d_atom_sys, c->d_sys_flag, c->d_sys_far, c->stream);
     rc = st_read(c);
+    if (!rc) rc = settle_positions(c, pos);
     if (rc) return rc;
     *result = c->h_status->rebuild ? 1 : 0;
     gm_launch_flags(list_args(c), false, c->stream);  // a query: leave no system marked
@@ -1957,6 +1981,7 @@ int32_t gm_geodesic_drift(gm_ctx *c, double *px, double *py, double *pz, double 
                           double dt, uint64_t step, gm_convergence *err) {
     if (!c) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
+    c->forces_current = false;
     int rc = upload3(c, c->d_pos, px, py, pz);
     if (!rc) rc = upload3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
@@ -1973,7 +1998,6 @@ int32_t gm_geodesic_drift(gm_ctx *c, double *px, double *py, double *pz, double 
     rc = download3(c, c->d_pos, px, py, pz);
     if (!rc) rc = download3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
-    c->forces_current = false;
     return check_status(c, err);
 }
 
@@ -1997,16 +2021,19 @@ int32_t gm_constrain_velocities(gm_ctx *c, const double *px, const double *py, c
     if (!c) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
     if (!c->n_clusters) return GM_OK;  // constraint.rs:183-186
-    int rc = upload3(c, c->d_pos, px, py, pz);
+    int rc = reset_status(c, step);
+    if (rc) return rc;
+    double *pos;
+    rc = put_positions(c, px, py, pz, &pos);
     if (!rc) rc = upload3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
-    rc = reset_status(c, step);
-    if (rc) return rc;
-    gm_launch_rattle(cluster_args(c), c->n, c->d_pos, c->d_vel, c->stream);
+    gm_launch_rattle(cluster_args(c), c->n, pos, c->d_vel, c->stream);
     c->launches += 3;
     rc = download3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
-    return check_status(c, err);
+    rc = check_status(c, err);
+    const int rs = settle_positions(c, pos);
+    return rc ? rc : rs;
 }
 
 int32_t gm_kinetic_energy(gm_ctx *c, const double *vx, const double *vy, const double *vz, double *ke) {
