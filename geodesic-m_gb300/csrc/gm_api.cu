@@ -86,6 +86,7 @@ struct gm_ctx {
     int *d_count_in = nullptr, *d_gmax_in = nullptr;  // without the last distance bucket
     unsigned int *d_sys_far = nullptr;                // see ForceArgs::sys_far
     bool far_marked = false;                          // every system is marked far
+    unsigned int *d_sys_wrapped = nullptr;            // systems that a build's first attempt has wrapped
     bool built = false;
     // exclusions
     int *d_excl_start = nullptr, *d_excl = nullptr;
@@ -441,11 +442,11 @@ long long issue_shake(gm_ctx *c, cudaStream_t s, bool resident) {
 
 // The list rebuild of every system (all) or of the systems the rebuild check
 // flagged; the flags are cleared at the end.  `wrap`: the positions are wrapped
-// into the box first.
-int seq_rebuild(gm_ctx *c, cudaStream_t s, bool all, bool wrap = true) {
+// into the box first, but those of the systems with nonzero `wrapped`.
+int seq_rebuild(gm_ctx *c, cudaStream_t s, bool all, bool wrap = true, const unsigned int *wrapped = nullptr) {
     ListArgs a = list_args(c);
     if (all) gm_launch_flags(a, true, s);
-    if (wrap) gm_launch_wrap(a, c->d_pos, s);
+    if (wrap) gm_launch_wrap(a, c->d_pos, wrapped, s);
     gm_launch_grid(a, s);
     gm_launch_bin(a, s);
     gm_launch_pack(a, c->fp64, s);
@@ -733,12 +734,18 @@ int do_build(gm_ctx *c, bool all = true) {
     // list build on the resident positions (every system, or the flagged
     // ones), growing the capacity on overflow (then rebuilding every system)
     unsigned long long counted = 0;
+    const bool some = !all && c->n_sys > 1;  // some systems of a batch, perhaps
     for (int attempt = 0; attempt < 6; attempt++) {
         int rc = reset_status(c);
         if (rc) return rc;
         // a build wraps once (neighbor.rs:13-15): what the first attempt put
-        // exactly on a face must not become 0 in the next
-        c->launches += seq_rebuild(c, c->stream, all || attempt > 0, !(all && attempt > 0));
+        // exactly on a face must not become 0 in the next, so a second one
+        // wraps only the systems of a batch that the first left out
+        if (attempt == 0 && some)
+            GM_CUDA(c, cudaMemcpyAsync(c->d_sys_wrapped, c->d_sys_flag, sizeof(unsigned int) * (size_t)c->n_sys,
+                                       cudaMemcpyDeviceToDevice, c->stream));
+        c->launches += seq_rebuild(c, c->stream, all || attempt > 0, attempt == 0 || (attempt == 1 && some),
+                                   attempt == 1 ? c->d_sys_wrapped : nullptr);
         c->far_marked = false;
         rc = check_status(c, nullptr);
         if (attempt == 0) counted = c->h_status->n_rebuilds;
@@ -1786,6 +1793,7 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         TRY(dupload(c, &c->d_group_sys, group_sys.data(), group_sys.size()));
         TRY(dalloc(c, &c->d_sys_flag, (size_t)n_sys));
         TRY(dalloc(c, &c->d_sys_far, (size_t)n_sys));
+        TRY(dalloc(c, &c->d_sys_wrapped, (size_t)n_sys));
         cudaMemset(c->d_sys_far, 0xFF, sizeof(unsigned int) * (size_t)n_sys);
         TRY(dalloc(c, &c->d_e_sys, (size_t)n_sys));
         cudaMemset(c->d_sys_flag, 0, sizeof(unsigned int) * (size_t)n_sys);

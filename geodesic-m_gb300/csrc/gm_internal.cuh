@@ -334,7 +334,8 @@ struct ListArgs {
 
 // set (every system) or clear the rebuild flags; clearing also clears status->rebuild
 void gm_launch_flags(const ListArgs &a, bool set, cudaStream_t s);
-void gm_launch_wrap(const ListArgs &a, double *pos, cudaStream_t s);
+// `done` (or nullptr): nonzero for the systems to leave as they are.
+void gm_launch_wrap(const ListArgs &a, double *pos, const unsigned int *done, cudaStream_t s);
 void gm_launch_grid(const ListArgs &a, cudaStream_t s);
 void gm_launch_bin(const ListArgs &a, cudaStream_t s);
 void gm_launch_build(const ListArgs &a, cudaStream_t s);

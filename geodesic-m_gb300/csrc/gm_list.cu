@@ -55,9 +55,10 @@ __global__ void clear_flags_kernel(ListArgs a) {
     if (s == 0) a.status->rebuild = 0u;
 }
 
-__global__ void wrap_kernel(ListArgs a, double *pos) {
+// `done` (or nullptr): systems that are wrapped already.
+__global__ void wrap_kernel(ListArgs a, double *pos, const unsigned int *done) {
     int a0, a1;
-    if (!sys_atoms(a, a0, a1)) return;
+    if (!sys_atoms(a, a0, a1) || (done && done[blockIdx.y])) return;
     const int n = a.n;
     for (int i = a0 + blockIdx.x * blockDim.x + threadIdx.x; i < a1; i += gridDim.x * blockDim.x) {
         pos[i] = exact_wrap(pos[i], a.box[0]);
@@ -840,9 +841,9 @@ void gm_launch_flags(const ListArgs &a, bool set, cudaStream_t s) {
     else clear_flags_kernel<<<(a.n_sys + 255) / 256, 256, 0, s>>>(a);
 }
 
-void gm_launch_wrap(const ListArgs &a, double *pos, cudaStream_t s) {
+void gm_launch_wrap(const ListArgs &a, double *pos, const unsigned int *done, cudaStream_t s) {
     if (!a.periodic || a.n == 0) return;
-    wrap_kernel<<<sys_grid(a, 256, 4096), 256, 0, s>>>(a, pos);
+    wrap_kernel<<<sys_grid(a, 256, 4096), 256, 0, s>>>(a, pos, done);
 }
 
 void gm_launch_grid(const ListArgs &a, cudaStream_t s) {

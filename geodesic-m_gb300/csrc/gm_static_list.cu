@@ -292,7 +292,7 @@ extern "C" int32_t gm_build_pairs_static(double *d_pos, int32_t n_atoms, const i
 
     if (cudaMemsetAsync(&S->status, 0, sizeof(DevStatus), s) != cudaSuccess) return GM_ERR_DEVICE;
     gm_launch_flags(a, true, s);
-    gm_launch_wrap(a, d_pos, s);  // neighbor.rs:10-16
+    gm_launch_wrap(a, d_pos, nullptr, s);  // neighbor.rs:10-16
     gm_launch_grid(a, s);
     gm_launch_bin(a, s);
 
