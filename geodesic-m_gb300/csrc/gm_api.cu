@@ -923,7 +923,7 @@ int issue_step_tail(gm_ctx *c, cudaStream_t s, double dt, long long *count, unsi
         k++;
     } else if (c->n_clusters) {
         gm_launch_half_kick(c->n, c->d_vel, c->d_force, c->d_inv_mass, dt / 2.0, c->d_status, s); k++;
-        gm_launch_rattle(cluster_args(c), c->n, c->d_pos, c->d_vel, s); k += 3;
+        gm_launch_rattle(cluster_args(c), c->n, c->d_pos, c->d_vel, true, s); k += 3;
         gm_launch_step(c->d_status, s); k++;
     }
     // (without constraints the closing half-kick is done by the next step's
@@ -1123,17 +1123,20 @@ int stage_positions(gm_ctx *c, const double *px, const double *py, const double 
 }
 
 // Caller positions for a call that reads them but evaluates no forces: into the
-// resident array, or, while the resident forces are current, beside it with a
-// comparison on the device (no wait of its own).  After the caller's read of
-// the status word settle_positions makes them resident if they differ, and the
-// forces stale with them.  The status word was reset on the stream before.
+// resident array, or, while the resident forces are current, beside it
+// (put_positions) with a comparison on the device after the status reset
+// (compare_positions; no wait of its own).  After the caller's read of the
+// status word settle_positions makes them resident if they differ, and the
+// forces stale with them.  (The uploads come before the reset: a copy from
+// pageable memory waits for kernels queued before it.)
 int put_positions(gm_ctx *c, const double *px, const double *py, const double *pz, double **where) {
     *where = c->forces_current ? c->d_dref : c->d_pos;
-    int rc = upload3(c, *where, px, py, pz);
-    if (rc || !c->forces_current) return rc;
-    gm_launch_differs(c->n, c->d_dref, c->d_pos, &c->d_status->differs, c->stream);
+    return upload3(c, *where, px, py, pz);
+}
+void compare_positions(gm_ctx *c, const double *where) {
+    if (where == c->d_pos) return;
+    gm_launch_differs(c->n, where, c->d_pos, &c->d_status->differs, c->stream);
     c->launches++;
-    return GM_OK;
 }
 int settle_positions(gm_ctx *c, const double *where) {
     if (where == c->d_pos || !c->h_status->differs) return GM_OK;
@@ -1967,11 +1970,11 @@ int32_t gm_needs_rebuild(gm_ctx *c, const double *px, const double *py, const do
     if (!c || !result) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
     if (!c->built) { *result = 1; return GM_OK; }
-    int rc = reset_status(c);
-    if (rc) return rc;
     double *pos;
-    rc = put_positions(c, px, py, pz, &pos);
+    int rc = put_positions(c, px, py, pz, &pos);
+    if (!rc) rc = reset_status(c);
     if (rc) return rc;
+    compare_positions(c, pos);
     const double half_skin = (c->p.r_skin - c->p.r_cutoff) / 2.0;
     gm_launch_check(c->n, pos, c->d_ref, half_skin * half_skin, far_sq(c), c->d_status, 0ull,
                     gm_check_blocks(c->n), c->d_atom_sys, c->d_sys_flag, c->d_sys_far, c->stream);
@@ -2029,14 +2032,14 @@ int32_t gm_constrain_velocities(gm_ctx *c, const double *px, const double *py, c
     if (!c) return GM_ERR_INVALID_ARGUMENT;
     GM_CUDA(c, cudaSetDevice(c->device));
     if (!c->n_clusters) return GM_OK;  // constraint.rs:183-186
-    int rc = reset_status(c, step);
-    if (rc) return rc;
     double *pos;
-    rc = put_positions(c, px, py, pz, &pos);
+    int rc = put_positions(c, px, py, pz, &pos);
     if (!rc) rc = upload3(c, c->d_vel, vx, vy, vz);
+    if (!rc) rc = reset_status(c, step);
     if (rc) return rc;
-    gm_launch_rattle(cluster_args(c), c->n, pos, c->d_vel, c->stream);
-    c->launches += 3;
+    compare_positions(c, pos);
+    gm_launch_rattle(cluster_args(c), c->n, pos, c->d_vel, false, c->stream);
+    c->launches += 2;
     rc = download3(c, c->d_vel, vx, vy, vz);
     if (rc) return rc;
     rc = check_status(c, err);

@@ -1659,9 +1659,9 @@ void gm_launch_shake(const ClusterArgs &c, int n_atoms, const double *dref, doub
     gm_launch_shake_solve(c, n_atoms, pos, s);
 }
 
-void gm_launch_rattle(const ClusterArgs &c, int n_atoms, const double *pos, double *vel, cudaStream_t s) {
+void gm_launch_rattle(const ClusterArgs &c, int n_atoms, const double *pos, double *vel, bool reset, cudaStream_t s) {
     if (c.n_clusters == 0) return;
-    reset_T<<<1, 1, 0, s>>>(c.status, 1);
+    if (reset) reset_T<<<1, 1, 0, s>>>(c.status, 1);
     const int b = cluster_blocks(c);
     cluster_phase1<true><<<b, 32, 0, s>>>(c, const_cast<double *>(pos), vel, n_atoms);
     cluster_phase2<true><<<b, 32, 0, s>>>(c, const_cast<double *>(pos), vel, n_atoms);

@@ -462,7 +462,8 @@ void gm_launch_shake(const ClusterArgs &c, int n_atoms, const double *dref, doub
 // (warm-start displacement when c.lam0 is set, then both phases)
 void gm_launch_shake_prepare(const ClusterArgs &c, int n_atoms, const double *dref, cudaStream_t s);
 int gm_launch_shake_solve(const ClusterArgs &c, int n_atoms, double *pos, cudaStream_t s);
-void gm_launch_rattle(const ClusterArgs &c, int n_atoms, const double *pos, double *vel, cudaStream_t s);
+// `reset`: clear rattle_T first (a status reset has cleared it already).
+void gm_launch_rattle(const ClusterArgs &c, int n_atoms, const double *pos, double *vel, bool reset, cudaStream_t s);
 void gm_launch_step(DevStatus *st, cudaStream_t s);
 // Unconstrained step: half-kicks (the previous step's closing one and this
 // step's opening one) + drift (with the velocity resync) + rebuild check +
