@@ -61,6 +61,12 @@ __device__ __forceinline__ double rsqrt64(double x) {
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// Image count up to which the FP32 distance of a pair k boxes of length L apart
+// is within rc2_pre's margin of 1e-3 + 1e-6 (L + cutoff): a component carries
+// at most (3 k + 2) L 2^-24 (raw difference, FP32 box, product), the distance
+// sqrt(3) of that, 8.3e-7 L for k = 2.
+constexpr float kPreImages = 2.f;
+
 // FP64 nonbonded kernel (the FP64 path): force/nonbonded.rs:20-82 in FP64 on
 // the sorted FP64 copies.  The same work split as the mixed kernel (a 32-atom
 // group's columns over `split` warps, 2/4/8 warps per block, optional
@@ -70,7 +76,8 @@ __device__ __forceinline__ double rsqrt64(double x) {
 // work is moved off it where that costs no bit of precision:
 //   * an entry beyond the cutoff (42 % of a column) is dropped by an FP32
 //     distance from the slot records with a margin (rc2_pre) that covers its
-//     rounding, and the FP64 cutoff test is an integer comparison;
+//     rounding up to kPreImages boxes apart (positions unwrapped further go to
+//     the FP64 test), and that test is an integer comparison;
 //   * the nearest image is taken without a division (gm_min_image);
 //   * one reciprocal square root (rsqrt64) replaces a square root and a
 //     division, and the switch multiplies by 1 / (cutoff - switch radius).
@@ -122,12 +129,15 @@ pair_kernel_f64(int n, int n_slots, int cap, int split, const double4 *__restric
                 gm_ld_coord(coord + 2 * j, jh, jl);
                 float x = (jh.x - mh.x) + (jl.x - ml.x), y = (jh.y - mh.y) + (jl.y - ml.y),
                       z = (jh.z - mh.z) + (jl.z - ml.z);
+                bool sure = true;
                 if (PERIODIC) {
-                    x = fmaf(-(float)bx, rintf(x * ibox.x), x);
-                    y = fmaf(-(float)by, rintf(y * ibox.y), y);
-                    z = fmaf(-(float)bz, rintf(z * ibox.z), z);
+                    const float kx = rintf(x * ibox.x), ky = rintf(y * ibox.y), kz = rintf(z * ibox.z);
+                    x = fmaf(-(float)bx, kx, x);
+                    y = fmaf(-(float)by, ky, y);
+                    z = fmaf(-(float)bz, kz, z);
+                    sure = fmaxf(fabsf(kx), fmaxf(fabsf(ky), fabsf(kz))) <= kPreImages;
                 }
-                if (fmaf(z, z, fmaf(y, y, x * x)) > rc2_pre) continue;
+                if (fmaf(z, z, fmaf(y, y, x * x)) > rc2_pre && sure) continue;
             }
             const double4 pj = p64[j];
             double dx = pj.x - mi.x, dy = pj.y - mi.y, dz = pj.z - mi.z;
