@@ -171,8 +171,12 @@ pair_item_mixed(int wid, int lane, int n, int cap, int split, const float4 *__re
     const int group = wid / split, part = wid - group * split;
     // without the outer half of the skin while nothing can have come in from it
     const bool inner = sys_far && sys_far[group_sys[group]] == 0u;
-    const int gm = inner ? gmax_in[group] : gmax[group];
-    const int per = ((gm + split - 1) / split + kChunk - 1) / kChunk * kChunk;
+    // With energies the parts are those of the whole columns, so that the energy
+    // partials hold the same chunks whichever columns a call walks; the forces
+    // are the same bits for any parts (98,304 atoms of water, 10 steps: 6,795 us
+    // so, 6,845 with the whole columns' parts in every step).
+    const int gm = inner ? gmax_in[group] : gmax[group], cols = ENERGY ? gmax[group] : gm;
+    const int per = ((cols + split - 1) / split + kChunk - 1) / kChunk * kChunk;
     const int e_begin = part * per, e_end = min(gm, e_begin + per);
     if (e_begin >= e_end) {  // no columns left for this part
         if (ENERGY && lane == 0) epart[wid] = 0.0;
@@ -280,8 +284,8 @@ pair_item_quad(int wid, int warp, int lane, const ForceArgs &fa, const float4 *s
     const PairConst &k = fa.pc;
     const int split = fa.split, group = wid / split, part = wid - group * split;
     const bool inner = fa.sys_far && fa.sys_far[fa.group_sys[group]] == 0u;
-    const int gm = inner ? fa.gmax_in[group] : fa.gmax[group];
-    const int per = ((gm + split - 1) / split + kChunk - 1) / kChunk * kChunk;
+    const int gm = inner ? fa.gmax_in[group] : fa.gmax[group], cols = ENERGY ? fa.gmax[group] : gm;
+    const int per = ((cols + split - 1) / split + kChunk - 1) / kChunk * kChunk;
     const int e_begin = part * per, e_end = min(gm, e_begin + per);
     if (e_begin >= e_end) {  // block-uniform: no columns left for this part
         if (ENERGY && warp == 0 && lane == 0) fa.epart[wid] = 0.0;
