@@ -79,7 +79,8 @@ struct gm_ctx {
     int bbox_blocks = 0;
     // list
     int cap = 0, cap_seg = 0, n_groups = 0;  // list entries per atom; staging entries per atom and z layer
-    int split = 1;                   // warps per group in the pair kernel
+    int split = 1;                   // parts of a group's columns in the pair kernel, 1 to GM_SET_SPLIT
+    int fine = 1;                    // work items per part: 2 in mixed systems whose items would else be too long
     int term_chunk = 128;            // bonded terms per work item of the persistent kernel
     int pair_warps = 4, pair_grid = 0;  // FP32 pair kernel block size and grid (0: one item per warp)
     int *d_list = nullptr, *d_count = nullptr, *d_gmax = nullptr, *d_stage = nullptr;
@@ -306,7 +307,7 @@ ForceArgs force_args(gm_ctx *c) {
     a.atom_sys = c->d_atom_sys;
     a.e_sys = c->n_sys > 1 ? c->d_e_sys : nullptr;
     a.cap = c->cap;
-    a.split = c->split;
+    a.split = c->split * c->fine;
     a.term_chunk = c->term_chunk;
     a.quad = c->n_sys == 1 && c->n_groups <= kQuadGroups;
     a.pair_warps = c->pair_warps;
@@ -1846,8 +1847,15 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         const int warps = 24 * std::max(dev_sms, 1);
         // The FP64 pair kernel is no queue and waits for one pipe: two items
         // per warp (5,000 atoms: 1.54 ms for five steps, 1.90 with eight).
-        const int want = (c->fp64 ? 2 : 8) * warps, most = c->fp64 ? GM_SET_SPLIT : GM_MAX_SPLIT;
-        c->split = std::max(1, std::min(most, (want + c->n_groups - 1) / std::max(c->n_groups, 1)));
+        const int want = ((c->fp64 ? 2 : 8) * warps + c->n_groups - 1) / std::max(c->n_groups, 1);
+        // The split that callers set and the tuner times ends at 16; where more
+        // is wanted (mixed, up to 1,824 groups) every part is two items.  With
+        // 16 items a group 20 steps of 1,536 atoms of water 2,143 -> 2,164 us, a
+        // trait iteration of 5,184 525 -> 546, 10 steps of 24,000 with frames
+        // 3,465 -> 3,570 (5 of a 20,011-atom chain 1,067 -> 1,039: the tuner's
+        // to find).
+        c->fine = !c->fp64 && want > GM_SET_SPLIT ? GM_MAX_SPLIT / GM_SET_SPLIT : 1;
+        c->split = std::max(1, std::min(GM_SET_SPLIT, (want + c->fine - 1) / c->fine));
         const long long terms = (long long)c->n_bonds + c->n_angles + c->n_diheds + c->n14;
         c->term_chunk = terms > 32ll * warps ? 128 : 32;
     }
@@ -2697,7 +2705,8 @@ int32_t gm_autotune(gm_ctx *c, int32_t reps, int64_t *choice) {
     cudaEvent_t e0, e1;
     GM_CUDA(c, cudaEventCreate(&e0));
     GM_CUDA(c, cudaEventCreate(&e1));
-    const int splits[] = {1, 2, 3, 4, 6, 8, 12, 16};
+    std::vector<int> splits = {1, 2, 3, 4, 6, 8, 12, 16};
+    if (std::find(splits.begin(), splits.end(), c->split) == splits.end()) splits.push_back(c->split);
     const int warps[] = {2, 4, 8};
     const int grids[] = {0, 2, 4, 8, 16};  // 0: one work item per warp, else blocks per SM (persistent)
     double best = 1e300;

@@ -35,7 +35,7 @@ constexpr double GM_FORCE_TO_ACCEL = 20.455 * 20.455;  // kcal/mol/A/amu -> A/ps
 #define GM_MAX_TYPES 64
 #define GM_WARP 32
 #define GM_MAX_SPLIT 32      // largest number of work items per 32-atom group in the pair kernels
-#define GM_SET_SPLIT 16      // largest one gm_pair_shape accepts and gm_autotune tries
+#define GM_SET_SPLIT 16      // largest split (parts of a group, each one or two work items) of a context
 // The list build runs GM_NSEG warps per 32-atom group, one per z layer of the
 // 5 x 5 x (span + 4) cell box the group's candidates come from (cells are at
 // least half the list radius wide).  Each warp fills its own staging segment;
@@ -356,7 +356,7 @@ struct ForceArgs {
     int n_slots;             // n_groups * 32 (each system padded to whole groups)
     const int *group_sys, *atom_sys;
     long long *e_sys;        // per-system potential energy, fixed point 2^-32 kcal/mol (batches), or nullptr
-    int split;               // warps per 32-atom group in the FP32 pair kernel
+    int split;               // work items per 32-atom group in the pair kernels
     int quad;                // the persistent kernel gives a pair item a block (small systems)
     int term_chunk;          // bonded terms (or 1-4 pairs) per work item of the persistent kernel
     int pair_warps;          // warps per block of the FP32 pair kernel (2, 4, 8)

@@ -242,9 +242,11 @@ int32_t gm_frames_take(gm_ctx *ctx, int64_t max_frames, float *xyz, uint64_t *st
  *
  * Times the context's pair kernel (mixed or FP64) on the current list
  * (reps launches per candidate, CUDA events on the context's stream) over
- * warps per 32-atom group (1-16: list columns per warp), warps per block (2,
- * 4, 8) and grid (one work item per warp, or a persistent grid of 2-16
- * blocks per SM), and keeps the fastest.  In the persistent step form
+ * the split of a 32-atom group's list columns (1-16 parts and the context's
+ * present split; a part is one warp's work item, or two of them in a mixed
+ * system too small to fill the device with 16), warps per block (2, 4, 8) and
+ * grid (one work item per warp, or a persistent grid of 2-16 blocks per SM),
+ * and keeps the fastest.  In the persistent step form
  * (gm_step_form) the split is then timed again on the persistent kernel's
  * force phase and the fastest kept.  Every candidate computes the same force
  * bits (fixed 32-entry chunks folded into int64 sums).  choice (nullable):
