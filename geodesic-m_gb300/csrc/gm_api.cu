@@ -468,9 +468,15 @@ bool force_phase(const gm_ctx *c) { return c->step_form == GM_STEP_PERSISTENT &&
 
 // Constrained resident steps run as two cooperative launches around the force
 // evaluation when every cluster is a star, their lanes are resident at once,
-// and no warm start needs the solve's own launches.
+// no warm start needs the solve's own launches, and the longest solve that the
+// caller allows ends well within the barrier's limit: the lanes that are done
+// wait for those that are not.  An iteration takes 2.9 us (64 constraints) to 10
+// us (60,000), so 20,000 of them are under a fifth of the 1.35 s after which a
+// waiting block gives up; a solver allowed more keeps the separate launches.
+constexpr unsigned kFusedIterations = 20000;
 bool fused_solve(gm_ctx *c) {
     if (!c->n_clusters || c->n_star_end != c->n_clusters || c->ws_on || c->ws_rec_stride > 0) return false;
+    if (c->p.max_constr_iter > kFusedIterations) return false;
     if (c->solve_blocks < 0) gm_solve_step_grid(cluster_args(c), c->n_free, &c->solve_threads, &c->solve_blocks,
                                                &c->solve_quads);
     return c->solve_blocks > 0;

@@ -284,7 +284,7 @@ int32_t gm_step_form(gm_ctx *ctx, int32_t form);
 /* Error-path test of the persistent form's grid barrier: the next call that
  * runs persistent steps starts with the barrier's arrival count far past the
  * grid, so no block can release it.  Every block waits out the barrier's
- * poll limit (a fraction of a second), records the timeout and returns; the
+ * poll limit (about 1.35 s), records the timeout and returns; the
  * call returns GM_ERR_DEVICE with nothing stepped, and the context is usable
  * afterwards.  GM_ERR_UNSUPPORTED unless the context steps in the
  * persistent form. */
