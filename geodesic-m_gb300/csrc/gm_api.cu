@@ -1550,7 +1550,9 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
                 // nonbonded.rs:46-47 Lorentz-Berthelot, evaluated as the reference does
                 const double sg = 0.5 * (sg_[a] + sg_[b]);
                 const double ep = std::sqrt(ep_[a] * ep_[b]);
-                tab64[T2 * (size_t)sy + a * (size_t)c->ntypes + b] = make_double2(sg * sg, 24.0 * ep);
+                // without a well depth no radius either: (sigma / r)^6 of a pair
+                // in contact would overflow, and infinity times 0 is NaN
+                tab64[T2 * (size_t)sy + a * (size_t)c->ntypes + b] = make_double2(ep != 0.0 ? sg * sg : 0.0, 24.0 * ep);
                 // the mixed pair kernel's double-float (sigma^2, 24 epsilon)
                 const double s2 = sg * sg, e24 = 24.0 * ep;
                 const float s2h = (float)s2, e24h = (float)e24;

@@ -376,7 +376,7 @@ struct ForceArgs {
     const unsigned int *sys_far;
     int ntypes;
     const float4 *tab32;     // (sigma_ij^2, 24 epsilon_ij) per type pair, each a double-float (hi, lo)
-    const double2 *tab64;    // (sigma_ij^2, 24 epsilon_ij)
+    const double2 *tab64;    // (sigma_ij^2, 24 epsilon_ij), or zeros where epsilon_ij is 0
     PairConst pc;            // the mixed pair kernel's constants
     double rc2_64, rsw_64, rc_64, inv_wsw_64;
     float rc2_pre;           // FP64 kernel's FP32 pre-test: beyond it a pair is outside the cutoff for certain
