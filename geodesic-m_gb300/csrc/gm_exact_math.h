@@ -19,6 +19,9 @@
  * gm_abs_ge: |v| >= t for a positive finite t, by integer comparison of the
  *            bits (an FP64 comparison occupies the FP64 pipe like any other
  *            FP64 instruction); false for a NaN.
+ * gm_moved_far: d2 >= far_sq for a squared distance d2 >= 0 and far_sq >= 0,
+ *            rounded towards yes (the high words, no FP64 comparison); a NaN of
+ *            either sign counts as far.
  * gm_min_image: d - L round(d / L), round half away from zero, each operation
  *            rounded on its own: the reference's min_image
  *            (neighbor.rs:74-76).  Away from |d| = L/2 the rounded quotient
@@ -96,6 +99,10 @@ GM_HD int gm_abs_ge(double v, double t) {
     return a >= tb && a <= 0x7ff0000000000000ull;
 }
 
+GM_HD int gm_moved_far(double d2, double far_sq) {
+    return (unsigned)gm_hi_word(d2) >= (unsigned)gm_hi_word(far_sq);
+}
+
 GM_HD double gm_min_image(double d, double L) {
     const int hd = gm_hi_word(d) & 0x7fffffff, hl = gm_hi_word(L);
     if (hd < hl - 0x101000) return d; /* |d| < L/2 (1 - 2^-8) */
@@ -107,6 +114,5 @@ GM_HD double gm_min_image(double d, double L) {
     return d - L * round(d / L);
 #endif
 }
-
 
 #endif

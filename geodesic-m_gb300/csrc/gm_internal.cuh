@@ -284,12 +284,6 @@ __device__ __forceinline__ bool gm_grid_barrier(unsigned *arrive, unsigned *gen,
     return s_ok != 0;
 }
 
-// d2 > far_sq for d2 >= 0, rounded towards yes (the high words: no FP64
-// comparison); a NaN counts as far.
-__device__ __forceinline__ bool gm_moved_far(double d2, double far_sq) {
-    return __double2hiint(d2) >= __double2hiint(far_sq);
-}
-
 // ------------------------------------------------------- launcher exports
 
 struct ListArgs {
