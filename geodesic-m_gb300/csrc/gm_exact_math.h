@@ -16,6 +16,13 @@
  *            correction for any den of ordinary size (2^-200 to 2^200, the
  *            caller's to see); a numerator that is zero, tiny or huge takes
  *            the division.
+ * gm_rsqrt_step: 1 / sqrt(x) from a seed y within 2^-22 of it: one step of
+ *            Chebyshev's third-order method (J. F. Traub, "Iterative Methods for
+ *            the Solution of Equations", 1964) for y^-2 - x, which is
+ *            y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.  |e| < 2^-20.9, so the
+ *            next term of the series, 5/16 e^3, is below 2^-64; the rounding of
+ *            x y moves the result by half an ulp at most, its own rounding by
+ *            another half.
  * gm_abs_ge: |v| >= t for a positive finite t, by integer comparison of the
  *            bits (an FP64 comparison occupies the FP64 pipe like any other
  *            FP64 instruction); false for a NaN.
@@ -85,6 +92,11 @@ GM_HD double gm_div_rcp(double num, double den, double y) {
     /* |num| in [2^-700, 2^700) */
     if ((unsigned)((gm_hi_word(num) & 0x7fffffff) - ((1023 - 700) << 20)) >= (unsigned)(1400 << 20)) return num / den;
     return gm_div_by_dt(num, den, y);
+}
+
+GM_HD double gm_rsqrt_step(double x, double y) {
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 GM_HD int gm_abs_ge(double v, double t) {

@@ -45,20 +45,18 @@ pair_kernel_mixed(int n, int n_slots, int cap, int split, const float4 *__restri
 
 // 1/sqrt(x) in FP64 from the MUFU seed: the seed's argument is x truncated to
 // FP32 and the seed is widened again by moving bits (no conversion
-// instruction: those run on the FP64 pipe), then one cubically convergent step,
-// y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2 (|e| < 2^-20, so the error of the
-// step is below 2^-60): five FP64 operations, within 2 ulp.  x is a squared
-// distance, far inside FP32's normal range for every pair inside a cutoff
-// and away from contact; outside it (x < 2^-100 or beyond 2^100) the library's
-// square root and a division are used.
+// instruction: those run on the FP64 pipe), then one step of Chebyshev's
+// third-order method (gm_rsqrt_step): five FP64 operations, within 1 ulp and a
+// little (the square root and the division it replaces: 1 ulp too).  x is a
+// squared distance, far inside FP32's normal range for every pair inside a
+// cutoff and away from contact; outside it (x < 2^-100 or beyond 2^100) the
+// library's square root and a division are used.
 __device__ __forceinline__ double rsqrt64(double x) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
     if ((unsigned)(hi - ((1023 - 100) << 20)) >= (unsigned)(200 << 20)) return 1.0 / sqrt(x);
     const unsigned f = __funnelshift_l((unsigned)lo, (unsigned)hi, 3) + 0x40000000u;
     const unsigned g = __float_as_uint(rsqrt_approx(__uint_as_float(f)));
-    const double y = __hiloint2double((int)((g >> 3) + (896u << 20)), (int)(g << 29));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    return gm_rsqrt_step(x, __hiloint2double((int)((g >> 3) + (896u << 20)), (int)(g << 29)));
 }
 
 // Image count up to which the FP32 distance of a pair k boxes of length L apart
