@@ -5,12 +5,18 @@
 // and the force buffer, on the device.  Host entry points upload the caller's
 // arrays, run the kernels on the context's stream and copy results back;
 // the resident entry points keep everything on the device and run the BAB
-// loop as a CUDA graph, one captured step per launch: without constraints the
-// fused kernel (the previous step's closing half-kick, this step's opening
-// one, drift, rebuild check, coordinate pack), an IF node holding the list
-// rebuild, and the forces (pair kernel beside the bonded/1-4 kernel); with
-// constraints half-kick, drift, SHAKE, check, the IF node, forces,
-// half-kick, RATTLE.
+// loop as CUDA graphs whose IF node holds the list rebuild.  A step is
+//   * without constraints, mixed precision: one persistent launch (gm_step.cu;
+//     for small systems up to GM_LOOP_STEPS steps a launch);
+//   * without constraints otherwise (FP64, trajectory frames, GM_STEP_GRAPH):
+//     the fused kernel (the previous step's closing half-kick, this step's
+//     opening one, drift, rebuild check, coordinate pack), the IF node, the
+//     forces;
+//   * with constraints: two cooperative launches round the IF node and the
+//     forces (half-kick, drift, SHAKE, check, pack; half-kick, RATTLE), or the
+//     separate kernels of those phases (fused_solve).
+// A call's steps are one graph with a WHILE node round the step (loops), or one
+// graph launch each.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -78,7 +84,7 @@ struct gm_ctx {
     double *d_bbox = nullptr;
     int bbox_blocks = 0;
     // list
-    int cap = 0, cap_seg = 0, n_groups = 0;  // list entries per atom; staging entries per atom and z layer
+    int cap = 0, cap_seg = 0, n_groups = 0;  // list entries per atom; staged rows of 32 ints per group and z layer
     int split = 1;                   // parts of a group's columns in the pair kernel, 1 to GM_SET_SPLIT
     int fine = 1;                    // work items per part: 2 in mixed systems whose items would else be too long
     int term_chunk = 128;            // bonded terms per work item of the persistent kernel
@@ -328,7 +334,6 @@ ForceArgs force_args(gm_ctx *c) {
     const double rc = c->p.r_cutoff, rsw = c->p.r_switch;
     a.rc2_64 = rc * rc;
     a.rsw_64 = rsw;
-    a.rc_64 = rc;
     a.inv_wsw_64 = 1.0 / (rc - rsw);
     {
         // the FP32 distance carries the box's FP32 rounding for image pairs
@@ -686,7 +691,8 @@ void drop_graph(gm_ctx *c) {
 }
 
 // The list (cap entries per atom) and the list build's staging area (GM_NSEG
-// z layers of cap_seg entries per atom).
+// z layers of cap_seg rows of 32 ints per group; a word of 32 candidates takes
+// four rows).
 int ensure_list_buffers(gm_ctx *c, int cap, int cap_seg) {
     if (cap == c->cap && cap_seg == c->cap_seg && c->d_list && c->d_stage) return GM_OK;
     if (cap != c->cap || !c->d_list) {
@@ -711,8 +717,9 @@ int ensure_list_buffers(gm_ctx *c, int cap, int cap_seg) {
 int round32(double x) { return std::max(((int)std::ceil(x) + 31) / 32 * 32, 32); }
 
 // List capacity from the densest system's mean density, and the staging
-// capacity of one z layer: a layer of cells about half the list radius thick
-// through the middle of the sphere holds ~37 % of it.
+// capacity of one z layer, one row for each entry that an atom may have there: a
+// layer of cells about half the list radius thick through the middle of the
+// sphere holds ~37 % of it.
 int ensure_estimated_buffers(gm_ctx *c, const double *px, const double *py, const double *pz) {
     // densest system: its atoms over its bounding box (or the periodic box)
     double est = 32.0;
@@ -1794,8 +1801,8 @@ gm_ctx *create_impl(int n_sys, const gm_atoms *sys_atoms, const gm_topology *sys
         }
         c->n_slots = slot_off.back();
         c->total_cells = cell_off.back();
-        if (c->n_slots > GM_SLOT_MASK) {
-            fail(c, GM_ERR_UNSUPPORTED, "%d padded atom slots; at most %d are supported", c->n_slots, GM_SLOT_MASK);
+        if (c->n_slots > GM_MAX_SLOTS) {
+            fail(c, GM_ERR_UNSUPPORTED, "%d padded atom slots; at most %d are supported", c->n_slots, GM_MAX_SLOTS);
             return bail(GM_ERR_UNSUPPORTED);
         }
         TRY(dupload(c, &c->d_sys_atom_off, mg.atom_off.data(), mg.atom_off.size()));

@@ -9,7 +9,8 @@
 // every constraint per Jacobi iteration and stops when max|lambda| < tol
 // over all of them.  Constraints only couple through shared atoms, so the
 // work splits into independent clusters (connected components of the
-// constraint graph, found once on the host); one thread owns one cluster.
+// constraint graph, found once on the host): a star has a lane per constraint
+// (or four), another cluster a warp, a large one a thread.
 // Phase 1 iterates each cluster until its own max|lambda| < tol and records
 // its count t_c; the global count is T = max t_c (the first iteration where
 // every cluster is below tol, given that a converged cluster stays below

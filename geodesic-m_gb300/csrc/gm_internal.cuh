@@ -38,17 +38,16 @@ constexpr double GM_FORCE_TO_ACCEL = 20.455 * 20.455;  // kcal/mol/A/amu -> A/ps
 #define GM_SET_SPLIT 16      // largest split (parts of a group, each one or two work items) of a context
 // The list build runs GM_NSEG warps per 32-atom group, one per z layer of the
 // 5 x 5 x (span + 4) cell box the group's candidates come from (cells are at
-// least half the list radius wide).  Each warp fills its own staging segment;
-// the block then concatenates the segments, layer by layer, into each lane's
-// list column.
+// least half the list radius wide), or one per layer and y row.  Each warp
+// stages the candidates its lanes accept, as masks over words of 32 candidates,
+// in its own segment; the block then writes the segments' entries, one after
+// the other, into each lane's list column.
 #define GM_NSEG 5
 // Threads per block of the bonded and 1-4 kernels.
 #define GM_BONDED_THREADS 64
-// List columns are ordered by build-time distance in GM_NBUCKET buckets; the
-// build stages a slot index with its bucket in the top bits.
+// List columns are ordered by build-time distance in GM_NBUCKET buckets.
 #define GM_NBUCKET 4
-#define GM_BUCKET_SHIFT 27
-#define GM_SLOT_MASK ((1 << GM_BUCKET_SHIFT) - 1)  // slots per context stay below 2^27
+#define GM_MAX_SLOTS ((1 << 27) - 1)  // padded atom slots of a context
 
 // Device status bits (DevStatus::error).
 enum : unsigned int {
@@ -309,7 +308,7 @@ struct ListArgs {
     int *list, *count, *gmax;
     int *count_in, *gmax_in;        // the same without the last distance bucket (the outer half of the skin)
     unsigned int *sys_far;          // nonzero: an atom of the system moved more than far_sq since its build (or nullptr)
-    int *stage;              // [group][layer][entry][lane], cap_seg entries per layer
+    int *stage;              // [group][warp][word][4 rows][lane], cap_seg rows per layer
     double *ref;             // FP64 x|y|z copy at each system's build
     long long *force;        // zeroed with the pack
     GridInfo *grid;          // one per system
@@ -372,7 +371,7 @@ struct ForceArgs {
     const float4 *tab32;     // (sigma_ij^2, 24 epsilon_ij) per type pair, each a double-float (hi, lo)
     const double2 *tab64;    // (sigma_ij^2, 24 epsilon_ij), or zeros where epsilon_ij is 0
     PairConst pc;            // the mixed pair kernel's constants
-    double rc2_64, rsw_64, rc_64, inv_wsw_64;
+    double rc2_64, rsw_64, inv_wsw_64;
     float rc2_pre;           // FP64 kernel's FP32 pre-test: beyond it a pair is outside the cutoff for certain
     int coulomb;
     float box[3], inv_box[3];
@@ -540,12 +539,14 @@ void gm_launch_rattle_step(const ClusterArgs &c, const SolveStepArgs &sa, int th
 int gm_step_persistent_blocks(const ForceArgs &fa);
 void gm_launch_step_persistent(const ForceArgs &fa, const StepArgs &sa, const PackArgs &pk, int blocks,
                                cudaStream_t s);
+// Whether the step kernel of these arguments can run several steps a launch.
+bool gm_step_loops(const ForceArgs &a);
+// Clears the step's words; `fresh`: the forces are summed already; `todo`: the
+// steps of the call.
+void gm_launch_step_begin(StepSync *sync, bool fresh, long long todo, cudaStream_t s);
 // The persistent kernel's force phase alone, with energies (the force
 // kernels' partials, the same bits), as a plain launch: pair items and bonded
 // / 1-4 blocks from one queue.  The queue words must be zero.
-// Whether the step kernel of these arguments can run several steps a launch.
-bool gm_step_loops(const ForceArgs &a);
-void gm_launch_step_begin(StepSync *sync, bool fresh, long long todo, cudaStream_t s);
 void gm_launch_forces_persistent(const ForceArgs &fa, StepSync *sync, int blocks, cudaStream_t s);
 void gm_launch_kick_drift_check(int n, double *pos, double *vel, double *dref, long long *force,
                                 const double *inv_mass, double dt_half, double dt, const double *ref, double thr_sq,

@@ -10,11 +10,11 @@
 // systems that need it.  Each system owns a range of atoms, a 32-aligned
 // range of sorted slots (padding slots have perm = -1 and no list), a range
 // of cells and its own grid; perm and the list entries hold global indices.
-// The list build gives each warp 32 consecutive cell-sorted atoms of one
-// system and one z layer of their candidate cell box (five warps per group,
-// each filling its own list segment); the warp streams the candidates of
-// each cell row of its layer through shared memory and each lane tests them
-// against its own atom.  The
+// The list build gives a block 32 consecutive cell-sorted atoms of one system
+// and each of its warps one z layer of their candidate cell box (or a share of a
+// layer's y rows); the warp streams the candidates near the 32 atoms through
+// shared memory, each lane tests them against its own atom and stages what it
+// accepts as bits, and the block writes them into the lanes' columns.  The
 // test runs in FP32 on hi+lo coordinates; candidates within `margin` of the
 // list radius are re-decided with the reference's exact FP64 expression
 // (min-image, then dx*dx + dy*dy + dz*dz, no fused multiply-add), so the pair

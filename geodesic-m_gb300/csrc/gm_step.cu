@@ -26,7 +26,7 @@
 // second grid barrier ends each step, and its last block decides whether the
 // launch goes on (no rebuild, no error, steps left).  The call is one graph:
 // WHILE steps are left, the launch, IF rebuild.  50 steps of 224 atoms: 1,902 us
-// with a launch a step, 1,471 so, 1,376 with phase 3 a component per lane.
+// with a launch a step, 1,471 so, 1,420 with phase 3 a component per lane.
 // Larger systems keep a launch a step: coordinates that the launch itself writes
 // cannot be read through the read-only path, and without it 98,304 atoms were
 // 1.5 % and 786,432 1.6 % slower.
