@@ -456,7 +456,7 @@ int seq_rebuild(gm_ctx *c, cudaStream_t s, bool all, bool wrap = true, const uns
     gm_launch_grid(a, s);
     gm_launch_bin(a, s);
     gm_launch_pack(a, c->fp64, s);
-    gm_launch_build(a, s);
+    gm_launch_build(a, all, s);
     gm_launch_flags(a, false, s);
     // [flags], wrap or bbox, grid (clears the cells), assign, scan, scatter,
     // rank, pack, build and its second kernel, clear flags
@@ -767,7 +767,11 @@ int do_build(gm_ctx *c, bool all = true) {
         // overflow, or (when every system was built) within 20 % of a
         // capacity, since a resident run cannot grow the list, grow that
         // capacity to a third above the need
-        const int need = (int)c->h_status->max_count, need_l = (int)c->h_status->max_layer;
+        // (a build of some systems may split the layers' rows where this one
+        // did not: about twice the words for the same candidates)
+        const bool rows = gm_build_splits_rows(list_args(c), all || attempt > 0);
+        const int need = (int)c->h_status->max_count,
+                  need_l = (int)c->h_status->max_layer * (!rows && gm_build_splits_rows(list_args(c), false) ? 2 : 1);
         const bool over = rc == GM_ERR_LIST_OVERFLOW;
         const bool room = !rc && (all || attempt > 0);
         const bool grow = need > (over ? c->cap : c->cap - c->cap / 5);
@@ -2191,7 +2195,7 @@ int32_t gm_profile(gm_ctx *c, int32_t which, int32_t n_iter, double dt, double *
             case 6: gm_launch_pair14(fa, c->fp64, c->stream); break;
             case 7:  // the list build kernel alone, every system
                 gm_launch_flags(la, true, c->stream);
-                gm_launch_build(la, c->stream);
+                gm_launch_build(la, true, c->stream);
                 gm_launch_flags(la, false, c->stream);
                 break;
             default: gm_launch_pack(la, c->fp64, c->stream); break;

@@ -331,7 +331,10 @@ void gm_launch_flags(const ListArgs &a, bool set, cudaStream_t s);
 void gm_launch_wrap(const ListArgs &a, double *pos, const unsigned int *done, cudaStream_t s);
 void gm_launch_grid(const ListArgs &a, cudaStream_t s);
 void gm_launch_bin(const ListArgs &a, cudaStream_t s);
-void gm_launch_build(const ListArgs &a, cudaStream_t s);
+// `all`: every system is marked.
+void gm_launch_build(const ListArgs &a, bool all, cudaStream_t s);
+// Whether that build splits a layer's y rows over warps.
+bool gm_build_splits_rows(const ListArgs &a, bool all);
 void gm_launch_pack(const ListArgs &a, bool fp64, cudaStream_t s);
 
 // Constants of the mixed pair kernel; the low parts complete double-floats.

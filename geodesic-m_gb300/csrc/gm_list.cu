@@ -433,9 +433,10 @@ constexpr int kRound = 256, kRoundY = 64;
 constexpr int kWordRows = 4;
 // gmax of a group whose words did not fit the staging area
 constexpr int kStageOver = -1;
-// Groups (per system) up to which the build splits a layer's y rows over
-// warps: 162 groups 125 us against 191, 48 groups 66 against 144; 750 groups
-// 291 against 259, 3,072 groups 921 against 793 (partly filled words).
+// Groups up to which a build splits a layer's y rows over warps: 48 groups 66 us
+// against 144, 162 groups 125 against 191, 252 (four systems of 2,000 atoms) 116
+// against 135; 256 (16 of 500) 103 against 91, 500 (two of 8,000) 238 against
+// 185, 3,072 groups 921 against 793 (partly filled words).
 constexpr int kYSplitGroups = 300;
 
 // One block per group, one warp per z layer: warp `seg` tests the candidates
@@ -866,7 +867,16 @@ void gm_launch_pack(const ListArgs &a, bool fp64, cudaStream_t s) {
     pack_kernel<<<(a.n_slots + 255) / 256, 256, 0, s>>>(a, fp64);
 }
 
-void gm_launch_build(const ListArgs &a, cudaStream_t s) {
+// A build of every system covers all groups, another of a batch a few systems,
+// as many groups as one of them on average: with the average for both the first
+// build of 64 systems of 2,000 atoms took 1,323 us (now 709), of 256 of 500 1,235
+// (535).
+bool gm_build_splits_rows(const ListArgs &a, bool all) {
+    const int groups = a.n_slots / 32;
+    return (all ? groups : groups / a.n_sys) <= kYSplitGroups;
+}
+
+void gm_launch_build(const ListArgs &a, bool all, cudaStream_t s) {
     if (a.n_slots == 0) return;
     const int groups = a.n_slots / 32;
     const double rl2 = a.r_list * a.r_list;  // neighbor.rs:25
@@ -875,8 +885,7 @@ void gm_launch_build(const ListArgs &a, cudaStream_t s) {
     const double rsh = 0.5 * (a.r_cut + a.r_list);
     const float3 bk = make_float3((float)(a.r_switch * a.r_switch), (float)(a.r_cut * a.r_cut), (float)(rsh * rsh));
     const float lo = (float)(rl2 - margin), hi = (float)(rl2 + margin);
-    // a system's rebuild covers groups / n_sys groups on average
-    const bool ysplit = groups / a.n_sys <= kYSplitGroups;
+    const bool ysplit = gm_build_splits_rows(a, all);
 #define GM_BUILD(P, Y) build_kernel<P, Y><<<groups, GM_NSEG * Y * 32, 0, s>>>(a, lo, hi, rl2, bk)
     if (a.periodic) { if (ysplit) GM_BUILD(true, 5); else GM_BUILD(true, 1); }
     else { if (ysplit) GM_BUILD(false, 5); else GM_BUILD(false, 1); }
