@@ -321,7 +321,7 @@ pair_item_quad(int wid, int warp, int lane, const ForceArgs &fa, const float4 *s
         for (int t = 0; t < kChunk / 4; t++) {
             jh = nh;
             jl = nl;
-            if (t + 1 < kChunk / 4) gm_ld_coord_rw(fa.coord + 2 * jj[t + 1], nh, nl);  // beside this round's arithmetic
+            if (t + 1 < kChunk / 4) gm_ld_coord_rw(fa.coord + 2 * jj[t + 1], nh, nl);  // beside these entries' arithmetic
             float d_h[3], d_l[3];
             const gm_df R = pair_r2<PERIODIC>(mh, ml, jh, jl, k, d_h, d_l);
             const bool in = R.h <= k.rc2 && R.h > 0.f;
